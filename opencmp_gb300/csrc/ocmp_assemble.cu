@@ -954,6 +954,12 @@ __global__ void __launch_bounds__(256) csr_gather_kernel(int64_t nnz, const int3
     }
 }
 
+// Per-label boundary data, by value: an allocation of the stream-ordered pool costs 210 us when the
+// stream was waited for since the last one (the pool gives its memory back), three times a small step.
+struct LabelData {
+    double bval[32], gval[32];
+};
+
 // Element right-hand sides: dt (f, phi_i) + mass (u_prev, phi_i) + boundary data.
 template <int D, int L>
 __global__ void rhs_elem_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
@@ -962,8 +968,8 @@ __global__ void rhs_elem_kernel(int64_t ne, const double* __restrict__ X, const 
                                 int nq, const double* __restrict__ qw, const double* __restrict__ qphi,
                                 const double* __restrict__ mvec, const double* __restrict__ Rm,
                                 const int32_t* __restrict__ ebf_ptr, const int32_t* __restrict__ ebf,
-                                const int32_t* __restrict__ bfac, const double* __restrict__ bval, uint32_t bval_mask,
-                                const double* __restrict__ gval, const double* __restrict__ bfq,
+                                const int32_t* __restrict__ bfac, LabelData lab_data, uint32_t bval_mask,
+                                const double* __restrict__ bfq,
                                 const double* __restrict__ gfq, int is_l2, int nfq, const double* __restrict__ fw,
                                 const double* __restrict__ fphi, const double* __restrict__ fdphi,
                                 const double* __restrict__ flam, const float2* __restrict__ Rmf,
@@ -1049,8 +1055,8 @@ __global__ void rhs_elem_kernel(int64_t ne, const double* __restrict__ X, const 
             const size_t base = ((size_t)lf * nfq + q) * L;
             const double wq = fw[q] * meas * dt;
             const double wn = hg ? wind_dot_n<D>(a, conn, e, flam + ((size_t)lf * nfq + q) * (D + 1), nrm) : 0.0;
-            const double bv = hb ? (bfq ? bfq[(size_t)b * nfq + q] : bval[lab]) : 0.0;
-            const double gv = hg ? (gfq ? gfq[(size_t)b * nfq + q] : gval[lab]) : 0.0;
+            const double bv = hb ? (bfq ? bfq[(size_t)b * nfq + q] : lab_data.bval[lab]) : 0.0;
+            const double gv = hg ? (gfq ? gfq[(size_t)b * nfq + q] : lab_data.gval[lab]) : 0.0;
 #pragma unroll
             for (int i = 0; i < L; i++) {
                 const double vi = fphi[base + i];
@@ -1391,22 +1397,17 @@ int rhs_impl(ocmp_space_s* s, const ocmp_form_t* f, const ocmp_rhs_t* r, double*
         OCMP_CUDA(cudaGetLastError());
         return OCMP_OK;
     }
-    // per-label data travels by value through a small device buffer owned by the call's stream
-    double* dvals = nullptr;
-    OCMP_CUDA(cudaMallocAsync((void**)&dvals, sizeof(double) * 64, st));
-    double hv[64];
+    LabelData lab_data;
     for (int k = 0; k < 32; k++) {
-        hv[k] = r->bval[k];
-        hv[32 + k] = r->gval[k];
+        lab_data.bval[k] = r->bval[k];
+        lab_data.gval[k] = r->gval[k];
     }
-    OCMP_CUDA(cudaMemcpyAsync(dvals, hv, sizeof(hv), cudaMemcpyHostToDevice, st));
     OCMP_LAUNCH(rhs_elem_kernel<D, L><<<nblk(ne, 128), 128, 0, st>>>(
         ne, mesh->dX, mesh->dconn, s->d_dofs, a, r->dt, r->src_kind, r->src_const, r->src_qp, r->mass, r->uprev,
-        s->T.nq, s->d_qw, s->d_qphi, s->d_mvec, s->d_Rc, s->d_ebf_ptr, s->d_ebf, s->d_bfac, dvals, r->bval_mask,
-        dvals + 32, r->bval_fq, r->gval_fq, s->kind == OCMP_L2, s->T.nfq, s->d_fw, s->d_fphi, s->d_fdphi, s->d_flam,
+        s->T.nq, s->d_qw, s->d_qphi, s->d_mvec, s->d_Rc, s->d_ebf_ptr, s->d_ebf, s->d_bfac, lab_data, r->bval_mask,
+        r->bval_fq, r->gval_fq, s->kind == OCMP_L2, s->T.nfq, s->d_fw, s->d_fphi, s->d_fdphi, s->d_flam,
         r->dfloat ? s->d_Rm_ff : nullptr, r->dfloat ? s->d_geo_ff : nullptr, s->d_Fe));
     OCMP_LAUNCH(rhs_gather_kernel<<<nblk(s->ndof, 256), 256, 0, st>>>(s->ndof, s->d_inc_ptr, s->d_inc, s->d_Fe, b, r->accumulate));
-    OCMP_CUDA(cudaFreeAsync(dvals, st));
     OCMP_CUDA(cudaGetLastError());
     return OCMP_OK;
 }

@@ -22,6 +22,7 @@
 
 #include "ocmp_internal.h"
 #include "ocmp_spmv.cuh"
+#include "ocmp_cg.cuh"
 
 namespace ocmp {
 // Per-instance strides of a batch of independent systems that share one sparsity pattern: the
@@ -101,9 +102,12 @@ struct ocmp_solver_s {
     float* r32 = nullptr;
     float* p32 = nullptr;
     float* d32 = nullptr;       // inner correction
+    double* pb = nullptr;       // second search direction (CG)
+    float* p32b = nullptr;
+    ocmp::CgResult* dcg = nullptr;   // CG: results and barrier state
+    ocmp::CgResult* hcg = nullptr;   // pinned
     // reductions and small state
     double* part = nullptr;     // (m+4) x nb
-    double* pspmv = nullptr;    // one partial per SpMV block (CG p . Ap)
     double* red = nullptr;      // m+2 reduced values
     double* st = nullptr;       // small state, see enum below
     double* H = nullptr;        // (m+1) x m
@@ -176,89 +180,6 @@ constexpr int kThreads = 256;
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
 template <class T>
-__device__ __forceinline__ double block_sum(T v) {
-    __shared__ double sh[kThreads / 32];
-    double d = (double)v;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[wid] = d;
-    __syncthreads();
-    double t = 0;
-    if (wid == 0) {
-        t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    }
-    return t;  // valid in thread 0
-}
-
-// out[k] = sum_b part[k * nb + b]; one block per k
-__global__ void reduce_kernel(int nb, int nk, const double* __restrict__ part, double* __restrict__ out,
-                              const int* __restrict__ flags, int gate) {
-    if (gate >= 0 && flags[gate] == 0) return;
-    const int k = blockIdx.x;
-    if (k >= nk) return;
-    double acc = 0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) acc += part[(int64_t)k * nb + b];
-    double t = block_sum(acc);
-    if (threadIdx.x == 0) out[k] = t;
-}
-
-// y = free ? A x : 0, optional partial of dot(x, y) (CG: p . A p).
-template <class TM, class TV, int TPR>
-__global__ void __launch_bounds__(kThreads) spmv_masked(int64_t n, const int32_t* __restrict__ rp,
-                                                        const int32_t* __restrict__ col, const TM* __restrict__ val,
-                                                        const uint8_t* __restrict__ freed, const TV* __restrict__ x,
-                                                        TV* __restrict__ y, double* __restrict__ part,
-                                                        const int* __restrict__ flags) {
-    if (flags && flags[F_CONV]) return;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t r = t / TPR;
-    const int lane = threadIdx.x % TPR;
-    TV acc = 0;
-    if (r < n) {
-        const int32_t a = rp[r], b = rp[r + 1];
-        for (int32_t k = a + lane; k < b; k += TPR) acc += (TV)__ldg(val + k) * __ldg(x + __ldg(col + k));
-    }
-#pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, TPR);
-    TV dv = 0;
-    if (r < n && lane == 0) {
-        const TV yv = freed[r] ? acc : (TV)0;
-        y[r] = yv;
-        dv = yv * x[r];
-    }
-    if (part) {
-        double s = block_sum(dv);
-        if (threadIdx.x == 0) part[blockIdx.x] = s;
-    }
-}
-
-// r = free ? b - Ax : 0 ; partial of |r|^2.  Also used with Ax = A x_D to get the rhs norm.
-template <class T>
-__global__ void resid_kernel(int64_t n, const double* __restrict__ b, const double* __restrict__ Ax,
-                             const uint8_t* __restrict__ freed, T* __restrict__ r, double* __restrict__ part,
-                             int nparts) {
-    double acc = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double v = freed[i] ? b[i] - Ax[i] : 0.0;
-        if (r) r[i] = (T)v;
-        acc += v * v;
-    }
-    double s = block_sum(acc);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-    (void)nparts;
-}
-
-__global__ void zero_free(int64_t n, const uint8_t* __restrict__ freed, const double* __restrict__ x,
-                          double* __restrict__ xd) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        xd[i] = freed[i] ? 0.0 : x[i];
-}
-
-template <class T>
 __global__ void jacobi_setup(int64_t n, const int32_t* __restrict__ diag, const double* __restrict__ vals,
                              const uint8_t* __restrict__ freed, T* __restrict__ dinv) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -313,123 +234,6 @@ __global__ void block_jacobi_setup(int64_t ne, const int32_t* __restrict__ rp, c
         }
 }
 
-template <class T, int L>
-__global__ void block_prec(int64_t ne, const T* __restrict__ Binv, const T* __restrict__ v, T* __restrict__ z,
-                           const int* __restrict__ flags) {
-    if (flags && flags[F_CONV]) return;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= ne * L) return;
-    const int64_t e = t / L;
-    const int i = (int)(t % L);
-    T acc = 0;
-#pragma unroll
-    for (int j = 0; j < L; j++) acc += Binv[(e * L + i) * L + j] * v[e * L + j];
-    z[t] = acc;
-}
-
-// ---- CG pieces
-template <class T>
-__global__ void cg_update(int64_t n, const double* __restrict__ st, T* __restrict__ x, T* __restrict__ r,
-                          const T* __restrict__ p, const T* __restrict__ q, const T* __restrict__ dinv,
-                          T* __restrict__ z, double* __restrict__ part, int nb, const int* __restrict__ flags) {
-    if (flags[F_CONV]) return;
-    const T alpha = (T)st[S_ALPHA];
-    T rz = 0, rr = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        const T ri = r[i] - alpha * q[i];
-        r[i] = ri;
-        const T zi = dinv[i] * ri;
-        z[i] = zi;
-        rz += ri * zi;
-        rr += ri * ri;
-    }
-    double s1 = block_sum(rz);
-    if (threadIdx.x == 0) part[blockIdx.x] = s1;
-    double s2 = block_sum(rr);
-    if (threadIdx.x == 0) part[nb + blockIdx.x] = s2;
-}
-
-template <class T>
-__global__ void cg_pupdate(int64_t n, const double* __restrict__ st, const T* __restrict__ z, T* __restrict__ p,
-                           const int* __restrict__ flags) {
-    if (flags[F_CONV]) return;
-    const T beta = (T)st[S_SCALE];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = z[i] + beta * p[i];
-}
-
-template <class T>
-__global__ void cg_init(int64_t n, const T* __restrict__ r, const T* __restrict__ dinv, T* __restrict__ z,
-                        T* __restrict__ p, double* __restrict__ part, int nb) {
-    T rz = 0, rr = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const T zi = dinv[i] * r[i];
-        z[i] = zi;
-        p[i] = zi;
-        rz += r[i] * zi;
-        rr += r[i] * r[i];
-    }
-    double s1 = block_sum(rz);
-    if (threadIdx.x == 0) part[blockIdx.x] = s1;
-    double s2 = block_sum(rr);
-    if (threadIdx.x == 0) part[nb + blockIdx.x] = s2;
-}
-
-__global__ void cg_scalars_init(const double* __restrict__ red, double* st, int* flags) {
-    st[S_RZ] = red[0];
-    const double res = sqrt(fmax(red[1], 0.0)) / st[S_NB];
-    st[S_RES] = res;
-    flags[F_CONV] = res <= st[S_TOL] ? 1 : 0;
-    if (!isfinite(res)) {
-        flags[F_NONFIN] = 1;
-        flags[F_CONV] = 1;
-    }
-}
-__global__ void cg_alpha(const double* __restrict__ red, double* st, int* flags) {
-    if (flags[F_CONV]) return;
-    const double pq = red[0];
-    if (pq == 0.0 || !isfinite(pq)) {
-        flags[pq == 0.0 ? F_BREAK : F_NONFIN] = 1;
-        flags[F_CONV] = 1;
-        st[S_ALPHA] = 0;
-        return;
-    }
-    st[S_ALPHA] = st[S_RZ] / pq;
-}
-__global__ void cg_beta(const double* __restrict__ red, double* st, int* flags) {
-    if (flags[F_CONV]) return;
-    const double rz1 = red[0];
-    st[S_SCALE] = st[S_RZ] != 0.0 ? rz1 / st[S_RZ] : 0.0;
-    st[S_RZ] = rz1;
-    const double res = sqrt(fmax(red[1], 0.0)) / st[S_NB];
-    st[S_RES] = res;
-    flags[F_ITERS] += 1;
-    if (!isfinite(res)) {
-        flags[F_NONFIN] = 1;
-        flags[F_CONV] = 1;
-    } else if (res <= st[S_TOL])
-        flags[F_CONV] = 1;
-}
-
-__global__ void set_state(double* st, int slot, double v) { st[slot] = v; }
-__global__ void set_nb_from(const double* __restrict__ red, double* st) {
-    const double nb = sqrt(fmax(red[0], 0.0));
-    st[S_NB] = nb > 0 ? nb : 1.0;
-}
-__global__ void scale_to_float(int64_t n, const double* __restrict__ r, const double* __restrict__ st,
-                               float* __restrict__ r32) {
-    const double inv = st[S_BETA] > 0 ? 1.0 / st[S_BETA] : 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        r32[i] = (float)(r[i] * inv);
-}
-__global__ void add_scaled_float(int64_t n, const float* __restrict__ d, const double* __restrict__ st,
-                                 double* __restrict__ x) {
-    const double s = st[S_BETA];
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] += s * (double)d[i];
-}
-
 // ------------------------------------------------------------------ host-side drivers
 struct Ctx {
     ocmp_solver_s* sv;
@@ -446,54 +250,6 @@ int pick_tpr(const ocmp_space_s* s) {
     return 16;
 }
 
-template <class TM, class TV>
-void launch_spmv_masked(const Ctx& c, const TM* vals, const TV* x, TV* y, double* part, const int* flags) {
-    const ocmp_space_s* s = c.sv->s;
-    const int64_t n = s->ndof;
-    switch (c.tpr) {
-    case 2: OCMP_LAUNCH(spmv_masked<TM, TV, 2><<<nblk(n * 2, kThreads), kThreads, 0, c.st>>>(n, s->d_rowptr, s->d_col, vals, s->d_free, x, y, part, flags)); break;
-    case 4: OCMP_LAUNCH(spmv_masked<TM, TV, 4><<<nblk(n * 4, kThreads), kThreads, 0, c.st>>>(n, s->d_rowptr, s->d_col, vals, s->d_free, x, y, part, flags)); break;
-    case 8: OCMP_LAUNCH(spmv_masked<TM, TV, 8><<<nblk(n * 8, kThreads), kThreads, 0, c.st>>>(n, s->d_rowptr, s->d_col, vals, s->d_free, x, y, part, flags)); break;
-    default: OCMP_LAUNCH(spmv_masked<TM, TV, 16><<<nblk(n * 16, kThreads), kThreads, 0, c.st>>>(n, s->d_rowptr, s->d_col, vals, s->d_free, x, y, part, flags)); break;
-    }
-}
-inline int spmv_blocks(const Ctx& c) { return (int)nblk(c.sv->s->ndof * c.tpr, kThreads); }
-
-template <class T>
-void launch_block_prec(const Ctx& c, const T* Binv, const T* v, T* z, const int* flags) {
-    const ocmp_space_s* s = c.sv->s;
-    const int64_t ne = s->mesh->ne;
-    switch (s->nloc) {
-    case 3: OCMP_LAUNCH(block_prec<T, 3><<<nblk(ne * 3, kThreads), kThreads, 0, c.st>>>(ne, Binv, v, z, flags)); break;
-    case 6: OCMP_LAUNCH(block_prec<T, 6><<<nblk(ne * 6, kThreads), kThreads, 0, c.st>>>(ne, Binv, v, z, flags)); break;
-    case 10: OCMP_LAUNCH(block_prec<T, 10><<<nblk(ne * 10, kThreads), kThreads, 0, c.st>>>(ne, Binv, v, z, flags)); break;
-    default: break;
-    }
-}
-
-// ||(b - A x_D)_free||: the norm the relative residual is measured against
-int rhs_norm(const Ctx& c, const double* b, const double* x) {
-    ocmp_solver_s* sv = c.sv;
-    const int64_t n = sv->n;
-    OCMP_LAUNCH(zero_free<<<c.grid, kThreads, 0, c.st>>>(n, sv->s->d_free, x, sv->z));
-    launch_spmv64(sv->s, sv->mat->vals, sv->z, sv->w, c.st);
-    OCMP_LAUNCH(resid_kernel<double><<<sv->nb, kThreads, 0, c.st>>>(n, b, sv->w, sv->s->d_free, (double*)nullptr, sv->part, sv->nb));
-    OCMP_LAUNCH(reduce_kernel<<<1, kThreads, 0, c.st>>>(sv->nb, 1, sv->part, sv->red, nullptr, -1));
-    OCMP_LAUNCH(set_nb_from<<<1, 1, 0, c.st>>>(sv->red, sv->st));
-    OCMP_CUDA(cudaGetLastError());
-    return OCMP_OK;
-}
-
-// FP64 residual r = (b - A x)_free into dst (double or float-scaled), |r|^2 into red[0]
-int residual64(const Ctx& c, const double* b, const double* x, double* dst) {
-    ocmp_solver_s* sv = c.sv;
-    launch_spmv64(sv->s, sv->mat->vals, x, sv->w, c.st);
-    OCMP_LAUNCH(resid_kernel<double><<<sv->nb, kThreads, 0, c.st>>>(sv->n, b, sv->w, sv->s->d_free, dst, sv->part, sv->nb));
-    OCMP_LAUNCH(reduce_kernel<<<1, kThreads, 0, c.st>>>(sv->nb, 1, sv->part, sv->red, nullptr, -1));
-    OCMP_CUDA(cudaGetLastError());
-    return OCMP_OK;
-}
-
 int read_flags(const Ctx& c) {
     OCMP_CUDA(cudaMemcpyAsync(c.sv->hflags, c.sv->flags, sizeof(int) * F_NFLAG * c.sv->B, cudaMemcpyDeviceToHost,
                               c.st));
@@ -503,38 +259,34 @@ int read_flags(const Ctx& c) {
 
 // GMRES lives in the fused section below (gm_*).
 
-template <class T, class TM, class TX>
-int cg_core(const Ctx& c, const TM* vals, const T* dinv, T* r, T* z, T* p, T* q, TX* x, int maxit, double tol,
-            int* iters_out) {
-    ocmp_solver_s* sv = c.sv;
-    const int64_t n = sv->n;
-    OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_TOL, tol));
-    OCMP_CUDA(cudaMemsetAsync(sv->flags, 0, sizeof(int) * F_NFLAG, c.st));
-    OCMP_LAUNCH(cg_init<T><<<sv->nb, kThreads, 0, c.st>>>(n, r, dinv, z, p, sv->part, sv->nb));
-    OCMP_LAUNCH(reduce_kernel<<<2, kThreads, 0, c.st>>>(sv->nb, 2, sv->part, sv->red, nullptr, -1));
-    OCMP_LAUNCH(cg_scalars_init<<<1, 1, 0, c.st>>>(sv->red, sv->st, sv->flags));
-    int it = 0;
-    if (read_flags(c)) return OCMP_ERR_CUDA;
-    if (!sv->hflags[F_CONV]) {
-        const int nbs = spmv_blocks(c);
-        while (it < maxit) {
-            launch_spmv_masked<TM, T>(c, vals, p, q, sv->pspmv, sv->flags);
-            OCMP_LAUNCH(reduce_kernel<<<1, kThreads, 0, c.st>>>(nbs, 1, sv->pspmv, sv->red, nullptr, -1));
-            OCMP_LAUNCH(cg_alpha<<<1, 1, 0, c.st>>>(sv->red, sv->st, sv->flags));
-            OCMP_LAUNCH(cg_update<T><<<sv->nb, kThreads, 0, c.st>>>(n, sv->st, x, r, p, q, dinv, z, sv->part, sv->nb, sv->flags));
-            OCMP_LAUNCH(reduce_kernel<<<2, kThreads, 0, c.st>>>(sv->nb, 2, sv->part, sv->red, sv->flags, -1));
-            OCMP_LAUNCH(cg_beta<<<1, 1, 0, c.st>>>(sv->red, sv->st, sv->flags));
-            OCMP_LAUNCH(cg_pupdate<T><<<c.grid, kThreads, 0, c.st>>>(n, sv->st, z, p, sv->flags));
-            it++;
-            if ((it % std::max(1, sv->prm.check_every)) == 0 || it >= maxit) {
-                if (read_flags(c)) return OCMP_ERR_CUDA;
-                if (sv->hflags[F_CONV]) break;
-            }
-        }
+// The whole CG solve in one cooperative launch. Rows per block of a small system: up to kCgOneBlock rows
+// one block does all of it (its barrier is a __syncthreads); above, a block per tile of rows up to one
+// per SM. fusep: see ocmp_cg.cuh.
+constexpr int64_t kCgOneBlock = 512;
+constexpr int64_t kCgFuseNnz = 4096;   // matrix entries per block up to which the third barrier is saved
+
+template <class T>
+int cg_solve(const CgArgs<T>& args, const ocmp_space_s* s, bool can_fuse, cudaStream_t st, CgResult* out) {
+    CgArgs<T> a = args;
+    const int tpr = pick_tpr(s), rt = kCgThreads / tpr;
+    int dev = 0, sms = 152;
+    OCMP_CUDA(cudaGetDevice(&dev));
+    OCMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t tiles = (a.n + rt - 1) / rt;
+    const int grid = a.n <= kCgOneBlock ? 1 : (int)std::min<int64_t>(sms, tiles);
+    a.fusep = can_fuse && grid > 1 && s->nnz <= kCgFuseNnz * grid;
+    const void* k = tpr == 2   ? (const void*)cg_solve_kernel<T, 2>
+                    : tpr == 4 ? (const void*)cg_solve_kernel<T, 4>
+                    : tpr == 8 ? (const void*)cg_solve_kernel<T, 8>
+                               : (const void*)cg_solve_kernel<T, 16>;
+    void* kp[] = {&a};
+    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kCgThreads), kp, 0, st)));
+    OCMP_CUDA(cudaMemcpyAsync(out, a.out, sizeof(CgResult), cudaMemcpyDeviceToHost, st));
+    OCMP_CUDA(cudaStreamSynchronize(st));
+    if (out->team.abort) {
+        OCMP_CUDA(cudaMemsetAsync(&a.out->team, 0, sizeof(TeamState), st));
+        return fail(OCMP_TIMEOUT, "CG: a block gave up waiting for the others");
     }
-    OCMP_CUDA(cudaGetLastError());
-    if (read_flags(c)) return OCMP_ERR_CUDA;
-    *iters_out = sv->hflags[F_ITERS];
     return OCMP_OK;
 }
 
@@ -1541,7 +1293,7 @@ using namespace ocmp;
 
 static void free_solver(ocmp_solver_s* sv) {
     void* ps[] = {sv->udiag, sv->dinv, sv->Binv, sv->V,   sv->w,     sv->z,   sv->r,     sv->p,    sv->dinv32, sv->Binv32,
-                  sv->V32,  sv->w32,  sv->z32, sv->r32,   sv->p32, sv->d32,   sv->part, sv->pspmv,  sv->red,
+                  sv->V32,  sv->w32,  sv->z32, sv->r32,   sv->p32, sv->d32,   sv->pb,   sv->p32b,  sv->dcg, sv->part, sv->red,
                   sv->st,   sv->H,    sv->flags, sv->As64, sv->As32, sv->scale, sv->cnt};
     for (void* q : ps) dfree(q);
     if (sv->strip) strip_destroy(sv->strip);
@@ -1554,6 +1306,7 @@ static void free_solver(ocmp_solver_s* sv) {
         delete sv->cc;
     }
     if (sv->hflags) cudaFreeHost(sv->hflags);
+    if (sv->hcg) cudaFreeHost(sv->hcg);
     if (sv->gexec) cudaGraphExecDestroy(sv->gexec);
     if (sv->gstream) cudaStreamDestroy(sv->gstream);
     for (cudaEvent_t e : sv->tev) cudaEventDestroy(e);
@@ -1641,7 +1394,10 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
     A(&sv->r, n);
     if (!mixed) {
         if (gm) A(&sv->V, (size_t)(m + 1) * n * NB);
-        else A(&sv->p, n);
+        else {
+            A(&sv->p, n);
+            A(&sv->pb, n);
+        }
     }
     if (blk) A(&sv->Binv, (size_t)s->mesh->ne * s->nloc * s->nloc);
     if (!st && prm->precond == OCMP_PRE_STRIP) st = strip_create(s, &sv->strip);
@@ -1654,11 +1410,17 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
         else {
             A(&sv->r32, n);
             A(&sv->p32, n);
+            A(&sv->p32b, n);
         }
         if (blk) A(&sv->Binv32, (size_t)s->mesh->ne * s->nloc * s->nloc);
     }
     A(&sv->part, (size_t)std::max<int64_t>((int64_t)(m + 4) * kGridCap, (int64_t)(m + 4) * sv->grid * NB));
-    A(&sv->pspmv, (size_t)nbs);
+    if (!gm) {
+        A(&sv->dcg, 1);
+        if (!st && cudaMemset(sv->dcg, 0, sizeof(CgResult)) != cudaSuccess) st = fail(OCMP_ERR_CUDA, "cudaMemset");
+        if (!st && cudaMallocHost((void**)&sv->hcg, sizeof(CgResult)) != cudaSuccess)
+            st = fail(OCMP_ERR_NOMEM, "cudaMallocHost");
+    }
     A(&sv->red, (size_t)(3 * m + 12) * NB);
     A(&sv->st, (size_t)S_NSLOT * NB);
     A(&sv->H, (size_t)hsz * NB);
@@ -1993,64 +1755,25 @@ int ocmp_solve(ocmp_solver_t sv, const double* b, double* x, void* stream, ocmp_
         }
         sv->tev_used = 0;
     } else {
-        st = rhs_norm(c, b, x);
-        if (st) return st;
-        st = residual64(c, b, x, sv->r);
-        if (st) return st;
-        double red0 = 0;
-        OCMP_CUDA(cudaMemcpyAsync(&red0, sv->red, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-        OCMP_CUDA(cudaMemcpyAsync(hst, sv->st, sizeof(hst), cudaMemcpyDeviceToHost, c.st));
-        OCMP_CUDA(cudaStreamSynchronize(c.st));
-        const double nbv = hst[S_NB];
-        relres0 = std::sqrt(std::max(red0, 0.0)) / nbv;
-        nonfin = !std::isfinite(relres0);
-        if (!nonfin && relres0 > P.tol) {
-            if (!mixed) {
-                st = cg_core<double, double, double>(c, sv->mat->vals, sv->dinv, sv->r, sv->z, sv->p, sv->w, x,
-                                                     P.maxit, P.tol, &iters);
-                if (st) return st;
-                nonfin = sv->hflags[F_NONFIN] != 0;
-                brk = sv->hflags[F_BREAK] != 0;
-            } else {
-                double beta = std::sqrt(std::max(red0, 0.0));
-                while (iters < P.maxit) {
-                    OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_BETA, beta));
-                    OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_NB, 1.0));
-                    const double itol = std::max(P.inner_tol > 0 ? P.inner_tol : 1e-4, kTargetMargin * P.tol * nbv / beta);
-                    OCMP_CUDA(cudaMemsetAsync(sv->d32, 0, sizeof(float) * n, c.st));
-                    int it_in = 0;
-                    OCMP_LAUNCH(scale_to_float<<<c.grid, kThreads, 0, c.st>>>(n, sv->r, sv->st, sv->r32));
-                    st = cg_core<float, float, float>(c, sv->mat->vals32, sv->dinv32, sv->r32, sv->z32, sv->p32,
-                                                      sv->w32, sv->d32, P.maxit - iters, itol, &it_in);
-                    if (st) return st;
-                    iters += std::max(it_in, 1);
-                    outer++;
-                    if (sv->hflags[F_NONFIN]) {
-                        nonfin = true;
-                        break;
-                    }
-                    OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_BETA, beta));
-                    OCMP_LAUNCH(add_scaled_float<<<c.grid, kThreads, 0, c.st>>>(n, sv->d32, sv->st, x));
-                    OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_NB, nbv));
-                    st = residual64(c, b, x, sv->r);
-                    if (st) return st;
-                    OCMP_CUDA(cudaMemcpyAsync(&red0, sv->red, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-                    OCMP_CUDA(cudaStreamSynchronize(c.st));
-                    beta = std::sqrt(std::max(red0, 0.0));
-                    if (!std::isfinite(beta)) {
-                        nonfin = true;
-                        break;
-                    }
-                    if (beta / nbv <= P.tol) break;
-                }
-            }
+        CgResult& R = *sv->hcg;
+        if (mixed) {
+            CgArgs<float> a{n, sv->s->d_rowptr, sv->s->d_col, sv->mat->vals, sv->mat->vals32, sv->s->d_free, sv->s->d_lift_ptr,
+                            sv->s->d_lift_pos, sv->dinv32, b, x, sv->r, sv->r32, sv->z32, sv->p32, sv->p32b, sv->w32, sv->d32,
+                            sv->part, sv->dcg, P.tol, P.inner_tol > 0 ? P.inner_tol : 1e-4, kTargetMargin, P.maxit, 0};
+            st = cg_solve(a, sv->s, true, c.st, &R);
+        } else {
+            CgArgs<double> a{n, sv->s->d_rowptr, sv->s->d_col, sv->mat->vals, sv->mat->vals, sv->s->d_free, sv->s->d_lift_ptr,
+                             sv->s->d_lift_pos, sv->dinv, b, x, nullptr, sv->r, sv->z, sv->p, sv->pb, sv->w, nullptr,
+                             sv->part, sv->dcg, P.tol, 0.0, kTargetMargin, P.maxit, 0};
+            st = cg_solve(a, sv->s, true, c.st, &R);
         }
-        OCMP_LAUNCH(set_state<<<1, 1, 0, c.st>>>(sv->st, S_NB, nbv));
-        st = residual64(c, b, x, (double*)nullptr);
         if (st) return st;
-        OCMP_CUDA(cudaMemcpyAsync(&red0, sv->red, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-        OCMP_CUDA(cudaStreamSynchronize(c.st));
-        relres = std::sqrt(std::max(red0, 0.0)) / nbv;
+        relres0 = R.res0;
+        relres = R.res;
+        iters = R.iters;
+        outer = R.outer;
+        nonfin = (R.bits & CG_NONFIN) != 0;
+        brk = (R.bits & CG_BREAK) != 0;
     }
     int status = OCMP_OK;
     if (nonfin || !std::isfinite(relres)) status = OCMP_ERR_NONFINITE;
@@ -2300,70 +2023,30 @@ extern "C" int ocmp_solve_cg_noalloc(ocmp_matrix_t mat, const double* b, double*
     if (n > kNoAllocMaxN)
         return fail(OCMP_ERR_ARG, "ocmp_solve_cg_noalloc: " + std::to_string(n) + " dofs exceed the " +
                                       std::to_string(kNoAllocMaxN) + "-dof limit of its static workspace");
-    const int tpr = pick_tpr(s);
-    if ((n * tpr + kThreads - 1) / kThreads > kNoAllocRed)
-        return fail(OCMP_ERR_ARG, "ocmp_solve_cg_noalloc: SpMV partials exceed the static workspace");
     double* scr = nullptr;
     int* flg = nullptr;
     int st = noalloc_scratch(&scr, &flg);
     if (st) return st;
-    // A solver view over the static workspace: nothing here touches the allocator.
-    ocmp_solver_s sv;
-    sv.mat = mat;
-    sv.s = s;
-    sv.prm.method = OCMP_CG;
-    sv.prm.precond = OCMP_PRE_JACOBI;
-    sv.prm.precision = OCMP_FP64;
-    sv.prm.tol = tol;
-    sv.prm.maxit = maxit;
-    sv.prm.check_every = 8;
-    sv.n = n;
-    sv.m = 1;
-    sv.nb = (int)std::max<int64_t>(1, std::min<int64_t>(1216, (n + 1023) / 1024));
-    sv.dinv = scr;
-    sv.r = scr + n;
-    sv.z = scr + 2 * n;
-    sv.p = scr + 3 * n;
-    sv.w = scr + 4 * n;
-    double* tail = scr + 5 * kNoAllocMaxN;
-    sv.pspmv = tail;
-    sv.part = tail;  // CG partials (2 x nb) never overlap a live SpMV partial
-    sv.red = tail + kNoAllocRed;
-    sv.st = sv.red + 64;
-    sv.flags = flg;
-    int hflags[F_NFLAG] = {0};
-    sv.hflags = hflags;
-    Ctx c;
-    c.sv = &sv;
-    c.st = (cudaStream_t)stream;
-    c.tpr = tpr;
-    c.grid = sv.nb;
-    // the workspace keeps the previous call's contents: reset the flags and scalars
-    OCMP_CUDA(cudaMemsetAsync(flg, 0, sizeof(int) * 64, c.st));
-    OCMP_CUDA(cudaMemsetAsync(sv.red, 0, sizeof(double) * kNoAllocState, c.st));
-    OCMP_LAUNCH(jacobi_setup<double><<<nblk(n, kThreads), kThreads, 0, c.st>>>(n, s->d_diag, mat->vals, s->d_free, sv.dinv));
-    st = rhs_norm(c, b, x);
+    // the search direction's second buffer fits beside the other five vectors unless the system is one of
+    // the largest, which do not use it
+    cudaStream_t cst = (cudaStream_t)stream;
+    double *dinv = scr, *r = scr + n, *z = scr + 2 * n, *p = scr + 3 * n, *w = scr + 4 * n, *pb = scr + 5 * n;
+    const bool two = 6 * n <= 5 * kNoAllocMaxN;
+    auto* dres = reinterpret_cast<CgResult*>(flg);
+    static_assert(sizeof(CgResult) <= 64 * sizeof(int), "results of the allocation-free CG");
+    // the workspace keeps the previous call's contents: reset the barrier's state
+    OCMP_CUDA(cudaMemsetAsync(flg, 0, sizeof(int) * 64, cst));
+    OCMP_LAUNCH(jacobi_setup<double><<<nblk(n, kThreads), kThreads, 0, cst>>>(n, s->d_diag, mat->vals, s->d_free, dinv));
+    OCMP_CUDA(cudaGetLastError());
+    CgArgs<double> a{n, s->d_rowptr, s->d_col, mat->vals, mat->vals, s->d_free, s->d_lift_ptr, s->d_lift_pos, dinv, b, x,
+                     nullptr, r, z, p, two ? pb : p, w, nullptr, scr + 5 * kNoAllocMaxN, dres, tol, 0.0, kTargetMargin,
+                     maxit, 0};
+    CgResult R{};
+    st = cg_solve(a, s, two, cst, &R);
     if (st) return st;
-    st = residual64(c, b, x, sv.r);
-    if (st) return st;
-    double red0 = 0, nbv = 1;
-    OCMP_CUDA(cudaMemcpyAsync(&red0, sv.red, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    OCMP_CUDA(cudaMemcpyAsync(&nbv, sv.st + S_NB, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    OCMP_CUDA(cudaStreamSynchronize(c.st));
-    const double relres0 = std::sqrt(std::max(red0, 0.0)) / nbv;
-    int iters = 0;
-    bool nonfin = !std::isfinite(relres0), brk = false;
-    if (!nonfin && relres0 > tol) {
-        st = cg_core<double, double, double>(c, mat->vals, sv.dinv, sv.r, sv.z, sv.p, sv.w, x, maxit, tol, &iters);
-        if (st) return st;
-        nonfin = hflags[F_NONFIN] != 0;
-        brk = hflags[F_BREAK] != 0;
-    }
-    st = residual64(c, b, x, (double*)nullptr);
-    if (st) return st;
-    OCMP_CUDA(cudaMemcpyAsync(&red0, sv.red, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    OCMP_CUDA(cudaStreamSynchronize(c.st));
-    const double relres = std::sqrt(std::max(red0, 0.0)) / nbv;
+    const double relres0 = R.res0, relres = R.res;
+    const int iters = R.iters;
+    const bool nonfin = (R.bits & CG_NONFIN) != 0, brk = (R.bits & CG_BREAK) != 0;
     int status = OCMP_OK;
     if (nonfin || !std::isfinite(relres)) status = OCMP_ERR_NONFINITE;
     else if (relres > tol) status = brk ? OCMP_BREAKDOWN : OCMP_NOT_CONVERGED;
