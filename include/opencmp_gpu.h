@@ -126,7 +126,7 @@ typedef struct {
     double inner_tol;        /* mixed: relative reduction asked of each inner solve               */
     int32_t check_every;     /* host reads the convergence flag every k iterations (>= 1; 0: 8); -1:
                                 GMRES checks first one iteration before the previous solve's count,
-                                then after every iteration                                          */
+                                then after every iteration. CG runs in one launch and ignores it     */
 } ocmp_solve_params_t;
 
 typedef struct {
@@ -443,10 +443,10 @@ int ocmp_spmv_transpose(ocmp_matrix_t mat, const double* x_dev, double* y_dev, v
  * matrices (B > 1) with OCMP_ERR_UNSUPPORTED. The first call on each device looks up that array's
  * device address (cudaGetSymbolAddress) with the device current. All calls share the one workspace
  * and it keeps the last call's contents (each call resets what must start at zero): calls whose
- * work overlaps on the GPU (different streams or threads) race, so serialise them. The host reads
- * the convergence flags every 8 iterations through a blocking copy into its own stack memory (no
- * pinned buffer is allocated for it), and the call returns OCMP_ERR_UNSUPPORTED on a stream that is
- * being captured, since those reads would invalidate the capture. */
+ * work overlaps on the GPU (different streams or threads) race, so serialise them. The host waits for
+ * the result through a blocking copy into its own stack memory (no pinned buffer is allocated for
+ * it), and the call returns OCMP_ERR_UNSUPPORTED on a stream that is being captured, since that wait
+ * would invalidate the capture. */
 #define OCMP_NOALLOC_MAX_NDOF 1048576
 int ocmp_solve_cg_noalloc(ocmp_matrix_t mat, const double* b_dev, double* x_dev, double tol, int32_t maxit,
                           void* stream, ocmp_solve_info_t* info);

@@ -55,6 +55,15 @@ static void parallel_for(int64_t n, const std::function<void(int64_t, int64_t)>&
     for (auto& x : th) x.join();
 }
 
+void set_slice_width(ocmp_space_s* s) {
+    const int64_t n = s->ndof, ns = (n + 31) / 32;
+    s->slice_width.assign(ns, 0);
+    for (int64_t r = 0; r < n; r++) {
+        uint16_t& w = s->slice_width[r / 32];
+        w = std::max(w, (uint16_t)std::min<int64_t>(0xffff, s->rowptr[r + 1] - s->rowptr[r]));
+    }
+}
+
 // ---------------------------------------------------------------- reference basis (host)
 struct Dn {
     double v, d[3];
@@ -777,6 +786,7 @@ int ocmp_space_create(ocmp_mesh_t mesh, int32_t kind, int32_t order, uint32_t di
     // ---- slot tables: for element e and local row i, the position within CSR row dof(e,i) of
     // each column dof(e,j); the same for the 2L columns of every interior-facet matrix row (L2).
     for (int64_t r = 0; r < nd; r++) s->maxrow = std::max<int>(s->maxrow, (int)(rl[r + 1] - rl[r]));
+    set_slice_width(s);
     s->row_ranges = {0};
     if (kind == OCMP_H1 && p >= 2 && nv < nd) s->row_ranges.push_back(nv);
     s->row_ranges.push_back(nd);

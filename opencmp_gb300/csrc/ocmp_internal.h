@@ -120,6 +120,7 @@ struct ocmp_space_s {
     int tuned_tpr = 0, tuned_u = 0; // SpMV row configuration chosen by ocmp_matrix_autotune (0: default)
     std::vector<int64_t> row_ranges;  // row ranges of similar length (vertex rows, the rest)
     std::vector<int> range_maxrow;
+    std::vector<uint16_t> slice_width;  // longest row of each slice of 32 rows
     int32_t* d_inc_ptr = nullptr;   // ndof+1: dof -> (element, local) incidence
     int32_t* d_inc = nullptr;       // ne*nloc: e*nloc + i
     int32_t* d_ifac = nullptr;
@@ -174,6 +175,8 @@ struct ocmp_matrix_s {
 };
 
 namespace ocmp {
+// the longest row of each slice of 32 rows, from rowptr (ocmp_host.cpp)
+void set_slice_width(ocmp_space_s* s);
 // reference basis values/gradients (ocmp_host.cpp) and the collapsed simplex rule
 int tabulate(int kind, int D, int p, int npts, const double* xi, double* val, double* grad);
 int quad_rule(int D, int n, std::vector<double>& pts, std::vector<double>& wts);

@@ -104,8 +104,8 @@ struct ocmp_solver_s {
     float* d32 = nullptr;       // inner correction
     double* pb = nullptr;       // second search direction (CG)
     float* p32b = nullptr;
-    ocmp::CgResult* dcg = nullptr;   // CG: results and barrier state
-    ocmp::CgResult* hcg = nullptr;   // pinned
+    ocmp::CgState* dcg = nullptr;    // CG: results and exchange slots
+    ocmp::CgState* hcg = nullptr;    // pinned: the results and the head of the slots
     // reductions and small state
     double* part = nullptr;     // (m+4) x nb
     double* red = nullptr;      // m+2 reduced values
@@ -259,32 +259,70 @@ int read_flags(const Ctx& c) {
 
 // GMRES lives in the fused section below (gm_*).
 
-// The whole CG solve in one cooperative launch. Rows per block of a small system: up to kCgOneBlock rows
-// one block does all of it (its barrier is a __syncthreads); above, a block per tile of rows up to one
-// per SM. fusep: see ocmp_cg.cuh.
-constexpr int64_t kCgOneBlock = 512;
-constexpr int64_t kCgFuseNnz = 4096;   // matrix entries per block up to which the third barrier is saved
-
-template <class T>
-int cg_solve(const CgArgs<T>& args, const ocmp_space_s* s, bool can_fuse, cudaStream_t st, CgResult* out) {
-    CgArgs<T> a = args;
-    const int tpr = pick_tpr(s), rt = kCgThreads / tpr;
-    int dev = 0, sms = 152;
+// Blocks of the current device's SMs a team may have.
+int team_blocks(int* out) {
+    int dev = 0, sms = 0;
     OCMP_CUDA(cudaGetDevice(&dev));
     OCMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t tiles = (a.n + rt - 1) / rt;
-    const int grid = a.n <= kCgOneBlock ? 1 : (int)std::min<int64_t>(sms, tiles);
-    a.fusep = can_fuse && grid > 1 && s->nnz <= kCgFuseNnz * grid;
-    const void* k = tpr == 2   ? (const void*)cg_solve_kernel<T, 2>
-                    : tpr == 4 ? (const void*)cg_solve_kernel<T, 4>
-                    : tpr == 8 ? (const void*)cg_solve_kernel<T, 8>
-                               : (const void*)cg_solve_kernel<T, 16>;
+    *out = std::max(1, std::min(sms, kTeamMaxBlocks));
+    return OCMP_OK;
+}
+
+template <class T>
+int cg_launch(const void* k, CgArgs<T>& a, int grid, int threads, size_t smem, cudaStream_t st) {
+    if (smem) OCMP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* kp[] = {&a};
-    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kCgThreads), kp, 0, st)));
-    OCMP_CUDA(cudaMemcpyAsync(out, a.out, sizeof(CgResult), cudaMemcpyDeviceToHost, st));
+    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(threads), kp, smem, st)));
+    return OCMP_OK;
+}
+
+// The whole CG solve in one cooperative launch. Resident form: a system of few rows and entries is one
+// block's (its exchanges are __syncthreads); above, the slices of 32 rows are dealt to the SMs.
+constexpr int64_t kCgOneBlockRows = 1024, kCgOneBlockNnz = 8192;
+constexpr int64_t kCgFuseNnz = 4900;   // entries per block whose second FMA costs the barrier's 2,450 clocks
+constexpr size_t kCgSmem = 200 * 1024;
+
+template <class T>
+int cg_solve(const CgArgs<T>& args, const ocmp_space_s* s, bool two_p, cudaStream_t st, CgState* out) {
+    CgArgs<T> a = args;
+    constexpr bool D = sizeof(T) == 8;
+    int sms = 1;
+    if (const int r = team_blocks(&sms)) return r;
+    const int64_t slices = (a.n + 31) / 32;
+    int r = -1;
+    if (a.n <= (int64_t)sms * kCgRowsRes) {
+        const int grid = a.n <= kCgOneBlockRows && s->nnz <= kCgOneBlockNnz ? 1 : (int)std::min<int64_t>(sms, slices);
+        const int per = (int)((slices + grid - 1) / grid);   // slices of a block
+        int64_t cap = 0;
+        for (int b = 0; b < grid; b++) {
+            int64_t c = 0;
+            for (int64_t q = b; q < slices; q += grid) c += s->slice_width[q];
+            cap = std::max(cap, 32 * c);
+        }
+        const size_t smem = (size_t)cap * (sizeof(T) + 4) + (grid == 1 ? 2 * kCgRowsRes * sizeof(T) : 0);
+        a.cap = (int)cap;
+        a.fuse = grid > 1 && two_p && (!D || cap <= kCgFuseNnz);
+        const int threads = 32 * std::max(4, std::min(kCgThreadsRes / 32, per));
+        if (per <= kCgSlicesRes && smem <= kCgSmem)
+            r = cg_launch((const void*)cg_res_kernel<T>, a, grid, threads, smem, st);
+    }
+    if (r < 0) {
+        // few lanes per row where the FP64 pipe bounds the product
+        const double avg = (double)s->nnz / (double)s->ndof;
+        const int tpr = avg <= 14 ? (D ? 2 : 4) : avg <= 40 ? (D ? 4 : 8) : (D ? 8 : 16);
+        const int rt = kCgThreadsStream / tpr;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, (a.n + rt - 1) / rt));
+        const void* k = tpr == 2   ? (const void*)cg_stream_kernel<double, 2>
+                        : tpr == 4 ? (const void*)cg_stream_kernel<T, 4>
+                        : tpr == 8 ? (const void*)cg_stream_kernel<T, 8>
+                                   : (const void*)cg_stream_kernel<float, 16>;
+        r = cg_launch(k, a, grid, kCgThreadsStream, 0, st);
+    }
+    if (r) return r;
+    OCMP_CUDA(cudaMemcpyAsync(out, a.state, kCgReadBytes, cudaMemcpyDeviceToHost, st));
     OCMP_CUDA(cudaStreamSynchronize(st));
-    if (out->team.abort) {
-        OCMP_CUDA(cudaMemsetAsync(&a.out->team, 0, sizeof(TeamState), st));
+    if (out->t.abort) {
+        OCMP_CUDA(cudaMemsetAsync(a.state, 0, sizeof(CgState), st));
         return fail(OCMP_TIMEOUT, "CG: a block gave up waiting for the others");
     }
     return OCMP_OK;
@@ -1417,8 +1455,8 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
     A(&sv->part, (size_t)std::max<int64_t>((int64_t)(m + 4) * kGridCap, (int64_t)(m + 4) * sv->grid * NB));
     if (!gm) {
         A(&sv->dcg, 1);
-        if (!st && cudaMemset(sv->dcg, 0, sizeof(CgResult)) != cudaSuccess) st = fail(OCMP_ERR_CUDA, "cudaMemset");
-        if (!st && cudaMallocHost((void**)&sv->hcg, sizeof(CgResult)) != cudaSuccess)
+        if (!st && cudaMemset(sv->dcg, 0, sizeof(CgState)) != cudaSuccess) st = fail(OCMP_ERR_CUDA, "cudaMemset");
+        if (!st && cudaMallocHost((void**)&sv->hcg, kCgReadBytes) != cudaSuccess)
             st = fail(OCMP_ERR_NOMEM, "cudaMallocHost");
     }
     A(&sv->red, (size_t)(3 * m + 12) * NB);
@@ -1755,19 +1793,19 @@ int ocmp_solve(ocmp_solver_t sv, const double* b, double* x, void* stream, ocmp_
         }
         sv->tev_used = 0;
     } else {
-        CgResult& R = *sv->hcg;
         if (mixed) {
             CgArgs<float> a{n, sv->s->d_rowptr, sv->s->d_col, sv->mat->vals, sv->mat->vals32, sv->s->d_free, sv->s->d_lift_ptr,
                             sv->s->d_lift_pos, sv->dinv32, b, x, sv->r, sv->r32, sv->z32, sv->p32, sv->p32b, sv->w32, sv->d32,
-                            sv->part, sv->dcg, P.tol, P.inner_tol > 0 ? P.inner_tol : 1e-4, kTargetMargin, P.maxit, 0};
-            st = cg_solve(a, sv->s, true, c.st, &R);
+                            sv->dcg, P.tol, P.inner_tol > 0 ? P.inner_tol : 1e-4, kTargetMargin, P.maxit, 0};
+            st = cg_solve(a, sv->s, true, c.st, sv->hcg);
         } else {
             CgArgs<double> a{n, sv->s->d_rowptr, sv->s->d_col, sv->mat->vals, sv->mat->vals, sv->s->d_free, sv->s->d_lift_ptr,
-                             sv->s->d_lift_pos, sv->dinv, b, x, nullptr, sv->r, sv->z, sv->p, sv->pb, sv->w, nullptr,
-                             sv->part, sv->dcg, P.tol, 0.0, kTargetMargin, P.maxit, 0};
-            st = cg_solve(a, sv->s, true, c.st, &R);
+                             sv->s->d_lift_pos, sv->dinv, b, x, sv->r, sv->r, sv->z, sv->p, sv->pb, sv->w, nullptr,
+                             sv->dcg, P.tol, 0.0, kTargetMargin, P.maxit, 0};
+            st = cg_solve(a, sv->s, true, c.st, sv->hcg);
         }
         if (st) return st;
+        const CgResult& R = sv->hcg->r;
         relres0 = R.res0;
         relres = R.res;
         iters = R.iters;
@@ -1962,44 +2000,36 @@ int ocmp_group_solve(ocmp_group_t g, const double* const* b, double* const* x, v
 // whose device memory belongs to another allocator's fixed pool (cudaMalloc would take memory that
 // pool has already claimed, or fail), and loops that cannot take the implicit device-wide
 // synchronisation of cudaFree. ocmp_solve_cg_noalloc serves them: it runs the
-// same FP64 Jacobi-preconditioned CG as ocmp_solve with method OCMP_CG, but its workspace (five
-// n-vectors, reduction partials, scalars and flags) lives in the file-scope device arrays below,
+// same FP64 Jacobi-preconditioned CG as ocmp_solve with method OCMP_CG, but its workspace (the
+// vectors, the blocks' exchange slots and the results) lives in the file-scope device array below,
 // which the CUDA driver allocates once per device when this library is loaded and keeps until exit.
 // The caller passes only the assembled matrix, the right-hand side and the initial guess/result.
 namespace {
 
 constexpr int64_t kNoAllocMaxN = OCMP_NOALLOC_MAX_NDOF;      // 1,048,576 dofs
-constexpr int64_t kNoAllocRed = int64_t(1) << 17;            // reduction partials
-constexpr int64_t kNoAllocState = 256;                        // reduced values + scalars
-constexpr int64_t kNoAllocDoubles = 5 * kNoAllocMaxN + kNoAllocRed + kNoAllocState;  // 41 MiB
+constexpr int64_t kNoAllocState = int64_t(1) << 17;          // exchange slots and results (1 MiB)
+constexpr int64_t kNoAllocDoubles = 5 * kNoAllocMaxN + kNoAllocState;  // 41 MiB
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
-static __device__ __align__(256) int g_noalloc_flags[64];
 
 std::mutex g_noalloc_mu;
 double* g_noalloc_ptr[128] = {};
-int* g_noalloc_fptr[128] = {};
 
-// Device addresses of the scratch arrays for the current device. Host code must not use the
-// arrays' names as pointers (they name host-side shadows); cudaGetSymbolAddress gives the device
-// address. Done once per device, under a lock, with that device current.
-int noalloc_scratch(double** scratch, int** flags) {
+// Device address of the scratch array for the current device. Host code must not use the array's
+// name as a pointer (it names a host-side shadow); cudaGetSymbolAddress gives the device address.
+// Done once per device, under a lock, with that device current.
+int noalloc_scratch(double** scratch) {
     int dev = 0;
     OCMP_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 128) return fail(OCMP_ERR_ARG, "ocmp_solve_cg_noalloc: device index out of range");
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_ptr[dev]) {
         double* p = nullptr;
-        int* f = nullptr;
         cudaError_t e = cudaGetSymbolAddress((void**)&p, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-        e = cudaGetSymbolAddress((void**)&f, g_noalloc_flags);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_flags)");
         g_noalloc_ptr[dev] = p;
-        g_noalloc_fptr[dev] = f;
     }
     *scratch = g_noalloc_ptr[dev];
-    *flags = g_noalloc_fptr[dev];
     return OCMP_OK;
 }
 
@@ -2010,8 +2040,8 @@ extern "C" int ocmp_solve_cg_noalloc(ocmp_matrix_t mat, const double* b, double*
     if (!mat || !b || !x) return fail(OCMP_ERR_ARG, "ocmp_solve_cg_noalloc: null argument");
     if (mat->B != 1) return fail(OCMP_ERR_UNSUPPORTED, "ocmp_solve_cg_noalloc: batched matrices are not supported");
     {
-        // the solve reads its convergence flags on the host (stream synchronisation, device-to-host
-        // copies); on a stream under capture those calls would invalidate the caller's capture
+        // the solve waits for its result on the host (device-to-host copy, stream synchronisation); on a
+        // stream under capture those calls would invalidate the caller's capture
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         OCMP_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &cs));
         if (cs != cudaStreamCaptureStatusNone)
@@ -2024,26 +2054,24 @@ extern "C" int ocmp_solve_cg_noalloc(ocmp_matrix_t mat, const double* b, double*
         return fail(OCMP_ERR_ARG, "ocmp_solve_cg_noalloc: " + std::to_string(n) + " dofs exceed the " +
                                       std::to_string(kNoAllocMaxN) + "-dof limit of its static workspace");
     double* scr = nullptr;
-    int* flg = nullptr;
-    int st = noalloc_scratch(&scr, &flg);
+    int st = noalloc_scratch(&scr);
     if (st) return st;
-    // the search direction's second buffer fits beside the other five vectors unless the system is one of
-    // the largest, which do not use it
+    // the second search direction fits beside the other five vectors in every system of the resident form
     cudaStream_t cst = (cudaStream_t)stream;
     double *dinv = scr, *r = scr + n, *z = scr + 2 * n, *p = scr + 3 * n, *w = scr + 4 * n, *pb = scr + 5 * n;
     const bool two = 6 * n <= 5 * kNoAllocMaxN;
-    auto* dres = reinterpret_cast<CgResult*>(flg);
-    static_assert(sizeof(CgResult) <= 64 * sizeof(int), "results of the allocation-free CG");
-    // the workspace keeps the previous call's contents: reset the barrier's state
-    OCMP_CUDA(cudaMemsetAsync(flg, 0, sizeof(int) * 64, cst));
+    // results and exchange slots follow the vectors; the workspace keeps the previous call's contents
+    auto* state = reinterpret_cast<CgState*>(scr + 5 * kNoAllocMaxN);
+    static_assert(sizeof(CgState) <= kNoAllocState * sizeof(double), "state of the CG");
+    OCMP_CUDA(cudaMemsetAsync(state, 0, sizeof(CgState), cst));
     OCMP_LAUNCH(jacobi_setup<double><<<nblk(n, kThreads), kThreads, 0, cst>>>(n, s->d_diag, mat->vals, s->d_free, dinv));
     OCMP_CUDA(cudaGetLastError());
     CgArgs<double> a{n, s->d_rowptr, s->d_col, mat->vals, mat->vals, s->d_free, s->d_lift_ptr, s->d_lift_pos, dinv, b, x,
-                     nullptr, r, z, p, two ? pb : p, w, nullptr, scr + 5 * kNoAllocMaxN, dres, tol, 0.0, kTargetMargin,
-                     maxit, 0};
-    CgResult R{};
-    st = cg_solve(a, s, two, cst, &R);
+                     r, r, z, p, two ? pb : p, w, nullptr, state, tol, 0.0, kTargetMargin, maxit, 0};
+    CgState H;
+    st = cg_solve(a, s, two, cst, &H);
     if (st) return st;
+    const CgResult& R = H.r;
     const double relres0 = R.res0, relres = R.res;
     const int iters = R.iters;
     const bool nonfin = (R.bits & CG_NONFIN) != 0, brk = (R.bits & CG_BREAK) != 0;

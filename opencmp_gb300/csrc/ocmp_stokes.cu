@@ -432,6 +432,7 @@ int th_build(ocmp_th_s* th) {
     int maxrow = 0;
     for (int64_t r = 0; r < nd; r++) maxrow = std::max(maxrow, (int)(C->rowptr[r + 1] - C->rowptr[r]));
     C->maxrow = maxrow;
+    set_slice_width(C);
 
     // ---- contribution lists: for each CSR entry, the element entries that sum into it
     auto pos = [&](int64_t r, int64_t c) -> int64_t {

@@ -45,8 +45,8 @@ def _problem(dim, n, order, mixed=False, seed=0):
     return sp, A, b, x0
 
 
-@pytest.mark.parametrize('dim,n,order', [(2, 1, 1), (2, 2, 1), (2, 21, 1), (2, 22, 1), (2, 8, 3), (2, 30, 2), (3, 9, 2),
-                                         (3, 4, 3)])
+@pytest.mark.parametrize('dim,n,order', [(2, 1, 1), (2, 2, 1), (2, 21, 1), (2, 22, 1), (2, 8, 3), (2, 24, 2), (3, 5, 2),
+                                         (3, 3, 3), (2, 33, 1)])
 @pytest.mark.parametrize('precision', ['fp64', 'mixed'])
 def test_cg_in_one_launch(gpu_lib, dim, n, order, precision):
     from opencmp_gb300 import fem
