@@ -257,6 +257,9 @@ __global__ void __launch_bounds__(kCgThreadsRes, 1) cg_res_kernel(CgArgs<T> a) {
                 else if (!MIX) o.brk = true;
                 break;
             }
+            // a step against the descent direction: the FP32 matrix is not definite (a mode the rounded
+            // values do not resolve). What was reached is kept, and refined from its true residual.
+            if (MIX && pap * rz <= 0) break;
             if (tid == 0) s_scal = rz / pap;
             __syncthreads();
             // x += alpha p, r -= alpha q, z, r . z, |r|^2
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(kCgThreadsRes, 1) cg_res_kernel(CgArgs<T> a) {
         }
         if (in_nonfin) o.nonfin = true;
         o.iters += MIX ? max(it, 1) : it;
+        if (MIX && it == 0) o.run = false;   // no step could be taken
         if (MIX) o.outer++;
         else o.run = false;
         if (MIX && in_nonfin) break;
@@ -388,6 +392,9 @@ __global__ void __launch_bounds__(kCgThreadsStream, 1) cg_stream_kernel(CgArgs<T
                 else if (!MIX) o.brk = true;
                 break;
             }
+            // a step against the descent direction: the FP32 matrix is not definite (a mode the rounded
+            // values do not resolve). What was reached is kept, and refined from its true residual.
+            if (MIX && pap * rz <= 0) break;
             if (tid == 0) s_scal = rz / pap;
             __syncthreads();
             // x += alpha p, r -= alpha q, z, r . z, |r|^2
@@ -421,6 +428,7 @@ __global__ void __launch_bounds__(kCgThreadsStream, 1) cg_stream_kernel(CgArgs<T
         }
         if (in_nonfin) o.nonfin = true;
         o.iters += MIX ? max(it, 1) : it;
+        if (MIX && it == 0) o.run = false;   // no step could be taken
         if (MIX) {
             o.outer++;
             if (in_nonfin) break;
