@@ -124,9 +124,10 @@ typedef struct {
     double tol;              /* on || (b - A x)_free ||_2 / || (b - A x_D)_free ||_2 (FP64)       */
     int32_t maxit;           /* total Krylov iterations                                             */
     double inner_tol;        /* mixed: relative reduction asked of each inner solve               */
-    int32_t check_every;     /* host reads the convergence flag every k iterations (>= 1; 0: 8); -1:
-                                GMRES checks first one iteration before the previous solve's count,
-                                then after every iteration. CG runs in one launch and ignores it     */
+    int32_t check_every;     /* strip and Cahouet-Chabard preconditioners: the host reads the convergence
+                                flag every k iterations (>= 1; 0: 8), or (-1) first one iteration
+                                before the previous solve's count, then after every iteration. The
+                                other solves are one launch and need no checks                       */
 } ocmp_solve_params_t;
 
 typedef struct {
@@ -228,19 +229,16 @@ int ocmp_solver_update(ocmp_solver_t solver, void* stream);
 int ocmp_solve(ocmp_solver_t solver, const double* b_dev, double* x_dev, void* stream, ocmp_solve_info_t* info);
 /* GMRES on all nbatch systems of a batched matrix at once (b, x: nbatch vectors of ndof, instance
  * after instance; infos: nbatch entries). Each system has its own Krylov space, Hessenberg matrix,
- * tolerance test and restart count; the kernels cover every instance in one launch (instance =
- * blockIdx.y) and instances that have converged return immediately. */
+ * tolerance test and restart count; one launch solves them all, a system on a block or on a team of
+ * blocks in proportion to its size. */
 int ocmp_solve_batch(ocmp_solver_t solver, const double* b_dev, double* x_dev, void* stream,
                      ocmp_solve_info_t* infos);
 /* Solver groups: uneven instances in one kernel sequence. The instances of several GMRES solvers
  * (each a single or batched matrix of its own space: different sizes, orders and patterns) are
- * solved together: every kernel of the GMRES iteration is launched once over all of them, a fixed
- * grid striding over a device list of (instance, block) pairs of the instances still iterating
- * (each instance's share proportional to its rows, the rows per thread of its SpMV from its
- * space's autotuned choice; the list shrinks after every restart cycle), one restart cycle
- * replayed from a CUDA graph. Each instance keeps its own Krylov space, tolerance and
- * convergence test; converged instances return at the top of every kernel. No kernel waits on
- * another block: reductions end in the last block to finish. Members must be GMRES with point
+ * solved together in one launch: each system gets a team of blocks in proportion to its rows and
+ * entries, systems of less than two blocks' work are taken one per block from a queue, largest
+ * first, and every team iterates on its own until its system has converged. Each instance keeps its
+ * own Krylov space, tolerance and convergence test. Members must be GMRES with point
  * Jacobi (or no) preconditioning, CSR Krylov matrices, and share restart, precision and maxit.
  * ocmp_group_solve takes one right-hand side and solution array per member (its instances one
  * after another) and fills infos for every instance in member order. The group borrows the
@@ -252,16 +250,16 @@ int ocmp_group_create(const ocmp_solver_t* solvers, int32_t count, ocmp_group_t*
 int ocmp_group_solve(ocmp_group_t group, const double* const* b_dev, double* const* x_dev, void* stream,
                      ocmp_solve_info_t* infos);
 int ocmp_group_destroy(ocmp_group_t group);
-/* Replay each GMRES restart cycle (m iterations, the x update and the next FP64 residual) from a
- * CUDA graph captured on first use (re-captured when b, x or the stream change). */
+/* Accepted and without effect: a GMRES solve is one launch (it used to replay each restart cycle from
+ * a CUDA graph when this was on). */
 int ocmp_solver_set_graph(ocmp_solver_t solver, int32_t on);
 /* OCMP_PRE_USER: the inverse diagonal (ndof, device) applied as the preconditioner; copied, and
  * taken over by the next ocmp_solver_update. */
 int ocmp_solver_set_diag(ocmp_solver_t solver, const double* dinv_dev, void* stream);
-/* Time every GMRES SpMV launch with CUDA events on its stream (single solves, outside graphs; up to
- * 4096 launches per solve); ocmp_solver_spmv_stats returns the launches that did the product (not
- * those queued past convergence, which return at once) and their total milliseconds since the
- * timing was switched on. No counterpart in the reference (measurement). */
+/* Time every GMRES product (single solves; up to 4096 per solve) inside the solve's kernel with the
+ * GPU's global timer, from the first block's start to the last block's end; ocmp_solver_spmv_stats
+ * returns the products and their total milliseconds since the timing was switched on. No counterpart
+ * in the reference (measurement). */
 int ocmp_solver_spmv_timing(ocmp_solver_t solver, int32_t on);
 int ocmp_solver_spmv_stats(ocmp_solver_t solver, int64_t* launches, double* total_ms);
 

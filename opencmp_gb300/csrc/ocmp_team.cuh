@@ -208,8 +208,10 @@ __device__ __forceinline__ bool team_reduce(Team& t, const double* v, double* ou
     if (t.size > 1) {
         if (w < NV) {
             const double* p = t.s->part[t.set][w];
-            const double s = t.size <= 32 ? team_list_sum<1>(t.size, lane, [&](int i) { return __ldcg(p + i); })
-                                          : team_list_sum<5>(t.size, lane, [&](int i) { return __ldcg(p + i); });
+            auto get = [&](int i) { return __ldcg(p + i); };
+            const double s = t.size <= 32   ? team_list_sum<1>(t.size, lane, get)
+                             : t.size <= 64 ? team_list_sum<2>(t.size, lane, get)
+                                            : team_list_sum<5>(t.size, lane, get);
             if (lane == 0) res[w] = s;
         }
         t.set ^= 1;
@@ -218,6 +220,23 @@ __device__ __forceinline__ bool team_reduce(Team& t, const double* v, double* ou
 #pragma unroll
     for (int i = 0; i < NV; i++) out[i] = res[i];
     return true;
+}
+
+// The same for one value held as float pairs: summed over the warps' lanes as pairs (48 bits).
+__device__ __forceinline__ bool team_reduce_ff(Team& t, float h, float l, double* out) {
+    __shared__ double wv[32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
+        ff_add(h, l, oh, ol);
+    }
+    if (lane == 0) wv[w] = ff_to_double(h, l);
+    __syncthreads();
+    double s = 0;
+    if (w == 0) s = team_list_sum<1>(nw, lane, [&](int i) { return wv[i]; });
+    double v[1] = {lane == 0 ? s : 0.0};
+    return team_reduce<1>(t, v, out, 1);
 }
 
 // After its last exchange every block leaves; the last one writes down where the count stands.
@@ -239,6 +258,7 @@ __device__ __forceinline__ TV team_row_dot(int32_t a, int32_t b, const int32_t* 
     for (int32_t base = a + lane; base < b; base += U * TPR) {
         int32_t c[U];
         TM v[U];
+        TV g[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int32_t k = base + u * TPR;
@@ -246,8 +266,9 @@ __device__ __forceinline__ TV team_row_dot(int32_t a, int32_t b, const int32_t* 
             v[u] = k < b ? __ldg(val + k) : (TM)0;
         }
 #pragma unroll
-        for (int u = 0; u < U; u++)
-            if (c[u] >= 0) (u & 1 ? acc1 : acc0) += (TV)v[u] * x[c[u]];
+        for (int u = 0; u < U; u++) g[u] = c[u] >= 0 ? x[c[u]] : (TV)0;
+#pragma unroll
+        for (int u = 0; u < U; u++) (u & 1 ? acc1 : acc0) += (TV)v[u] * g[u];
     }
     TV acc = acc0 + acc1;
 #pragma unroll

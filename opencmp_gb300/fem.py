@@ -324,11 +324,11 @@ class KrylovSolver:
         LB.call('ocmp_solver_set_diag', self.h, _ptr(dinv), _stream(stream))
 
     def spmv_timing(self, on: bool = True):
-        """Time each GMRES SpMV launch with CUDA events (resets the totals)."""
+        """Time each GMRES product inside the solve's kernel (resets the totals)."""
         LB.call('ocmp_solver_spmv_timing', self.h, int(on))
 
     def spmv_stats(self):
-        """(launches timed, total milliseconds) since spmv_timing(True)."""
+        """(products timed, total milliseconds) since spmv_timing(True)."""
         n, ms = C.c_int64(0), C.c_double(0)
         LB.call('ocmp_solver_spmv_stats', self.h, C.byref(n), C.byref(ms))
         return n.value, ms.value
@@ -361,7 +361,7 @@ class KrylovSolver:
         LB.call('ocmp_solver_strip_timing', self.h, int(on))
 
     def set_graph(self, on: bool = True):
-        """Replay each restart cycle from a captured CUDA graph (GMRES)."""
+        """Accepted, without effect: a GMRES solve is one launch."""
         LB.call('ocmp_solver_set_graph', self.h, int(on))
 
     def solve_batch(self, b: torch.Tensor, x: torch.Tensor, stream=None, raise_on_fail=True):
