@@ -19,7 +19,7 @@
 // every lane adding (a butterfly wastes 31 of 32 additions). Below about 10^4 rows: the exchanges,
 // 2,430 clocks each. Five launches per iteration with two-stage reductions in each took 54 us an
 // iteration at 79,507 rows (P2 tetrahedra, FP64, basis of 15) and 33 us at 1,156; one launch takes 32
-// (product 9.7, of which its gathers bound it; dots 4.6, orthogonalisation 4.6) and 13.
+// (product 9.5, bound by its gathers; dots 4.6, orthogonalisation 4.3) and 17 (on one block).
 #pragma once
 
 #include <type_traits>

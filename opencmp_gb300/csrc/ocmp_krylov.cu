@@ -255,41 +255,29 @@ __global__ void gm_cast(int64_t n, const double* __restrict__ a, float* __restri
     if (i < n) b[i] = (float)a[i];
 }
 
-// Cahouet-Chabard, part 1: z_u = sc D_u^-1 v_u, zp = sc v_p (the pressure solve's right-hand side)
+// Cahouet-Chabard after the pressure solve zp = S^-1 (sc v_p): z_u = sc D_u^-1 v_u,
+// z_p = -(alpha zp + beta M^-1 (sc v_p)) / tc^2; z may be v
 template <class T>
-__global__ void cc_pre1(int64_t nu, int64_t np, const T* __restrict__ v, const double* __restrict__ scale, int j,
-                        const double* __restrict__ vdinv, T* __restrict__ z, T* __restrict__ zp,
-                        const int* __restrict__ flags) {
+__global__ void cc_combine(int64_t nu, int64_t np, const T* v, const double* __restrict__ scale, int j,
+                           const double* __restrict__ vdinv, const double* __restrict__ mpinv,
+                           const T* __restrict__ zp, T* z, double alpha, double beta, double tc,
+                           const int* __restrict__ flags) {
     if (flags && flags[F_CONV]) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const double sc = scale ? scale[j] : 1.0;
-    if (i < nu) z[i] = (T)(sc * vdinv[i] * (double)v[i]);
-    else if (i < nu + np) zp[i - nu] = (T)(sc * (double)v[i]);
-}
-// part 2: z_p = -(alpha S^-1 (sc v_p) + beta M^-1 (sc v_p)) / tc^2 (S^-1 applied in place on zp)
-template <class T>
-__global__ void cc_pre2(int64_t nu, int64_t np, const T* __restrict__ v, const double* __restrict__ scale, int j,
-                        const double* __restrict__ mpinv, const T* __restrict__ zp, T* __restrict__ z, double alpha,
-                        double beta, double tc, const int* __restrict__ flags) {
-    if (flags && flags[F_CONV]) return;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const double sc = scale ? scale[j] : 1.0;
-    const double vp = sc * (double)v[nu + i];
-    z[nu + i] = (T)(-(alpha * (double)zp[i] + beta * mpinv[i] * vp) / (tc * tc));
+    if (i >= nu + np) return;
+    const double sv = (scale ? scale[j] : 1.0) * (i < nu ? vdinv[i] : 1.0) * (double)v[i];
+    z[i] = (T)(i < nu ? sv : -(alpha * (double)zp[i - nu] + beta * mpinv[i - nu] * sv) / (tc * tc));
 }
 
 template <class T>
-int cc_apply(CCPre* cc, const T* v, const double* scale, int j, T* z, const int* flags, cudaStream_t st) {
+int cc_apply(CCPre* cc, const T* v, const double* scale, int j, T* z, const int* flags, int* err, cudaStream_t st) {
     T* zp = nullptr;
     if constexpr (std::is_same<T, float>::value) zp = cc->zp32;
     else zp = cc->zp64;
-    OCMP_LAUNCH(cc_pre1<T><<<nblk(cc->nu + cc->np, kThreads), kThreads, 0, st>>>(cc->nu, cc->np, v, scale, j, cc->vdinv,
-                                                                              z, zp, flags));
-    int r = strip_apply<T>(cc->strip, cc->pop->space, cc->pop->vals, zp, nullptr, 0, zp, flags, st);
+    const int r = strip_apply<T>(cc->strip, v + cc->nu, scale, j, zp, flags, err, st);
     if (r) return r;
-    OCMP_LAUNCH(cc_pre2<T><<<nblk(cc->np, kThreads), kThreads, 0, st>>>(cc->nu, cc->np, v, scale, j, cc->mpinv, zp, z,
-                                                                     cc->alpha, cc->beta, cc->tc, flags));
+    OCMP_LAUNCH(cc_combine<T><<<nblk(cc->nu + cc->np, kThreads), kThreads, 0, st>>>(
+        cc->nu, cc->np, v, scale, j, cc->vdinv, cc->mpinv, zp, z, cc->alpha, cc->beta, cc->tc, flags));
     return OCMP_OK;
 }
 
@@ -518,15 +506,20 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
     int* flags = sv->gout->flags;
     double* scale = sv->small + m * (m + 1) / 2 + 3 * m + 2;
     const GmResult* H = sv->hout;
-    auto read = [&]() { return gm_read(sv->teams, sv->hout, sv->gout, 1, st); };
+    static_assert(kSweepAbort == GM_ABORT, "one bit for a wait that gave up");
+    auto read = [&]() {
+        const int r = gm_read(sv->teams, sv->hout, sv->gout, 1, st);
+        if (r == OCMP_TIMEOUT) strip_reset(sv->strip ? sv->strip : sv->cc->strip, st);
+        return r;
+    };
     auto launch = [&](int mode, int j) {
         a.mode = mode;
         a.j = j;
         return gm_launch<T>(a, sv->teams, st);
     };
     auto apply = [&](const T* v, const double* sc, int j, const int* fl) {
-        return sv->strip ? strip_apply<T>(sv->strip, sv->s, sv->mat->vals, v, sc, j, z, fl, st)
-                         : cc_apply<T>(sv->cc, v, sc, j, z, fl, st);
+        return sv->strip ? strip_apply<T>(sv->strip, v, sc, j, z, fl, &sv->gout->bits, st)
+                         : cc_apply<T>(sv->cc, v, sc, j, z, fl, &sv->gout->bits, st);
     };
     if (sv->time_spmv) OCMP_CUDA(cudaMemsetAsync(sv->tlog, 0, sizeof(unsigned long long) * 2 * kTimedProducts, st));
     int r = launch(GM_FIRST, 0);

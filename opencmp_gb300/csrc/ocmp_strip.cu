@@ -10,7 +10,7 @@
 // and a solve is a forward sweep y_k = G_k (b_k - A_k,k-1 y_k-1) and a backward sweep
 // x_k = y_k - G_k A_k,k+1 x_k+1. Every G_k is kept explicitly (FP32, dense), so each sweep step is
 // one dense matrix-vector product instead of two triangular solves; the sweeps of a
-// preconditioner application are replayed from a CUDA graph.
+// preconditioner application are one launch (ocmp_sweeps.cuh).
 //
 // Within a strip the dofs are ordered [N | I]: I = the dofs coupled to the previous strip (the
 // only rows and columns the Schur update A_k,k-1 S_{k-1}^-1 A_k-1,k touches), N = the rest, each
@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "ocmp_internal.h"
+#include "ocmp_sweeps.cuh"
 
 namespace ocmp {
 
@@ -81,18 +82,20 @@ struct Strip {
     int cmax = 0;                    // longest list
     float* d_T = nullptr;            // Schur update scratch: T = G_k-1[J, J] A[J, I] (nJ x nIp)
     StripWork work[kSide + 1];       // [0]: the caller's stream, [1..]: side streams
-    float* d_r = nullptr;            // solve scratch (one strip)
-    // ELL coupling lists of the sweeps' right-hand sides: per strip, the forward list (columns in
-    // the previous strip) then the backward one (columns in the next), entry-major; the values and
-    // the free rows' dofs are refreshed by every factorisation
-    std::vector<int64_t> eoff;       // per strip: first entry
-    std::vector<int> elo, ehi;       // per strip: widths
+    // the sweeps' steps and their coupling lists, whose values are refreshed by every factorisation, as
+    // are the free rows' dofs
+    SweepStep* d_steps = nullptr;
+    uint32_t* d_blob = nullptr;
+    uint2* d_words = nullptr;        // the sweeps' vector and results with their epochs
+    SweepState* d_state = nullptr;
+    SweepArgs sweep{};
+    int sweep_grid = 1;
+    size_t sweep_smem = 0;
     int32_t* d_prow = nullptr;       // per position (over all strips): its dof, -1 on padding
     int32_t* d_rdof = nullptr;       // per position: its dof if free, else -1
     int32_t* d_erow = nullptr;
-    int32_t* d_ecol = nullptr;       // per entry: the column's dof, -1 on padding
-    int32_t* d_epos = nullptr;       // per entry: its CSR position, -1 on padding
-    float* d_ev = nullptr;           // per entry: the value, 0 where the row or the column is constrained
+    int32_t* d_epos = nullptr;       // per entry of the lists: its CSR position, -1 on padding
+    int32_t* d_edst = nullptr;       // and its word of d_blob
     int64_t nell = 0, npos = 0;
     int* d_flag = nullptr;           // [0] pivot tiles that were singular or non-finite, [1] a tensor-core
                                      // product whose bounded wait gave up
@@ -104,14 +107,6 @@ struct Strip {
     cudaEvent_t ev_start = nullptr;
     cudaEvent_t ev_done = nullptr;
     std::vector<cudaEvent_t> ev_phase1;
-    // sweeps replayed from graphs: [0] gated on the solver's convergence flag, [1] not gated
-    cudaStream_t cap = nullptr;
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    unsigned long long gkernels[2] = {0, 0};
-    const void* g_z[2] = {nullptr, nullptr};
-    const int* g_flags[2] = {nullptr, nullptr};
-    const double* g_vals[2] = {nullptr, nullptr};
-    int g_type[2] = {0, 0};
     // statistics of the last factorisation
     bool timing = false;
     std::vector<cudaEvent_t> ev;
@@ -660,95 +655,24 @@ __global__ void k_infnorm(const float* __restrict__ A, int64_t lda, int rows, in
     if (lane == 0) atomicMax(out, sm == sm ? __float_as_uint(sm) : 0x7FFFFFFFu);
 }
 
-// ------------------------------------------------------------------ sweeps
-// z = sc v with sc = scale[j] (the GMRES basis vector into the preconditioner's input)
-template <class T>
-__global__ void k_scale_copy(int64_t n, const T* __restrict__ v, const double* __restrict__ scale, int j,
-                             T* __restrict__ z, const int* __restrict__ flags) {
-    if (flags && flags[0]) return;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) z[i] = (T)((double)v[i] * scale[j]);
-}
-
-// right-hand side of a strip step in the strip's order, from its ELL list (L entries per position,
-// entry-major: entry e of position q at e * mp + q): forward r_q = z_i - sum A[i, c] z_c over the
-// previous strip's columns, backward r_q = sum A[i, c] z_c over the next strip's; zero on
-// constrained rows and on the padding (rdof = -1)
-template <class T>
-__global__ void k_strip_rhs(int mp, int L, int fwd, const int32_t* __restrict__ rdof, const int32_t* __restrict__ ecol,
-                            const float* __restrict__ ev, const T* __restrict__ z, float* __restrict__ r,
-                            const int* __restrict__ flags) {
-    if (flags && flags[0]) return;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= mp) return;
-    const int row = rdof[q];
-    float acc = 0.f;
-    for (int e = 0; e < L; e++) {
-        const int cc = ecol[(int64_t)e * mp + q];
-        if (cc >= 0) acc = fmaf(ev[(int64_t)e * mp + q], (float)z[cc], acc);
-    }
-    r[q] = row < 0 ? 0.f : (fwd ? (float)z[row] - acc : acc);
-}
-
-// z_i = (G r)_p (mode 0) or z_i -= (G r)_p (mode 1), i = the local dof at position p. A block of
-// 8 warps takes 8 rows, a warp per row; r is staged in shared memory, and each lane keeps eight
-// 16-byte loads of G in flight (streamed past L1). mp is a multiple of 128.
-constexpr int kGemvDepth = 8;
-template <class T>
-__global__ void __launch_bounds__(256) k_strip_gemv(int mp, int64_t s0, const int32_t* __restrict__ perm,
-                                                    const float* __restrict__ G, const float* __restrict__ r,
-                                                    T* __restrict__ z, int mode, const int* __restrict__ flags) {
-    extern __shared__ float4 rs[];
-    if (flags && flags[0]) return;
-    const int nq = mp / 4;
-    const float4* r4 = reinterpret_cast<const float4*>(r);
-    for (int i = threadIdx.x; i < nq; i += blockDim.x) rs[i] = r4[i];
-    __syncthreads();
-    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= mp) return;
-    const int ld = perm[row];
-    if (ld < 0) return;
-    const float4* g = reinterpret_cast<const float4*>(G + (int64_t)row * mp);
-    float acc = 0.f;
-    for (int q0 = lane; q0 < nq; q0 += 32 * kGemvDepth) {
-        float4 a[kGemvDepth];
-#pragma unroll
-        for (int u = 0; u < kGemvDepth; u++)
-            if (q0 + 32 * u < nq) a[u] = __ldcs(g + q0 + 32 * u);
-#pragma unroll
-        for (int u = 0; u < kGemvDepth; u++)
-            if (q0 + 32 * u < nq) {
-                const float4 b = rs[q0 + 32 * u];
-                acc = fmaf(a[u].x, b.x, acc);
-                acc = fmaf(a[u].y, b.y, acc);
-                acc = fmaf(a[u].z, b.z, acc);
-                acc = fmaf(a[u].w, b.w, acc);
-            }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-        T* zi = z + s0 + ld;
-        if (mode == 0) *zi = (T)acc;
-        else *zi = (T)((float)*zi - acc);
-    }
-}
-
+// ------------------------------------------------------------------ around the sweeps
 template <class T>
 __global__ void k_add_to(int64_t n, const T* __restrict__ z, double* __restrict__ x) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) x[i] += (double)z[i];
 }
 
-// the ELL right-hand-side values and the free rows' dofs of every strip, after an assembly
-__global__ void k_ell_refresh(int64_t nent, const int32_t* __restrict__ erow, const int32_t* __restrict__ ecol,
-                              const int32_t* __restrict__ epos, const double* __restrict__ vals,
-                              const uint8_t* __restrict__ freed, float* __restrict__ ev, int64_t npos,
-                              const int32_t* __restrict__ prow, int32_t* __restrict__ rdof) {
+// the right-hand sides' values (0 where the row or the column is constrained) and the free rows' dofs
+// of every strip, after an assembly
+__global__ void k_list_refresh(int64_t nent, const int32_t* __restrict__ erow, const int32_t* __restrict__ epos,
+                               const int32_t* __restrict__ col, const double* __restrict__ vals,
+                               const uint8_t* __restrict__ freed, const int32_t* __restrict__ edst,
+                               uint32_t* __restrict__ blob, int64_t npos,
+                               const int32_t* __restrict__ prow, int32_t* __restrict__ rdof) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t < nent) {
         const int32_t q = epos[t];
-        ev[t] = (q >= 0 && freed[erow[t]] && freed[ecol[t]]) ? (float)vals[q] : 0.f;
+        blob[edst[t]] = __float_as_uint(q >= 0 && freed[erow[t]] && freed[col[q]] ? (float)vals[q] : 0.f);
     }
     if (t < npos) {
         const int32_t d = prow[t];
@@ -758,14 +682,14 @@ __global__ void k_ell_refresh(int64_t nent, const int32_t* __restrict__ erow, co
 
 // ------------------------------------------------------------------ host helpers
 void strip_free(Strip* p) {
-    void* ps[] = {p->d_perm, p->d_I, p->d_J, p->jrow, p->d_pinv, p->d_G, p->d_cptr, p->d_cb, p->d_crow, p->d_ccol, p->d_T, p->d_r, p->d_flag};
+    void* ps[] = {p->d_perm, p->d_I, p->d_J, p->jrow, p->d_pinv, p->d_G, p->d_cptr, p->d_cb, p->d_crow, p->d_ccol, p->d_T, p->d_flag};
     for (void* q : ps) dfree(q);
     for (auto& w : p->work) {
         dfree(w.P);
         dfree(w.Ck);
         dfree(w.Rt);
     }
-    void* qs2[] = {p->d_prow, p->d_rdof, p->d_erow, p->d_ecol, p->d_epos, p->d_ev};
+    void* qs2[] = {p->d_prow, p->d_rdof, p->d_erow, p->d_epos, p->d_edst, p->d_steps, p->d_blob, p->d_words, p->d_state};
     for (void* q : qs2) dfree(q);
     void* qs[] = {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Xa, p->d_Xb, p->d_R, p->d_Rt, p->d_Xt, p->d_T1, p->d_Zt, p->d_rmax,
                   p->d_H[0], p->d_H[1], p->d_H[2]};
@@ -781,9 +705,6 @@ void strip_free(Strip* p) {
     if (p->chain) cudaStreamDestroy(p->chain);
     for (cudaStream_t q : p->side)
         if (q) cudaStreamDestroy(q);
-    for (cudaGraphExec_t g : p->gexec)
-        if (g) cudaGraphExecDestroy(g);
-    if (p->cap) cudaStreamDestroy(p->cap);
 }
 
 // timing of the factorisation's kernels by class (ocmp_solver_strip_timing): an event pair around
@@ -1285,54 +1206,129 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         A(&w.Ck, (size_t)p->mp_max * kNb);
         A(&w.Rt, (size_t)p->mp_max * kNb);
     }
-    A(&p->d_r, (size_t)p->mp_max);
     A(&p->d_flag, 2);
     {
-        // ELL coupling lists of the sweeps' right-hand sides
-        std::vector<int64_t> eoff(K + 1, 0);
-        std::vector<int> elo(K, 0), ehi(K, 0);
-        std::vector<int32_t> prow, erow, ecol, epos;
+        int dev = 0, sms = 1;
+        if (!st && (cudaGetDevice(&dev) != cudaSuccess ||
+                    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
+            st = fail(OCMP_ERR_CUDA, "strip preconditioner: device attributes");
+        // a block per SM, but no more than leaves each a few rows
+        p->sweep_grid = std::max(1, std::min(sms, p->mp_max / kSweepMinRows));
+        std::vector<SweepStep> steps;
+        std::vector<int32_t> prow, erow, epos, edst;
+        std::vector<uint32_t> blob;
+        for (int k = 0; k < K; k++)
+            for (int q = 0; q < p->mp[k]; q++) {
+                const int32_t ld = perm[p->poff[k] + q];
+                prow.push_back(ld < 0 ? -1 : (int32_t)(p->s[k] + ld));
+            }
+        // strip k as a step of the forward (mode 0) or backward sweep
+        std::vector<int32_t> at(n);
+        auto step = [&](int k, int mode, int gs) {
+            const std::vector<int32_t>& ptr = mode == 0 ? lo_ptr : hi_ptr;
+            const std::vector<int32_t>& pos = mode == 0 ? lo_pos : hi_pos;
+            SweepStep t{};
+            t.G = p->d_G + p->goff[k];
+            t.p0 = (int32_t)p->poff[k];
+            t.mp = p->mp[k];
+            t.gs = gs;
+            t.per = sweep_rows(t.mp, gs);
+            std::vector<int32_t> cols, list;
+            for (int q = 0; q < t.mp; q++) {
+                const int32_t r = prow[t.p0 + q];
+                if (r < 0 || ptr[r] == ptr[r + 1]) continue;
+                list.push_back(q);
+                t.len = std::max(t.len, ptr[r + 1] - ptr[r]);
+                for (int32_t e = ptr[r]; e < ptr[r + 1]; e++) cols.push_back(col[pos[e]]);
+            }
+            std::sort(cols.begin(), cols.end());
+            cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
+            t.cnt = (int32_t)list.size();
+            t.nj = (int32_t)cols.size();
+            const SweepLists li = sweep_lists(t.cnt, t.len, t.nj);
+            t.blob = (int64_t)blob.size();
+            t.words = li.words;
+            blob.resize(blob.size() + li.words, 0u);
+            uint32_t* b = blob.data() + t.blob;
+            uint16_t* idx = reinterpret_cast<uint16_t*>(b + li.idx);
+            for (int q = 0; q < t.nj; q++) {
+                at[cols[q]] = q;
+                b[li.jd + q] = (uint32_t)cols[q];
+            }
+            for (int c = 0; c < t.cnt; c++) {
+                const int32_t r = prow[t.p0 + list[c]];
+                reinterpret_cast<uint16_t*>(b + li.cq)[c] = (uint16_t)list[c];
+                for (int e = 0; e < t.len; e++) {
+                    const int32_t cp = ptr[r] + e < ptr[r + 1] ? pos[ptr[r] + e] : -1;
+                    idx[e * t.cnt + c] = (uint16_t)(cp >= 0 ? at[col[cp]] : 0xffff);
+                    erow.push_back(r);
+                    epos.push_back(cp);
+                    edst.push_back((int32_t)(t.blob + e * t.cnt + c));
+                }
+            }
+            steps.push_back(t);
+        };
+        // forward over all strips, backward from the last but one
         for (int k = 0; k < K; k++) {
-            const int mpk = p->mp[k];
-            const int64_t s0 = p->s[k];
-            for (int q = 0; q < mpk; q++) {
-                const int ld = perm[p->poff[k] + q];
-                prow.push_back(ld < 0 ? -1 : (int32_t)(s0 + ld));
-                if (ld < 0) continue;
-                const int64_t r = s0 + ld;
-                elo[k] = std::max(elo[k], lo_ptr[r + 1] - lo_ptr[r]);
-                ehi[k] = std::max(ehi[k], hi_ptr[r + 1] - hi_ptr[r]);
-            }
-            eoff[k] = (int64_t)erow.size();
-            for (int part = 0; part < 2; part++) {
-                const int L = part == 0 ? elo[k] : ehi[k];
-                const std::vector<int32_t>& ptr = part == 0 ? lo_ptr : hi_ptr;
-                const std::vector<int32_t>& pos = part == 0 ? lo_pos : hi_pos;
-                for (int e = 0; e < L; e++)
-                    for (int q = 0; q < mpk; q++) {
-                        const int ld = perm[p->poff[k] + q];
-                        const int64_t r = ld < 0 ? -1 : s0 + ld;
-                        const bool has = ld >= 0 && ptr[r] + e < ptr[r + 1];
-                        const int32_t cp = has ? pos[ptr[r] + e] : -1;
-                        erow.push_back(ld < 0 ? 0 : (int32_t)r);
-                        ecol.push_back(has ? col[cp] : -1);
-                        epos.push_back(cp);
-                    }
-            }
+            step(k, 0, p->sweep_grid);
+            steps.push_back(SweepStep{});
         }
-        eoff[K] = (int64_t)erow.size();
-        p->eoff = eoff;
-        p->elo = elo;
-        p->ehi = ehi;
-        p->nell = (int64_t)erow.size();
+        for (int k = K - 2; k >= 0; k--) {
+            step(k, 1, p->sweep_grid);
+            steps.push_back(SweepStep{});
+        }
+        SweepArgs& a = p->sweep;
+        a.nsteps = (int)steps.size() / 2;
+        a.nfwd = K;
+        int most = 1, words = 0;   // floats of a step's rows in a block, words of its lists
+        for (const SweepStep& t : steps) {
+            a.rows = std::max(a.rows, t.per);
+            a.mp_max = std::max(a.mp_max, t.mp);
+            a.nj_max = std::max(a.nj_max, t.nj);
+            most = std::max(most, t.per * t.mp);
+            words = std::max(words, t.words);
+        }
+        // the lists are staged when they take no more than a third of the ring, in stages of a multiple
+        // of 128 bytes
+        const size_t fixed = sweep_fixed_smem(a.mp_max, a.nj_max, a.rows);
+        const int room = fixed < kSweepSmem ? (int)((kSweepSmem - fixed) / sizeof(float)) & ~31 : 0;
+        words = (words + 31) & ~31;
+        a.lists = words <= room / 3 ? words : 0;
+        a.stages = std::max(1, std::min({kSweepStages, room / (most + a.lists), a.nsteps}));
+        a.stage = std::min(most + a.lists, room);
+        p->sweep_smem = fixed + sizeof(float) * (size_t)a.stages * a.stage;
+        if (!st && (blob.size() > (size_t)INT32_MAX || a.nj_max >= 0xffff || p->sweep_smem > kSweepSmem))
+            st = fail(OCMP_ERR_UNSUPPORTED, "strip preconditioner: the couplings between the strips are too large");
+        for (SweepStep& t : steps) {
+            if (t.gs == 0) continue;
+            t.ns = std::min(t.per, (a.stage - a.lists) / t.mp);
+            const int groups = (t.ns + 7) / 8 + (t.per - t.ns + 7) / 8;
+            while (t.lwg < 4 && groups << (t.lwg + 1) <= kSweepWarps) t.lwg++;
+        }
+        if (!st && a.rows > kSweepThreads) st = fail(OCMP_ERR_UNSUPPORTED, "strip preconditioner: too few SMs");
+        p->nell = (int64_t)epos.size();
         p->npos = (int64_t)prow.size();
+        U(&p->d_steps, steps);
+        U(&p->d_blob, blob);
         U(&p->d_prow, prow);
         U(&p->d_erow, erow);
-        U(&p->d_ecol, ecol);
         U(&p->d_epos, epos);
+        U(&p->d_edst, edst);
         A(&p->d_rdof, prow.size());
-        A(&p->d_ev, std::max<size_t>(1, erow.size()));
-        p->bytes += (int64_t)(prow.size() * 2 + erow.size() * 4) * 4;
+        A(&p->d_words, 3 * (size_t)n);
+        A(&p->d_state, 1);
+        p->bytes += (int64_t)(prow.size() * 2 + epos.size() * 3 + blob.size() + 6 * n) * 4 +
+                    (int64_t)(steps.size() * sizeof(SweepStep));
+        a.steps = p->d_steps;
+        a.prow = p->d_prow;
+        a.rdof = p->d_rdof;
+        a.blob = p->d_blob;
+        a.b = p->d_words;
+        a.y = p->d_words + n;
+        a.x = p->d_words + 2 * n;
+        a.n = n;
+        a.state = p->d_state;
+        if (!st) st = strip_reset(p, nullptr);
     }
     if (p->nfast) {
         const size_t i2 = (size_t)p->nIp_max * p->nIp_max, mi = (size_t)p->mp_max * p->nIp_max;
@@ -1357,8 +1353,8 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
     p->bytes += (int64_t)Jpos.size() * 4;
     // every buffer a kernel of the factorisation or the sweeps dereferences must exist
     if (!st) {
-        const void* need_ptr[] = {p->d_perm, p->d_pinv, p->d_G, p->d_cptr, p->d_T, p->d_r, p->d_flag, p->d_prow, p->d_rdof,
-                                  p->d_ev, p->work[0].P, p->work[0].Ck, p->work[0].Rt};
+        const void* need_ptr[] = {p->d_perm, p->d_pinv, p->d_G, p->d_cptr, p->d_T, p->d_flag, p->d_prow, p->d_rdof,
+                                  p->d_steps, p->d_words, p->d_state, p->work[0].P, p->work[0].Ck, p->work[0].Rt};
         bool ok = std::all_of(std::begin(need_ptr), std::end(need_ptr), [](const void* q) { return q != nullptr; });
         if (p->nfast) {
             const void* fast_ptr[] = {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Xa, p->d_Xb, p->d_R, p->d_Rt, p->d_Xt,
@@ -1366,7 +1362,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
                                       p->d_Yt[2], p->d_rmax, p->h_rmax};
             ok = ok && std::all_of(std::begin(fast_ptr), std::end(fast_ptr), [](const void* q) { return q != nullptr; });
         }
-        if (p->nell) ok = ok && p->d_erow && p->d_ecol && p->d_epos;
+        if (p->nell) ok = ok && p->d_blob && p->d_erow && p->d_epos && p->d_edst;
         if (!ok) st = fail(OCMP_ERR_NOMEM, "strip preconditioner: a work buffer was not allocated");
     }
     if (!st && (cudaEventCreateWithFlags(&p->fev[0], cudaEventDefault) != cudaSuccess ||
@@ -1376,8 +1372,6 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
     for (int q = 0; q < kSide && !st; q++)
         if (cudaStreamCreateWithFlags(&p->side[q], cudaStreamNonBlocking) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "cudaStreamCreateWithFlags");
-    if (!st && cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess)
-        st = fail(OCMP_ERR_CUDA, "cudaStreamCreateWithFlags");
     if (!st) {
         int lo = 0, hi = 0;
         if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
@@ -1393,10 +1387,8 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         if (cudaFuncSetAttribute(k_tile_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_panel_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_panel_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_strip_gemv<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * p->mp_max) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(k_strip_gemv<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * p->mp_max) !=
-                cudaSuccess)
+            cudaFuncSetAttribute(k_sweeps<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess ||
+            cudaFuncSetAttribute(k_sweeps<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "strip preconditioner: shared-memory attribute");
     }
     if (st) {
@@ -1426,8 +1418,8 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
     OCMP_CUDA(cudaMemsetAsync(p->d_flag, 0, 2 * sizeof(int), st));
     {
         const int64_t nt = std::max(p->nell, p->npos);
-        OCMP_LAUNCH(k_ell_refresh<<<nblk(nt, 256), 256, 0, st>>>(p->nell, p->d_erow, p->d_ecol, p->d_epos, vals, s->d_free,
-                                                                  p->d_ev, p->npos, p->d_prow, p->d_rdof));
+        OCMP_LAUNCH(k_list_refresh<<<nblk(nt, 256), 256, 0, st>>>(p->nell, p->d_erow, p->d_epos, s->d_col, vals, s->d_free,
+                                                                 p->d_edst, p->d_blob, p->npos, p->d_prow, p->d_rdof));
     }
     OCMP_CUDA(cudaEventRecord(p->ev_start, st));
     for (int q = 0; q < kSide; q++) OCMP_CUDA(cudaStreamWaitEvent(p->side[q], p->ev_start, 0));
@@ -1499,66 +1491,24 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
     return OCMP_OK;
 }
 
-namespace {
-// the two sweeps, in place on z (input: the vector to precondition)
 template <class T>
-void sweeps(Strip* p, T* z, const int* flags, cudaStream_t st) {
-    const int K = p->K;
-    for (int pass = 0; pass < 2; pass++) {
-        for (int step = 0; step < (pass == 0 ? K : K - 1); step++) {
-            const int k = pass == 0 ? step : K - 2 - step;
-            const int mp = p->mp[k];
-            const int L = pass == 0 ? p->elo[k] : p->ehi[k];
-            const int64_t e0 = p->eoff[k] + (pass == 0 ? 0 : (int64_t)p->elo[k] * mp);
-            OCMP_LAUNCH(k_strip_rhs<T><<<nblk(mp, 128), 128, 0, st>>>(mp, L, pass == 0, p->d_rdof + p->poff[k],
-                                                                     p->d_ecol + e0, p->d_ev + e0, z, p->d_r, flags));
-            OCMP_LAUNCH(k_strip_gemv<T><<<nblk(mp, 8), 256, sizeof(float) * mp, st>>>(
-                mp, p->s[k], p->d_perm + p->poff[k], p->d_G + p->goff[k], p->d_r, z, pass, flags));
-        }
-    }
-}
-}  // namespace
-
-template <class T>
-int strip_apply(Strip* p, const ocmp_space_s* s, const double* vals, const T* v, const double* scale, int j, T* z,
-                const int* flags, cudaStream_t st) {
-    const int64_t n = s->ndof;
-    if (v != z) {
-        if (scale) OCMP_LAUNCH(k_scale_copy<T><<<nblk(n, 256), 256, 0, st>>>(n, v, scale, j, z, flags));
-        else OCMP_CUDA(cudaMemcpyAsync(z, v, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
-    }
-    // the sweeps (4 launches per strip) replay from a graph captured on first use for this
-    // (vector, flag, matrix) on the library's own stream
-    const int gi = flags ? 0 : 1;
-    const int type = sizeof(T) == 8 ? 1 : 2;
-    if (!p->gexec[gi] || p->g_z[gi] != z || p->g_flags[gi] != flags || p->g_vals[gi] != vals || p->g_type[gi] != type) {
-        if (p->gexec[gi]) {
-            cudaGraphExecDestroy(p->gexec[gi]);
-            p->gexec[gi] = nullptr;
-        }
-        cudaGraph_t g;
-        const unsigned long long l0 = g_launches.load();
-        OCMP_CUDA(cudaStreamBeginCapture(p->cap, cudaStreamCaptureModeThreadLocal));
-        sweeps<T>(p, z, flags, p->cap);
-        OCMP_CUDA(cudaStreamEndCapture(p->cap, &g));
-        p->gkernels[gi] = g_launches.load() - l0;
-        g_launches.fetch_sub(p->gkernels[gi]);
-        cudaError_t e = cudaGraphInstantiate(&p->gexec[gi], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate (strip sweeps)");
-        p->g_z[gi] = z;
-        p->g_flags[gi] = flags;
-        p->g_vals[gi] = vals;
-        p->g_type[gi] = type;
-    }
-    OCMP_CUDA(cudaGraphLaunch(p->gexec[gi], st));
-    g_launches.fetch_add(p->gkernels[gi]);
+int strip_apply(Strip* p, const T* v, const double* scale, int j, T* z, const int* flags, int* err, cudaStream_t st) {
+    SweepArgs a = p->sweep;
+    a.err = err;
+    void* kp[] = {&a, &v, &scale, &j, &z, &flags};
+    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel((const void*)k_sweeps<T>, dim3(p->sweep_grid), dim3(kSweepThreads),
+                                                      kp, p->sweep_smem, st)));
     return OCMP_OK;
 }
-template int strip_apply<double>(Strip*, const ocmp_space_s*, const double*, const double*, const double*, int,
-                                 double*, const int*, cudaStream_t);
-template int strip_apply<float>(Strip*, const ocmp_space_s*, const double*, const float*, const double*, int, float*,
-                                const int*, cudaStream_t);
+template int strip_apply<double>(Strip*, const double*, const double*, int, double*, const int*, int*, cudaStream_t);
+template int strip_apply<float>(Strip*, const float*, const double*, int, float*, const int*, int*, cudaStream_t);
+
+// no word of an earlier launch may carry a later epoch: the results are cleared with the count
+int strip_reset(Strip* p, cudaStream_t st) {
+    OCMP_CUDA(cudaMemsetAsync(p->d_state, 0, sizeof(SweepState), st));
+    OCMP_CUDA(cudaMemsetAsync(p->d_words, 0, sizeof(uint2) * 3 * (size_t)p->s.back(), st));
+    return OCMP_OK;
+}
 
 template <class T>
 int strip_add(int64_t n, const T* z, double* x, cudaStream_t st) {

@@ -27,6 +27,7 @@
 #include <string>
 
 #include "ocmp_internal.h"
+#include "ocmp_mbar.cuh"
 
 namespace ocmp {
 namespace {
@@ -36,37 +37,6 @@ constexpr int kBoxBytes = TBM * TBK * 4;            // 16 KiB, one 128 x 32 FP32
 constexpr int kStageBytes = 4 * kBoxBytes;          // A, B, A_low, B_low
 constexpr int kTcSmem = TST * kStageBytes + 1024 + 256;
 constexpr int kTcThreads = 192;
-constexpr long long kWaitCycles = 2000000000LL;     // about one second at the boost clock
-
-__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t a) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait; false when it gave up or another role already did (*abort)
-__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int* abort) {
-    const long long t0 = clock64();
-    while (!mbar_try(a, parity)) {
-        if (*abort) return false;
-        if (clock64() - t0 > kWaitCycles) return false;
-    }
-    return true;
-}
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
     asm volatile(
