@@ -42,6 +42,7 @@
 #include <cstring>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ocmp_internal.h"
@@ -318,98 +319,139 @@ __global__ void __launch_bounds__(128) k_schur_u(int nI, int nIp, int nNp, int64
 
 // ------------------------------------------------------------------ block Gauss-Jordan
 // P <- inverse of the tile S[t0:t0+128, t0:t0+128] by Gauss-Jordan with partial pivoting inside
-// the tile. The tile stays in registers (thread t holds column t % 128 of rows t / 128 + 8 j) and
-// rows are never moved: step k takes as pivot the largest |a_rk| over the rows not yet used, and
-// the row and column permutation is applied when the result is written (P[step(r)][piv(c)] =
-// M[r][c]). Per step the eight owners of column k publish it with their best unused row, every
-// thread reduces the eight candidates, the owners of the pivot row publish that row
-// (double-buffered in shared memory): two barriers per step. A zero or non-finite pivot is
-// counted in *flag and replaced by a tiny value.
-constexpr int kTileThreads = 1024;
-constexpr int kTileSmem = 0;
+// the tile. The tile stays in registers, 8 x 8 per thread, and rows are never moved: step k takes as
+// pivot the largest |a_rk| over the rows not yet used, and the row and column permutation is applied
+// when the result is written (P[step(r)][piv(c)] = M[r][c]). Per step the half warp that holds column
+// k publishes it with the pivot, the half warps' owners of the pivot row publish that row (both
+// double-buffered in shared memory): two barriers per step. The rank-1 update reads 16 values per 64
+// products; one row of 16 entries per thread (1,024 threads) read one value per product and was bound
+// by issue: 286 us a tile. A zero or non-finite pivot is counted in *flag and replaced by a tiny
+// value.
+constexpr int kTileThreads = 256;
 __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restrict__ S, int mp, int t0,
                                                            float* __restrict__ P, int* __restrict__ flag) {
-    __shared__ float colk[2][kNb];
-    __shared__ float prow[2][kNb];
-    __shared__ float cval[2][8];
-    __shared__ int crow[2][8];
+    __shared__ __align__(16) float colk[2][kNb];
+    __shared__ __align__(16) float prow[2][kNb];
+    __shared__ int pk[2];
+    __shared__ float dk[2];
     __shared__ int piv[kNb];
     __shared__ int step[kNb];
-    const int tid = threadIdx.x, c = tid & (kNb - 1), r0 = tid >> 7;
-    constexpr int R = kNb / 8;   // rows per thread
-    float v[R];
+    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4, lane = tid & 31;
+    const unsigned group = 0xffffu << (lane & 16);
+    float v[8][8];
 #pragma unroll
-    for (int j = 0; j < R; j++) v[j] = S[(int64_t)(t0 + r0 + 8 * j) * mp + t0 + c];
-    unsigned usedmask = 0;       // which of this thread's rows have been pivots
-    for (int k = 0; k < kNb; k++) {
-        const int b = k & 1;
-        if (c == k) {
-            float best = -1.f;
-            int bi = kNb;
+    for (int i = 0; i < 8; i++)
 #pragma unroll
-            for (int j = 0; j < R; j++) {
-                colk[b][r0 + 8 * j] = v[j];
-                const float a = (usedmask >> j) & 1u ? -1.f : fabsf(v[j]);
-                if (a > best) {
-                    best = a;
-                    bi = r0 + 8 * j;
+        for (int j = 0; j < 8; j += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(S + (int64_t)(t0 + tr * 8 + i) * mp + t0 + tc * 8 + j);
+            v[i][j] = x.x;
+            v[i][j + 1] = x.y;
+            v[i][j + 2] = x.z;
+            v[i][j + 3] = x.w;
+        }
+    unsigned used = 0;       // which of this thread's rows have been pivots
+    // (a column of NaNs leaves rows without a step: those keep their own places)
+    if (tid < kNb) piv[tid] = step[tid] = tid;
+    __syncthreads();
+    // step k = 8 kb + kk; kk is a constant so that v stays in registers
+    auto eliminate = [&](int kb, auto col) {
+        constexpr int kk = decltype(col)::value, b = kk & 1;
+        const int k = kb * 8 + kk;
+        if (tc == kb) {
+            // 1 + the bits of |a|: 0 for a used row and for a NaN
+            unsigned key[8], best = 0u;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float a = fabsf(v[i][kk]);
+                key[i] = (used >> i) & 1u || !(a == a) ? 0u : __float_as_uint(a) + 1u;
+                best = max(best, key[i]);
+            }
+            const unsigned top = __reduce_max_sync(group, best);
+            const int leader = __ffs(__ballot_sync(group, best == top)) - 1;
+            float pv = 0.f;
+            int p = k;   // every remaining |a_rk| is NaN
+            bool mine = lane == leader && top != 0u;
+#pragma unroll
+            for (int i = 7; i >= 0; i--)
+                if (key[i] == top) {
+                    pv = v[i][kk];
+                    if (top) p = tr * 8 + i;
                 }
+#pragma unroll
+            for (int i = 0; i < 8; i++) colk[b][tr * 8 + i] = v[i][kk];
+            if (lane == leader) {
+                if (!mine || !(fabsf(pv) > 0.f) || !isfinite(pv)) {
+                    atomicAdd(flag, 1);
+                    pv = 1e-30f;
+                }
+                // the pivot row becomes prow: 0 - (-1) prow below
+                if (mine) colk[b][p] = -1.f;
+                pk[b] = p;
+                dk[b] = 1.f / pv;
+                piv[k] = p;
+                step[p] = k;
             }
-            cval[b][r0] = best;
-            crow[b][r0] = bi;
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i][kk] = 0.f;
+            // the pivot row's entry of column k is 1 before the scaling
+            if (mine)
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i][kk] = p == tr * 8 + i ? 1.f : v[i][kk];
         }
         __syncthreads();
-        float best = cval[b][0];
-        int p = crow[b][0];
+        const int p = pk[b];
+        if (tr == p >> 3) {
+            const float d = dk[b];
+            auto take = [&](auto row) {
+                constexpr int i = decltype(row)::value;
 #pragma unroll
-        for (int g = 1; g < 8; g++) {
-            const float a = cval[b][g];
-            const int r = crow[b][g];
-            if (a > best || (a == best && r < p)) {
-                best = a;
-                p = r;
+                for (int j = 0; j < 8; j++) {
+                    prow[b][tc * 8 + j] = v[i][j] * d;
+                    v[i][j] = 0.f;
+                }
+            };
+            switch (p & 7) {
+                case 0: take(std::integral_constant<int, 0>{}); break;
+                case 1: take(std::integral_constant<int, 1>{}); break;
+                case 2: take(std::integral_constant<int, 2>{}); break;
+                case 3: take(std::integral_constant<int, 3>{}); break;
+                case 4: take(std::integral_constant<int, 4>{}); break;
+                case 5: take(std::integral_constant<int, 5>{}); break;
+                case 6: take(std::integral_constant<int, 6>{}); break;
+                default: take(std::integral_constant<int, 7>{});
             }
-        }
-        if (p >= kNb) {   // every remaining |a_rk| is NaN: take the smallest unused row
-            p = kNb;
-#pragma unroll
-            for (int g = 0; g < 8; g++) p = min(p, crow[b][g] < kNb ? crow[b][g] : kNb);
-            if (p >= kNb) p = k;
-        }
-        float pv = colk[b][p];
-        if (!(fabsf(pv) > 0.f) || !isfinite(pv)) {
-            if (tid == 0) atomicAdd(flag, 1);
-            pv = 1e-30f;
-        }
-        const float d = 1.f / pv;
-        if (r0 == (p & 7)) {
-            // v[p >> 3] without dynamic register indexing
-            float x = 0.f;
-#pragma unroll
-            for (int j = 0; j < R; j++)
-                if (j == (p >> 3)) x = v[j];
-            prow[b][c] = (c == k ? 1.f : x) * d;
-            usedmask |= 1u << (p >> 3);
+            used |= 1u << (p & 7);
         }
         __syncthreads();
-        if (tid == 0) {
-            piv[k] = p;
-            step[p] = k;
-        }
-        const float pr = prow[b][c];
+        float cr[8], pr[8];
 #pragma unroll
-        for (int j = 0; j < R; j++) {
-            const int r = r0 + 8 * j;
-            if (r == p) v[j] = pr;
-            else v[j] = (c == k ? 0.f : v[j]) - colk[b][r] * pr;
+        for (int i = 0; i < 8; i += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(&colk[b][tr * 8 + i]);
+            const float4 y = *reinterpret_cast<const float4*>(&prow[b][tc * 8 + i]);
+            cr[i] = x.x, cr[i + 1] = x.y, cr[i + 2] = x.z, cr[i + 3] = x.w;
+            pr[i] = y.x, pr[i + 1] = y.y, pr[i + 2] = y.z, pr[i + 3] = y.w;
         }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[i][j] -= cr[i] * pr[j];
+    };
+    for (int kb = 0; kb < kNb / 8; kb++) {
+        eliminate(kb, std::integral_constant<int, 0>{});
+        eliminate(kb, std::integral_constant<int, 1>{});
+        eliminate(kb, std::integral_constant<int, 2>{});
+        eliminate(kb, std::integral_constant<int, 3>{});
+        eliminate(kb, std::integral_constant<int, 4>{});
+        eliminate(kb, std::integral_constant<int, 5>{});
+        eliminate(kb, std::integral_constant<int, 6>{});
+        eliminate(kb, std::integral_constant<int, 7>{});
     }
     __syncthreads();
-    const int pc = piv[c];
 #pragma unroll
-    for (int j = 0; j < R; j++) {
-        const int r = r0 + 8 * j;
-        P[step[r] * kNb + pc] = v[j];
+    for (int i = 0; i < 8; i++) {
+        const int r = step[tr * 8 + i];
+#pragma unroll
+        for (int j = 0; j < 8; j++) P[r * kNb + piv[tc * 8 + j]] = v[i][j];
     }
 }
 
@@ -751,7 +793,7 @@ int gemm(Strip* p, int M, int N, int K, const float* A, int64_t lda, const float
 int gj_tiles(Strip* p, float* S, int mp, int t_begin, int t_end, const StripWork& w, cudaStream_t st) {
     for (int t0 = t_begin; t0 < t_end; t0 += kNb) {
         int r = tbegin(p, st);
-        OCMP_LAUNCH(k_tile_inv<<<1, kTileThreads, kTileSmem, st>>>(S, mp, t0, w.P, p->d_flag));
+        OCMP_LAUNCH(k_tile_inv<<<1, kTileThreads, 0, st>>>(S, mp, t0, w.P, p->d_flag));
         if (!r) r = tend(p, st, 1);
         if (!r) r = tbegin(p, st);
         OCMP_LAUNCH(k_panel_prep<<<mp / 32, 256, kPrepSmem, st>>>(S, mp, t0, w.P, w.Rt, w.Ck));
@@ -1384,8 +1426,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         if (cudaEventCreateWithFlags(&p->ev_phase1[k], cudaEventDisableTiming) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "cudaEventCreate");
     if (!st) {
-        if (cudaFuncSetAttribute(k_tile_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_panel_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem) != cudaSuccess ||
+        if (cudaFuncSetAttribute(k_panel_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_panel_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_sweeps<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_sweeps<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess)
