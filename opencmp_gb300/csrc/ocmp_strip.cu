@@ -12,6 +12,9 @@
 // one dense matrix-vector product instead of two triangular solves; the sweeps of a
 // preconditioner application are one launch (ocmp_sweeps.cuh).
 //
+// The elimination runs from both ends towards the middle strip (strip k of the second half takes
+// k + 1's place for k - 1 above, and the middle strip is updated from both sides): two chains at once,
+// half as long. "Previous" below is the neighbour farther from the middle, "next" the nearer one.
 // Within a strip the dofs are ordered [N | I]: I = the dofs coupled to the previous strip (the
 // only rows and columns the Schur update A_k,k-1 S_{k-1}^-1 A_k-1,k touches), N = the rest, each
 // part padded to a multiple of 128 with decoupled unit rows. G_k is the block Gauss-Jordan inverse
@@ -20,12 +23,12 @@
 // dominant flops. Since the Schur update only adds to the II block, the N pivots can be eliminated
 // before it:
 //   phase 1 (side streams, all strips independent): fill S_k, eliminate its N tiles;
-//   phase 2 (the chain stream, strip after strip): S_k[I,I] -= A[I,J] G_k-1[J,J] A[J,I] (J = the
+//   phase 2 (a stream per chain, strip after strip): S_k[I,I] -= A[I,J] G_k-1[J,J] A[J,I] (J = the
 //     dofs of strip k-1 coupled to strip k; A[I,J] and A[J,I] hold a few entries per row, so the
 //     update is two sparse-times-dense kernels over per-dof coupling lists), then eliminate the I
 //     tiles.
 // On a structured triangle mesh half of each strip's elements touch the previous row of elements,
-// so phase 2, the sequential chain, does half of the pivot tiles.
+// so phase 2, the sequential chains, does half of the pivot tiles.
 // Newton-Schulz path, for a strip whose N dofs fall into independent groups of at most 32 (the
 // elements of a row of DG elements that do not touch the previous row): phase 1 inverts the groups
 // (a warp each) and forms the interface complement W0 = S_II - S_IN S_NN^-1 S_NI with one dense
@@ -59,8 +62,34 @@ struct StripWork {
     float* Rt = nullptr;   // row panel (transposed), mp_max x kNb
 };
 
+// One of the two chains of phase 2: its stream (at the highest priority so that the side streams'
+// products never hold it back) and scratch.
+struct StripChain {
+    cudaStream_t stream = nullptr;
+    StripWork work;
+    float* T = nullptr;              // Schur update: G_prev[J, J] A[J, I] (nJ x nIp)
+    float* Xa = nullptr;             // Newton-Schulz iterates, residual, transposes
+    float* Xb = nullptr;
+    float* R = nullptr;
+    float* Rt = nullptr;
+    float* Xt = nullptr;
+    float* H[3] = {};                // the last three interface inverses, newest first (Newton-Schulz starts)
+    int h_n[3] = {0, 0, 0};          // their padded sizes (0: none)
+    float* T1 = nullptr;
+    float* Zt = nullptr;
+    unsigned* rmax = nullptr;
+    unsigned* h_rmax = nullptr;      // pinned
+    cudaEvent_t ev_read = nullptr;   // the residual's copy
+    cudaEvent_t ev_done = nullptr;   // the chain's last strip
+    // a strip in progress
+    float* cur = nullptr;
+    float* nxt = nullptr;
+    float rprev = 0.f;
+    int it = 0;
+};
+
 struct Strip {
-    int K = 0;
+    int K = 0, mid = 0;              // strips, the middle one
     std::vector<int64_t> s;          // K + 1 strip boundaries
     std::vector<int> m, mp;          // strip sizes and padded sizes (nNp + nIp)
     std::vector<int> nN, nNp, nI, nJ;
@@ -81,8 +110,9 @@ struct Strip {
     int32_t* d_crow = nullptr;
     int32_t* d_ccol = nullptr;
     int cmax = 0;                    // longest list
-    float* d_T = nullptr;            // Schur update scratch: T = G_k-1[J, J] A[J, I] (nJ x nIp)
-    StripWork work[kSide + 1];       // [0]: the caller's stream, [1..]: side streams
+    int64_t coff2 = 0;               // the middle strip's lists to its second neighbour, as an offset into d_cptr
+    StripWork work[kSide];           // of the side streams
+    StripChain chain[2];             // the strips below the middle and the middle one; those above
     // the sweeps' steps and their coupling lists, whose values are refreshed by every factorisation, as
     // are the free rows' dofs
     SweepStep* d_steps = nullptr;
@@ -103,10 +133,7 @@ struct Strip {
     int64_t bytes = 0;
     int64_t schur_flops_pending = 0;
     cudaStream_t side[kSide] = {};
-    cudaStream_t chain = nullptr;    // phase 2, at the highest stream priority so that the side streams'
-                                     // products never hold the chain's kernels back
     cudaEvent_t ev_start = nullptr;
-    cudaEvent_t ev_done = nullptr;
     std::vector<cudaEvent_t> ev_phase1;
     // statistics of the last factorisation
     bool timing = false;
@@ -127,18 +154,7 @@ struct Strip {
     int32_t* d_gidx = nullptr;       // group members: positions in the strip's order (all in N)
     int32_t* d_gcomp = nullptr;      // per member: its component within the group (start << 8 | size)
     float* d_Yt[kSide] = {};         // phase 1 scratch per side stream: Y^T
-    float* d_Xa = nullptr;           // chain scratch: Newton-Schulz iterates, residual, transposes
-    float* d_Xb = nullptr;
-    float* d_R = nullptr;
-    float* d_Rt = nullptr;
-    float* d_Xt = nullptr;
-    float* d_H[3] = {};              // the last three interface inverses, newest first (Newton-Schulz starts)
-    int h_n[3] = {0, 0, 0};          // their padded sizes (0: none)
     bool schulz = true;              // Newton-Schulz path on (off: block Gauss-Jordan throughout)
-    float* d_T1 = nullptr;
-    float* d_Zt = nullptr;
-    unsigned* d_rmax = nullptr;
-    unsigned* h_rmax = nullptr;      // pinned
     int nfast = 0;
     int ns_iters = 0, ns_strips = 0, ns_fallbacks = 0;
 };
@@ -724,7 +740,7 @@ __global__ void k_list_refresh(int64_t nent, const int32_t* __restrict__ erow, c
 
 // ------------------------------------------------------------------ host helpers
 void strip_free(Strip* p) {
-    void* ps[] = {p->d_perm, p->d_I, p->d_J, p->jrow, p->d_pinv, p->d_G, p->d_cptr, p->d_cb, p->d_crow, p->d_ccol, p->d_T, p->d_flag};
+    void* ps[] = {p->d_perm, p->d_I, p->d_J, p->jrow, p->d_pinv, p->d_G, p->d_cptr, p->d_cb, p->d_crow, p->d_ccol, p->d_flag};
     for (void* q : ps) dfree(q);
     for (auto& w : p->work) {
         dfree(w.P);
@@ -733,18 +749,22 @@ void strip_free(Strip* p) {
     }
     void* qs2[] = {p->d_prow, p->d_rdof, p->d_erow, p->d_epos, p->d_edst, p->d_steps, p->d_blob, p->d_words, p->d_state};
     for (void* q : qs2) dfree(q);
-    void* qs[] = {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Xa, p->d_Xb, p->d_R, p->d_Rt, p->d_Xt, p->d_T1, p->d_Zt, p->d_rmax,
-                  p->d_H[0], p->d_H[1], p->d_H[2]};
+    void* qs[] = {p->d_gptr, p->d_gidx, p->d_gcomp};
     for (void* q : qs) dfree(q);
+    for (auto& c : p->chain) {
+        void* cs[] = {c.work.P, c.work.Ck, c.work.Rt, c.T, c.Xa, c.Xb, c.R, c.Rt, c.Xt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax};
+        for (void* q : cs) dfree(q);
+        if (c.h_rmax) cudaFreeHost(c.h_rmax);
+        if (c.ev_read) cudaEventDestroy(c.ev_read);
+        if (c.ev_done) cudaEventDestroy(c.ev_done);
+        if (c.stream) cudaStreamDestroy(c.stream);
+    }
     for (float* q : p->d_Yt) dfree(q);
-    if (p->h_rmax) cudaFreeHost(p->h_rmax);
     for (cudaEvent_t e : p->ev) cudaEventDestroy(e);
     for (cudaEvent_t e : p->ev_phase1) cudaEventDestroy(e);
     for (cudaEvent_t e : p->fev)
         if (e) cudaEventDestroy(e);
     if (p->ev_start) cudaEventDestroy(p->ev_start);
-    if (p->ev_done) cudaEventDestroy(p->ev_done);
-    if (p->chain) cudaStreamDestroy(p->chain);
     for (cudaStream_t q : p->side)
         if (q) cudaStreamDestroy(q);
 }
@@ -836,96 +856,171 @@ int phase1_groups(Strip* p, int k, float* S, int q, cudaStream_t ss) {
     return OCMP_OK;
 }
 
-// Inverse of the interface Schur complement W = S_II (n x n, leading dimension mp) into a buffer
-// of the chain (returned in *X, its transpose in d_Xt). Newton-Schulz X <- X + X R, R = I - W X,
-// started from the previous strips' interface inverses extrapolated along the strips (quadratic
-// from three, linear from two, the last one alone; the interface complements of the strips of a
-// row-by-row structured mesh vary smoothly from row to row). The step squares R, so with
-// rho = ||R||_inf read back after each product: rho <= kSchulzTol: X is taken; rho^2 <= kSchulzTol:
-// one more step is taken unchecked; a step that does not reduce rho (or a non-finite rho, or
-// kSchulzMax steps) falls back to block Gauss-Jordan on a copy of W, as does a strip without a
-// previous inverse of its size.
+// Inverse of the interface Schur complement W = S_II (n x n, leading dimension mp) into the chain's
+// buffer `cur` (its transpose in Xt). Newton-Schulz X <- X + X R, R = I - W X, started from the previous
+// strips' interface inverses extrapolated along the strips (quadratic from three, linear from two, the
+// last one alone; the interface complements of the strips of a row-by-row structured mesh vary smoothly
+// from row to row). The step squares R, so with rho = ||R||_inf read back after each product:
+// rho <= kSchulzTol: X is taken; rho^2 <= kSchulzTol: one more step is taken unchecked; a step that does
+// not reduce rho (or a non-finite rho, or kSchulzMax steps) falls back to block Gauss-Jordan on a copy
+// of W, as does a strip without a previous inverse of its size. The host drives both chains: while it
+// waits for one's rho, the other's kernels run.
 constexpr float kSchulzTol = 1e-5f;
 constexpr int kSchulzMax = 8;
-int invert_interface(Strip* p, const float* W, int mp, int n, float** X, cudaStream_t cs) {
-    float* cur = p->d_Xa;
-    float* nxt = p->d_Xb;
+
+// the residual of the current iterate and its norm, on the way to the host
+int schulz_residual(Strip* p, StripChain& c, const float* W, int mp, int n) {
+    cudaStream_t cs = c.stream;
+    int r = transpose(c.cur, n, n, n, c.Xt, n, cs);
+    if (!r) r = copy2d(nullptr, 0, n, n, c.R, n, 1.f, cs);
+    if (!r) r = gemm(p, n, n, n, W, mp, c.Xt, n, c.R, n, -1.f, 1.f, cs);
+    if (r) return r;
+    OCMP_CUDA(cudaMemsetAsync(c.rmax, 0, sizeof(unsigned), cs));
+    OCMP_LAUNCH(k_infnorm<<<nblk(n, 8), 256, 0, cs>>>(c.R, n, n, n, c.rmax));
+    OCMP_CUDA(cudaMemcpyAsync(c.h_rmax, c.rmax, sizeof(unsigned), cudaMemcpyDeviceToHost, cs));
+    OCMP_CUDA(cudaEventRecord(c.ev_read, cs));
+    return OCMP_OK;
+}
+
+// start of an interface inversion: *pending when a residual is on its way
+int schulz_begin(Strip* p, StripChain& c, const float* W, int mp, int n, bool* pending) {
+    c.cur = c.Xa;
+    c.nxt = c.Xb;
+    c.rprev = INFINITY;
+    c.it = 0;
+    *pending = false;
     int hist = 0;
-    while (hist < 3 && p->h_n[hist] == n) hist++;
-    bool ok = false;
-    if (p->schulz && hist > 0) {
-        const int64_t n4 = (int64_t)n * n / 4;
-        const float c[3][3] = {{1.f, 0.f, 0.f}, {2.f, -1.f, 0.f}, {3.f, -3.f, 1.f}};
-        const float* cc = c[hist - 1];
-        OCMP_LAUNCH(k_extrap<<<nblk(n4, 256), 256, 0, cs>>>(
-            n4, reinterpret_cast<const float4*>(p->d_H[0]), hist > 1 ? reinterpret_cast<const float4*>(p->d_H[1]) : nullptr,
-            hist > 2 ? reinterpret_cast<const float4*>(p->d_H[2]) : nullptr, cc[0], cc[1], cc[2],
-            reinterpret_cast<float4*>(cur)));
-        float rprev = INFINITY;
-        for (int it = 0; it < kSchulzMax; it++) {
-            int r = transpose(cur, n, n, n, p->d_Xt, n, cs);
-            if (!r) r = copy2d(nullptr, 0, n, n, p->d_R, n, 1.f, cs);
-            if (!r) r = gemm(p, n, n, n, W, mp, p->d_Xt, n, p->d_R, n, -1.f, 1.f, cs);
-            if (r) return r;
-            OCMP_CUDA(cudaMemsetAsync(p->d_rmax, 0, sizeof(unsigned), cs));
-            OCMP_LAUNCH(k_infnorm<<<nblk(n, 8), 256, 0, cs>>>(p->d_R, n, n, n, p->d_rmax));
-            OCMP_CUDA(cudaMemcpyAsync(p->h_rmax, p->d_rmax, sizeof(unsigned), cudaMemcpyDeviceToHost, cs));
-            OCMP_CUDA(cudaStreamSynchronize(cs));
-            float rho;
-            std::memcpy(&rho, p->h_rmax, sizeof(float));
-            if (!std::isfinite(rho) || rho >= rprev) break;
-            if (rho <= kSchulzTol) {
-                ok = true;
-                break;
-            }
-            rprev = rho;
-            r = transpose(p->d_R, n, n, n, p->d_Rt, n, cs);
-            if (!r) r = copy2d(cur, n, n, n, nxt, n, 1.f, cs);
-            if (!r) r = gemm(p, n, n, n, cur, n, p->d_Rt, n, nxt, n, 1.f, 1.f, cs);
-            if (r) return r;
-            std::swap(cur, nxt);
-            p->ns_iters++;
-            if (rho * rho <= kSchulzTol) {
-                ok = true;
-                if ((r = transpose(cur, n, n, n, p->d_Xt, n, cs))) return r;
-                break;
-            }
-        }
-        if (ok) p->ns_strips++;
-        else p->ns_fallbacks++;
+    while (hist < 3 && c.h_n[hist] == n) hist++;
+    if (!p->schulz || hist == 0) return OCMP_OK;
+    const int64_t n4 = (int64_t)n * n / 4;
+    const float co[3][3] = {{1.f, 0.f, 0.f}, {2.f, -1.f, 0.f}, {3.f, -3.f, 1.f}};
+    const float* cc = co[hist - 1];
+    OCMP_LAUNCH(k_extrap<<<nblk(n4, 256), 256, 0, c.stream>>>(
+        n4, reinterpret_cast<const float4*>(c.H[0]), hist > 1 ? reinterpret_cast<const float4*>(c.H[1]) : nullptr,
+        hist > 2 ? reinterpret_cast<const float4*>(c.H[2]) : nullptr, cc[0], cc[1], cc[2],
+        reinterpret_cast<float4*>(c.cur)));
+    *pending = true;
+    return schulz_residual(p, c, W, mp, n);
+}
+
+// the residual is there: done (*pending false; *ok whether the iterate is taken) or one more step
+int schulz_step(Strip* p, StripChain& c, const float* W, int mp, int n, bool* pending, bool* ok) {
+    cudaStream_t cs = c.stream;
+    OCMP_CUDA(cudaEventSynchronize(c.ev_read));
+    float rho;
+    std::memcpy(&rho, c.h_rmax, sizeof(float));
+    *pending = false;
+    *ok = false;
+    if (!std::isfinite(rho) || rho >= c.rprev) return OCMP_OK;
+    if (rho <= kSchulzTol) {
+        *ok = true;
+        return OCMP_OK;
     }
+    c.rprev = rho;
+    int r = transpose(c.R, n, n, n, c.Rt, n, cs);
+    if (!r) r = copy2d(c.cur, n, n, n, c.nxt, n, 1.f, cs);
+    if (!r) r = gemm(p, n, n, n, c.cur, n, c.Rt, n, c.nxt, n, 1.f, 1.f, cs);
+    if (r) return r;
+    std::swap(c.cur, c.nxt);
+    p->ns_iters++;
+    if (rho * rho <= kSchulzTol) {
+        *ok = true;
+        return transpose(c.cur, n, n, n, c.Xt, n, cs);
+    }
+    if (++c.it >= kSchulzMax) return OCMP_OK;
+    *pending = true;
+    return schulz_residual(p, c, W, mp, n);
+}
+
+// End of an interface inversion: the fallback, the history. The end strip's inverse (step 0 of the chain)
+// starts the second strip's iteration (spectral radius 0.9, eight steps at 96 x 96 DG P2), but it lacks a
+// Schur update and would spoil the extrapolation (2 X_1 - X_0 for the third: 0.87, against 0.05 for X_1).
+int schulz_end(Strip* p, StripChain& c, const float* W, int mp, int n, int step, bool started, bool ok) {
+    cudaStream_t cs = c.stream;
+    if (ok) p->ns_strips++;
+    else if (started) p->ns_fallbacks++;
     if (!ok) {
-        int r = copy2d(W, mp, n, n, cur, n, 1.f, cs);
-        if (!r) r = gj_tiles(p, cur, n, 0, n, p->work[0], cs);
-        if (!r) r = transpose(cur, n, n, n, p->d_Xt, n, cs);
+        int r = copy2d(W, mp, n, n, c.cur, n, 1.f, cs);
+        if (!r) r = gj_tiles(p, c.cur, n, 0, n, c.work, cs);
+        if (!r) r = transpose(c.cur, n, n, n, c.Xt, n, cs);
         if (r) return r;
     }
     // the new inverse joins the history, the oldest buffer taking it
-    float* h = p->d_H[2];
-    p->d_H[2] = p->d_H[1];
-    p->d_H[1] = p->d_H[0];
-    p->d_H[0] = h;
-    p->h_n[2] = p->h_n[1];
-    p->h_n[1] = p->h_n[0];
-    p->h_n[0] = n;
-    OCMP_CUDA(cudaMemcpyAsync(h, cur, sizeof(float) * (size_t)n * n, cudaMemcpyDeviceToDevice, cs));
-    *X = cur;
+    float* h = c.H[2];
+    c.H[2] = c.H[1];
+    c.H[1] = c.H[0];
+    c.H[0] = h;
+    c.h_n[2] = step == 1 ? 0 : c.h_n[1];
+    c.h_n[1] = step == 1 ? 0 : c.h_n[0];
+    c.h_n[0] = n;
+    OCMP_CUDA(cudaMemcpyAsync(h, c.cur, sizeof(float) * (size_t)n * n, cudaMemcpyDeviceToDevice, cs));
     return OCMP_OK;
 }
 
 // Phase 2 of a block-diagonal-N strip after the Schur update: with X_I = W^-1 (W = S_II),
 //   G_II = X_I, G_IN = X_I Z, G_NI = -T, G_NN = X - T Z, T = Y X_I.
-int phase2_groups(Strip* p, int k, float* S, cudaStream_t cs) {
+int phase2_assemble(Strip* p, StripChain& c, int k, float* S) {
+    cudaStream_t cs = c.stream;
     const int mp = p->mp[k], nNp = p->nNp[k], n = mp - nNp;
-    float* Wi = nullptr;
-    int r = invert_interface(p, S + (int64_t)nNp * mp + nNp, mp, n, &Wi, cs);
-    if (!r) r = gemm(p, nNp, n, n, S + nNp, mp, p->d_Xt, n, p->d_T1, n, 1.f, 0.f, cs);
-    if (!r) r = transpose(S + (int64_t)nNp * mp, mp, n, nNp, p->d_Zt, n, cs);
-    if (!r) r = gemm(p, nNp, nNp, n, p->d_T1, n, p->d_Zt, n, S, mp, -1.f, 1.f, cs);
-    if (!r) r = gemm(p, n, nNp, n, Wi, n, p->d_Zt, n, S + (int64_t)nNp * mp, mp, 1.f, 0.f, cs);
-    if (!r) r = copy2d(p->d_T1, n, nNp, n, S + nNp, mp, -1.f, cs);
-    if (!r) r = copy2d(Wi, n, n, n, S + (int64_t)nNp * mp + nNp, mp, 1.f, cs);
+    int r = gemm(p, nNp, n, n, S + nNp, mp, c.Xt, n, c.T1, n, 1.f, 0.f, cs);
+    if (!r) r = transpose(S + (int64_t)nNp * mp, mp, n, nNp, c.Zt, n, cs);
+    if (!r) r = gemm(p, nNp, nNp, n, c.T1, n, c.Zt, n, S, mp, -1.f, 1.f, cs);
+    if (!r) r = gemm(p, n, nNp, n, c.cur, n, c.Zt, n, S + (int64_t)nNp * mp, mp, 1.f, 0.f, cs);
+    if (!r) r = copy2d(c.T1, n, nNp, n, S + nNp, mp, -1.f, cs);
+    if (!r) r = copy2d(c.cur, n, n, n, S + (int64_t)nNp * mp + nNp, mp, 1.f, cs);
     return r;
+}
+
+// S_k[I, I] -= A[I, J] G_prev[J, J] A[J, I], the couplings given by the lists at offset lists
+int schur_update(Strip* p, StripChain& c, int k, int prev, int64_t lists, const ocmp_space_s* s, const double* vals,
+                 float* S) {
+    if (p->nI[k] == 0 || p->nJ[prev] == 0) return OCMP_OK;
+    const int nI = p->nI[k], nJ = p->nJ[prev], nIp = pad(nI);
+    const int64_t s0 = p->s[k], sp = p->s[prev];
+    const int32_t* Irow = p->d_I + p->ioff[k];
+    const int32_t* Jrow = p->jrow + p->joff[prev];
+    const int32_t* cp = p->d_cptr + lists;
+    OCMP_LAUNCH(k_schur_t<<<dim3(nblk(nIp, 128), nblk(nJ, kSchurRows)), 128, 0, c.stream>>>(
+        nI, nJ, nIp, s0, sp, Irow, Jrow, p->d_J + p->joff[prev], cp, p->d_cb, p->d_ccol, vals, s->d_free,
+        p->d_G + p->goff[prev], p->mp[prev], c.T));
+    OCMP_LAUNCH(k_schur_u<<<dim3(nblk(nI, 4 * 128), nI), 128, 0, c.stream>>>(nI, nIp, p->nNp[k], s0, sp, Irow, Jrow, cp,
+                                                                           p->d_cb, p->d_crow, vals, s->d_free, c.T, S,
+                                                                           p->mp[k]));
+    return OCMP_OK;
+}
+
+// Phase 2 of up to one strip of each chain (-1: none), the chains' step-th, after their Schur updates:
+// the I pivots, the two chains' Newton-Schulz iterations in turns.
+int phase2(Strip* p, const int (&ks)[2], int step) {
+    bool pending[2] = {false, false}, started[2] = {false, false}, ok[2] = {false, false}, fast[2] = {false, false};
+    auto S = [&](int q) { return p->d_G + p->goff[ks[q]]; };
+    auto W = [&](int q) { return S(q) + (int64_t)p->nNp[ks[q]] * p->mp[ks[q]] + p->nNp[ks[q]]; };
+    auto n = [&](int q) { return p->mp[ks[q]] - p->nNp[ks[q]]; };
+    auto finish = [&](int q) {
+        const int r = schulz_end(p, p->chain[q], W(q), p->mp[ks[q]], n(q), step, started[q], ok[q]);
+        return r ? r : phase2_assemble(p, p->chain[q], ks[q], S(q));
+    };
+    for (int q = 0; q < 2; q++) {
+        const int k = ks[q];
+        if (k < 0) continue;
+        StripChain& c = p->chain[q];
+        fast[q] = p->schulz && p->fast[k];
+        if (!p->fast[k])
+            for (int& h : c.h_n) h = 0;
+        int r = fast[q] ? schulz_begin(p, c, W(q), p->mp[k], n(q), &pending[q])
+                        : gj_tiles(p, S(q), p->mp[k], p->nNp[k], p->mp[k], c.work, c.stream);
+        started[q] = pending[q];
+        if (!r && fast[q] && !pending[q]) r = finish(q);
+        if (r) return r;
+    }
+    while (pending[0] || pending[1])
+        for (int q = 0; q < 2; q++) {
+            if (!pending[q]) continue;
+            int r = schulz_step(p, p->chain[q], W(q), p->mp[ks[q]], n(q), &pending[q], &ok[q]);
+            if (!r && !pending[q]) r = finish(q);
+            if (r) return r;
+        }
+    return OCMP_OK;
 }
 
 }  // namespace
@@ -1028,8 +1123,10 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             }
         }
     }
-    // interface sets: I_k = dofs of strip k coupled to strip k-1 (by their row or their column),
-    // J_k = dofs of strip k coupled to strip k+1
+    // interface sets: I_k = dofs of strip k coupled to its previous strip (by their row or their
+    // column), the middle strip's to both neighbours; J_k = those coupled to its next strip
+    const int mid = p->mid = K / 2;
+    auto next_of = [&](int k) { return k < mid ? k + 1 : k - 1; };
     p->m.resize(K);
     p->nN.resize(K);
     p->nNp.resize(K);
@@ -1046,14 +1143,38 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         for (int64_t r = s0; r < s1; r++)
             for (int64_t q = rp[r]; q < rp[r + 1]; q++) {
                 const int64_t c = col[q];
-                if (c < s0) {
-                    inI[k][r - s0] = 1;
-                    inJ[k - 1][c - p->s[k - 1]] = 1;
-                } else if (c >= s1) {
-                    inJ[k][r - s0] = 1;
-                    inI[k + 1][c - s1] = 1;
-                }
+                if (c >= s0 && c < s1) continue;
+                const int o = c < s0 ? k - 1 : k + 1;
+                const bool outer = k != mid && next_of(k) == o;   // k is farther from the middle than o
+                (outer ? inJ : inI)[k][r - s0] = 1;
+                (outer ? inI : inJ)[o][c - p->s[o]] = 1;
             }
+    }
+    // the end strips have no previous one and may take any I: where the dofs coupled to the next strip
+    // form independent groups of at most 32 (a row of DG elements), the others, which makes them strips
+    // of the Newton-Schulz path like the rest (their I block then costs half the pivot tiles and starts
+    // the next strip's iteration)
+    for (const int k : {0, K - 1}) {
+        if (K == 1 || k == mid) continue;
+        const int64_t s0 = p->s[k], s1 = p->s[k + 1];
+        std::vector<int> par(p->m[k]), count(p->m[k], 0);
+        std::iota(par.begin(), par.end(), 0);
+        auto find = [&](int a) {
+            while (par[a] != a) a = par[a] = par[par[a]];
+            return a;
+        };
+        for (int i = 0; i < p->m[k]; i++)
+            if (inJ[k][i])
+                for (int64_t e = rp[s0 + i]; e < rp[s0 + i + 1]; e++)
+                    if (col[e] >= s0 && col[e] < s1 && inJ[k][col[e] - s0]) par[find(i)] = find((int)(col[e] - s0));
+        int largest = 0, nJ = 0;
+        for (int i = 0; i < p->m[k]; i++)
+            if (inJ[k][i]) {
+                nJ++;
+                largest = std::max(largest, ++count[find(i)]);
+            }
+        if (largest == 0 || largest > 32 || nJ == p->m[k]) continue;
+        for (int i = 0; i < p->m[k]; i++) inI[k][i] = !inJ[k][i];
     }
     p->mp.resize(K);
     p->goff.resize(K + 1);
@@ -1172,19 +1293,22 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         const int64_t s0 = p->s[k], s1 = p->s[k + 1];
         for (int64_t r = s0; r < s1; r++) {
             for (int64_t q = rp[r]; q < rp[r + 1]; q++) {
-                if (col[q] < s0) lo_pos.push_back((int32_t)q);
-                else if (col[q] >= s1) hi_pos.push_back((int32_t)q);
+                if (col[q] >= s0 && col[q] < s1) continue;
+                const bool next = k != mid && (col[q] >= s1) == (k < mid);
+                (next ? hi_pos : lo_pos).push_back((int32_t)q);
             }
             lo_ptr[r + 1] = (int32_t)lo_pos.size();
             hi_ptr[r + 1] = (int32_t)hi_pos.size();
         }
     }
-    // coupling lists of the I dofs to the previous strip's J dofs (the Schur update's sparse factors)
+    // coupling lists of the I dofs to the previous strip's J dofs (the Schur update's sparse factors):
+    // one list per I dof in the order of d_I; the middle strip's to the strip below it, and at the end
+    // those to the strip above
     std::vector<int32_t> cptr{0}, cb, crow, ccol;
-    for (int k = 0; k < K; k++) {
-        const int64_t s0 = p->s[k];
+    auto couple = [&](int k, int prev) {
         std::vector<std::vector<std::array<int32_t, 3>>> lists(p->nI[k]);
-        if (k > 0) {
+        if (prev >= 0 && prev < K) {
+            const int64_t s0 = p->s[k], s1 = p->s[k + 1], sp = p->s[prev], sq = p->s[prev + 1];
             auto entry = [&](int a, int32_t b) -> std::array<int32_t, 3>& {
                 for (auto& e : lists[a])
                     if (e[0] == b) return e;
@@ -1194,12 +1318,11 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             for (int a = 0; a < p->nI[k]; a++) {
                 const int64_t r = s0 + Ipos[p->ioff[k] + a];
                 for (int64_t q = rp[r]; q < rp[r + 1]; q++)
-                    if (col[q] < s0) entry(a, Jinv[col[q]])[1] = (int32_t)q;
+                    if (col[q] >= sp && col[q] < sq) entry(a, Jinv[col[q]])[1] = (int32_t)q;
             }
-            const int64_t sp = p->s[k - 1];
-            for (int64_t d = sp; d < s0; d++)
+            for (int64_t d = sp; d < sq; d++)
                 for (int64_t q = rp[d]; q < rp[d + 1]; q++)
-                    if (col[q] >= s0 && col[q] < p->s[k + 1]) entry(Iinv[col[q]], Jinv[d])[2] = (int32_t)q;
+                    if (col[q] >= s0 && col[q] < s1) entry(Iinv[col[q]], Jinv[d])[2] = (int32_t)q;
         }
         for (auto& l : lists) {
             std::sort(l.begin(), l.end());
@@ -1211,12 +1334,21 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             cptr.push_back((int32_t)cb.size());
             p->cmax = std::max(p->cmax, (int)l.size());
         }
-    }
-    const int64_t fast_floats = p->nfast ? (int64_t)8 * p->nIp_max * p->nIp_max +
-                                                (int64_t)(2 + kSide) * p->mp_max * p->nIp_max
+    };
+    for (int k = 0; k < K; k++) couple(k, k <= mid ? k - 1 : k + 1);
+    p->coff2 = (int64_t)cptr.size() - 1;
+    couple(mid, mid + 1);
+    // interface sizes of the strips that take the Newton-Schulz path; the second chain only where there
+    // are strips above the middle
+    int ns_max = 0;
+    for (int k = 0; k < K; k++)
+        if (p->fast[k]) ns_max = std::max(ns_max, p->mp[k] - p->nNp[k]);
+    const int chains = mid + 1 < K ? 2 : 1;
+    const int64_t fast_floats = p->nfast ? (int64_t)chains * (8 * (int64_t)ns_max * ns_max + 2 * (int64_t)p->mp_max * ns_max) +
+                                                (int64_t)kSide * p->mp_max * ns_max
                                           : 0;
-    const int64_t need = total * 4 + (int64_t)p->nJp_max * p->nIp_max * 4 +
-                         (int64_t)(kSide + 1) * (2 * p->mp_max * kNb + kNb * kNb) * 4 + fast_floats * 4;
+    const int64_t need = total * 4 + (int64_t)chains * p->nJp_max * p->nIp_max * 4 +
+                         (int64_t)(kSide + chains) * (2 * p->mp_max * kNb + kNb * kNb) * 4 + fast_floats * 4;
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     if ((size_t)need > fr) {
@@ -1242,11 +1374,15 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
     U(&p->d_crow, crow);
     U(&p->d_ccol, ccol);
     p->bytes += (int64_t)(cptr.size() + 3 * cb.size()) * 4;
-    A(&p->d_T, (size_t)std::max(1, p->nJp_max * p->nIp_max));
-    for (auto& w : p->work) {
+    auto work = [&](StripWork& w) {
         A(&w.P, (size_t)kNb * kNb);
         A(&w.Ck, (size_t)p->mp_max * kNb);
         A(&w.Rt, (size_t)p->mp_max * kNb);
+    };
+    for (auto& w : p->work) work(w);
+    for (int q = 0; q < chains; q++) {
+        work(p->chain[q].work);
+        A(&p->chain[q].T, (size_t)std::max<int64_t>(1, (int64_t)p->nJp_max * p->nIp_max));
     }
     A(&p->d_flag, 2);
     {
@@ -1310,18 +1446,29 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             }
             steps.push_back(t);
         };
-        // forward over all strips, backward from the last but one
-        for (int k = 0; k < K; k++) {
-            step(k, 0, p->sweep_grid);
-            steps.push_back(SweepStep{});
-        }
-        for (int k = K - 2; k >= 0; k--) {
-            step(k, 1, p->sweep_grid);
-            steps.push_back(SweepStep{});
-        }
+        // forward from both ends to the middle strip, backward from it; the strips of a pair on one half
+        // of the blocks each
+        const int half = p->sweep_grid / 2;
+        auto pair = [&](int k0, int k1, int mode) {
+            if (half > 0 && k0 >= 0 && k1 >= 0) {
+                step(k0, mode, half);
+                step(k1, mode, p->sweep_grid - half);
+                return;
+            }
+            for (const int k : {k0, k1})
+                if (k >= 0) {
+                    step(k, mode, p->sweep_grid);
+                    steps.push_back(SweepStep{});
+                }
+        };
+        const int up = K - 1 - mid;   // strips above the middle; below it are as many or one more
+        for (int t = mid - 1; t >= 0; t--) pair(mid - 1 - t, t < up ? mid + 1 + t : -1, 0);
+        pair(mid, -1, 0);
+        const int nfwd = (int)steps.size() / 2;
+        for (int t = 0; t < mid; t++) pair(mid - 1 - t, t < up ? mid + 1 + t : -1, 1);
         SweepArgs& a = p->sweep;
         a.nsteps = (int)steps.size() / 2;
-        a.nfwd = K;
+        a.nfwd = nfwd;
         int most = 1, words = 0;   // floats of a step's rows in a block, words of its lists
         for (const SweepStep& t : steps) {
             a.rows = std::max(a.rows, t.per);
@@ -1373,37 +1520,43 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         if (!st) st = strip_reset(p, nullptr);
     }
     if (p->nfast) {
-        const size_t i2 = (size_t)p->nIp_max * p->nIp_max, mi = (size_t)p->mp_max * p->nIp_max;
+        const size_t i2 = (size_t)ns_max * ns_max, mi = (size_t)p->mp_max * ns_max;
         U(&p->d_gptr, gptr);
         U(&p->d_gidx, gidx);
         U(&p->d_gcomp, gcomp);
-        A(&p->d_Xa, i2);
-        A(&p->d_Xb, i2);
-        A(&p->d_R, i2);
-        A(&p->d_Rt, i2);
-        A(&p->d_Xt, i2);
-        for (float*& h : p->d_H) A(&h, i2);
-        A(&p->d_T1, mi);
-        A(&p->d_Zt, mi);
+        for (int q = 0; q < chains; q++) {
+            StripChain& c = p->chain[q];
+            A(&c.Xa, i2);
+            A(&c.Xb, i2);
+            A(&c.R, i2);
+            A(&c.Rt, i2);
+            A(&c.Xt, i2);
+            for (float*& h : c.H) A(&h, i2);
+            A(&c.T1, mi);
+            A(&c.Zt, mi);
+            A(&c.rmax, 1);
+            if (!st && cudaMallocHost((void**)&c.h_rmax, sizeof(unsigned)) != cudaSuccess)
+                st = fail(OCMP_ERR_NOMEM, "strip preconditioner: pinned flag");
+        }
         for (float*& y : p->d_Yt) A(&y, mi);
-        A(&p->d_rmax, 1);
-        if (!st && cudaMallocHost((void**)&p->h_rmax, sizeof(unsigned)) != cudaSuccess)
-            st = fail(OCMP_ERR_NOMEM, "strip preconditioner: pinned flag");
         p->bytes += (int64_t)(gptr.size() + 2 * gidx.size()) * 4;
     }
     U(&p->jrow, Jpos);
     p->bytes += (int64_t)Jpos.size() * 4;
     // every buffer a kernel of the factorisation or the sweeps dereferences must exist
     if (!st) {
-        const void* need_ptr[] = {p->d_perm, p->d_pinv, p->d_G, p->d_cptr, p->d_T, p->d_flag, p->d_prow, p->d_rdof,
-                                  p->d_steps, p->d_words, p->d_state, p->work[0].P, p->work[0].Ck, p->work[0].Rt};
-        bool ok = std::all_of(std::begin(need_ptr), std::end(need_ptr), [](const void* q) { return q != nullptr; });
-        if (p->nfast) {
-            const void* fast_ptr[] = {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Xa, p->d_Xb, p->d_R, p->d_Rt, p->d_Xt,
-                                      p->d_H[0], p->d_H[1], p->d_H[2], p->d_T1, p->d_Zt, p->d_Yt[0], p->d_Yt[1],
-                                      p->d_Yt[2], p->d_rmax, p->h_rmax};
-            ok = ok && std::all_of(std::begin(fast_ptr), std::end(fast_ptr), [](const void* q) { return q != nullptr; });
+        std::vector<const void*> need_ptr{p->d_perm, p->d_pinv, p->d_G, p->d_cptr, p->d_flag, p->d_prow, p->d_rdof,
+                                          p->d_steps, p->d_words, p->d_state, p->work[0].P, p->work[0].Ck, p->work[0].Rt};
+        for (int q = 0; q < chains; q++) {
+            const StripChain& c = p->chain[q];
+            need_ptr.insert(need_ptr.end(), {c.T, c.work.P, c.work.Ck, c.work.Rt});
+            if (p->nfast)
+                need_ptr.insert(need_ptr.end(), {c.Xa, c.Xb, c.R, c.Rt, c.Xt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax,
+                                                 c.h_rmax});
         }
+        if (p->nfast)
+            need_ptr.insert(need_ptr.end(), {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Yt[0], p->d_Yt[1], p->d_Yt[2]});
+        bool ok = std::all_of(need_ptr.begin(), need_ptr.end(), [](const void* q) { return q != nullptr; });
         if (p->nell) ok = ok && p->d_blob && p->d_erow && p->d_epos && p->d_edst;
         if (!ok) st = fail(OCMP_ERR_NOMEM, "strip preconditioner: a work buffer was not allocated");
     }
@@ -1416,10 +1569,13 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             st = fail(OCMP_ERR_CUDA, "cudaStreamCreateWithFlags");
     if (!st) {
         int lo = 0, hi = 0;
-        if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess ||
-            cudaStreamCreateWithPriority(&p->chain, cudaStreamNonBlocking, hi) != cudaSuccess ||
-            cudaEventCreateWithFlags(&p->ev_done, cudaEventDisableTiming) != cudaSuccess)
-            st = fail(OCMP_ERR_CUDA, "strip preconditioner: chain stream");
+        if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess)
+            st = fail(OCMP_ERR_CUDA, "strip preconditioner: stream priorities");
+        for (int q = 0; q < chains && !st; q++)
+            if (cudaStreamCreateWithPriority(&p->chain[q].stream, cudaStreamNonBlocking, hi) != cudaSuccess ||
+                cudaEventCreateWithFlags(&p->chain[q].ev_read, cudaEventDisableTiming) != cudaSuccess ||
+                cudaEventCreateWithFlags(&p->chain[q].ev_done, cudaEventDisableTiming) != cudaSuccess)
+                st = fail(OCMP_ERR_CUDA, "strip preconditioner: chain stream");
     }
     p->ev_phase1.assign(K, nullptr);
     for (int k = 0; k < K && !st; k++)
@@ -1454,7 +1610,8 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
     p->gemm_flops_pending = 0;
     p->gemm_bytes_pending = 0;
     p->ns_iters = p->ns_strips = p->ns_fallbacks = 0;
-    for (int& h : p->h_n) h = 0;
+    for (auto& c : p->chain)
+        for (int& h : c.h_n) h = 0;
     OCMP_CUDA(cudaEventRecord(p->fev[0], st));
     OCMP_CUDA(cudaMemsetAsync(p->d_flag, 0, 2 * sizeof(int), st));
     {
@@ -1464,11 +1621,18 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
     }
     OCMP_CUDA(cudaEventRecord(p->ev_start, st));
     for (int q = 0; q < kSide; q++) OCMP_CUDA(cudaStreamWaitEvent(p->side[q], p->ev_start, 0));
-    cudaStream_t cs = p->chain;
-    OCMP_CUDA(cudaStreamWaitEvent(cs, p->ev_start, 0));
-    // phase 1: fill every strip and eliminate its N pivots, strips spread over the side streams
-    for (int k = 0; k < K; k++) {
-        const int q = k % kSide;
+    const int mid = p->mid, chains = mid + 1 < K ? 2 : 1;
+    for (int q = 0; q < chains; q++) OCMP_CUDA(cudaStreamWaitEvent(p->chain[q].stream, p->ev_start, 0));
+    // phase 1: fill every strip and eliminate its N pivots, strips spread over the side streams in the
+    // order in which phase 2 takes them
+    std::vector<int> order;
+    for (int t = 0; t < mid; t++) {
+        order.push_back(t);
+        if (K - 1 - t > mid) order.push_back(K - 1 - t);
+    }
+    order.push_back(mid);
+    for (int o = 0; o < K; o++) {
+        const int k = order[o], q = o % kSide;
         cudaStream_t ss = p->side[q];
         const int mp = p->mp[k];
         float* S = p->d_G + p->goff[k];
@@ -1476,38 +1640,34 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
         OCMP_LAUNCH(k_fill_strip<<<nblk(mp, 128), 128, 0, ss>>>(mp, p->s[k], p->d_perm + p->poff[k], p->d_pinv, s->d_rowptr,
                                                                s->d_col, vals, s->d_free, p->s[k + 1], S));
         const int r = p->schulz && p->fast[k] ? phase1_groups(p, k, S, q, ss)
-                                              : gj_tiles(p, S, mp, 0, p->nNp[k], p->work[1 + q], ss);
+                                              : gj_tiles(p, S, mp, 0, p->nNp[k], p->work[q], ss);
         if (r) return r;
         OCMP_CUDA(cudaEventRecord(p->ev_phase1[k], ss));
     }
-    // phase 2 on the chain stream, strip after strip: the Schur update from the previous strip's
-    // inverse, then the I pivots
-    for (int k = 0; k < K; k++) {
-        OCMP_CUDA(cudaStreamWaitEvent(cs, p->ev_phase1[k], 0));
-        const int mp = p->mp[k];
-        const int64_t s0 = p->s[k];
-        float* S = p->d_G + p->goff[k];
-        if (k > 0 && p->nI[k] > 0 && p->nJ[k - 1] > 0) {
-            const int nI = p->nI[k], nJ = p->nJ[k - 1], nIp = pad(nI);
-            const int64_t sp = p->s[k - 1];
-            const int32_t* Irow = p->d_I + p->ioff[k];
-            const int32_t* Jrow = p->jrow + p->joff[k - 1];
-            const int32_t* cp = p->d_cptr + p->ioff[k];
-            OCMP_LAUNCH(k_schur_t<<<dim3(nblk(nIp, 128), nblk(nJ, kSchurRows)), 128, 0, cs>>>(
-                nI, nJ, nIp, s0, sp, Irow, Jrow, p->d_J + p->joff[k - 1], cp, p->d_cb, p->d_ccol, vals, s->d_free,
-                p->d_G + p->goff[k - 1], p->mp[k - 1], p->d_T));
-            OCMP_LAUNCH(k_schur_u<<<dim3(nblk(nI, 4 * 128), nI), 128, 0, cs>>>(nI, nIp, p->nNp[k], s0, sp, Irow, Jrow,
-                                                                              cp, p->d_cb, p->d_crow, vals, s->d_free,
-                                                                              p->d_T, S, mp));
+    // phase 2: the two chains side by side, then the middle strip on the first
+    for (int t = 0; t <= mid; t++) {
+        const int ks[2] = {t, t < mid && K - 1 - t > mid ? K - 1 - t : -1};
+        for (int q = 0; q < 2; q++) {
+            const int k = ks[q];
+            if (k < 0) continue;
+            StripChain& c = p->chain[q];
+            float* S = p->d_G + p->goff[k];
+            OCMP_CUDA(cudaStreamWaitEvent(c.stream, p->ev_phase1[k], 0));
+            int r = OCMP_OK;
+            const int prev = q == 0 ? k - 1 : k + 1;
+            if (prev >= 0 && prev < K) r = schur_update(p, c, k, prev, p->ioff[k], s, vals, S);
+            if (!r && k == mid && mid + 1 < K) {
+                OCMP_CUDA(cudaEventRecord(p->chain[1].ev_done, p->chain[1].stream));
+                OCMP_CUDA(cudaStreamWaitEvent(c.stream, p->chain[1].ev_done, 0));
+                r = schur_update(p, c, k, mid + 1, p->coff2, s, vals, S);
+            }
+            if (r) return r;
         }
-        if (!p->fast[k])
-            for (int& h : p->h_n) h = 0;
-        const int r = p->schulz && p->fast[k] ? phase2_groups(p, k, S, cs) : gj_tiles(p, S, mp, p->nNp[k], mp, p->work[0], cs);
-        if (r) return r;
+        if (const int r = phase2(p, ks, t)) return r;
     }
     OCMP_CUDA(cudaGetLastError());
-    OCMP_CUDA(cudaEventRecord(p->ev_done, cs));
-    OCMP_CUDA(cudaStreamWaitEvent(st, p->ev_done, 0));
+    OCMP_CUDA(cudaEventRecord(p->chain[0].ev_done, p->chain[0].stream));
+    OCMP_CUDA(cudaStreamWaitEvent(st, p->chain[0].ev_done, 0));
     OCMP_CUDA(cudaEventRecord(p->fev[1], st));
     int flags[2] = {0, 0};
     OCMP_CUDA(cudaMemcpyAsync(flags, p->d_flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -1,6 +1,8 @@
 // The block elimination's two sweeps over the strips as one cooperative launch: forward
-// y_k = G_k (b_k - A_k,k-1 y_k-1), backward x_k = y_k - G_k A_k,k+1 x_k+1, one step per strip and
-// sweep, each a dense matrix-vector product whose right-hand side needs the step before.
+// y_k = G_k (b_k - A_k,p y_p), p the neighbour farther from the middle strip (both, for that one),
+// backward x_k = y_k - G_k A_k,q x_q, q the nearer one: from both ends to the middle and back, one step
+// per pair of strips and sweep, each a dense matrix-vector product whose right-hand side needs the step
+// before. Half of the blocks take either strip of a pair.
 //
 // What bounds a step is the way from one block's result to the next step's right-hand side, not the
 // bytes: a strip of 1,152 dofs holds 5.3 MB, 1.2 us of L2 or 0.8 us of HBM, and none of them depends on
@@ -15,8 +17,8 @@
 //    FP64 instruction takes its pipe for 64 clocks), and read as such words as well;
 //  - the few loads of a step that go to registers are issued one or two steps ahead.
 //
-// Measured (us per preconditioner application): 16,641 pressure dofs in 17 strips 226 -> 85, 110,592 dofs
-// in 96 strips 1,430 -> 690; before, two launches per strip and sweep, replayed from a graph. A step is
+// Measured (us per preconditioner application): 16,641 pressure dofs in 17 strips 226 -> 85 in one launch
+// -> 49 from both ends; before, two launches per strip and sweep, replayed from a graph. A step is
 // 5,000 clocks: 1,500 until the polled results are there, 1,500 for the product, the rest the gather,
 // the stores and the block's own barriers.
 #pragma once
