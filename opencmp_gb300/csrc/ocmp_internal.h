@@ -207,8 +207,22 @@ void strip_stats(const Strip* p, ocmp_strip_stats_t* out);
 void strip_set_timing(Strip* p, bool on);
 void strip_set_gemm(Strip* p, int kind);
 void strip_set_schulz(Strip* p, bool on);
-// C = beta C + alpha A B^T on the tensor cores (ocmp_tcgemm.cu): FP32 operands, 3xTF32 products;
-// M, N multiples of 128, K of 32; *err set when a bounded wait gave up
+// C = beta C0 + alpha A B^T, all row-major; C0 null with beta != 0 is the identity
+struct DenseProduct {
+    int M, N, K;
+    const float* A;
+    int64_t lda;
+    const float* B;
+    int64_t ldb;
+    float* C;
+    int64_t ldc;
+    float alpha, beta;
+    const float* C0;
+    int64_t ldc0;
+};
+// one or two products in one launch on the tensor cores (ocmp_tcgemm.cu): FP32 operands, 3xTF32
+// products; M, N multiples of 128, K of 32; *err set when a bounded wait gave up
+int tc_products(const DenseProduct* p, int count, int* err, cudaStream_t st);
 int tc_gemm_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
                float alpha, float beta, int* err, cudaStream_t st);
 int space_build_sell(ocmp_space_s* s);

@@ -1,4 +1,4 @@
-// Dense FP32 product on the 5th-generation tensor cores (sm_103a): C = beta C + alpha A B^T with A
+// Dense FP32 products on the 5th-generation tensor cores (sm_103a): C = beta C0 + alpha A B^T with A
 // (M x K) and B (N x K) row-major, K contiguous, the operation the strip factorisation
 // (ocmp_strip.cu) spends its flops in. FP32 accuracy from TF32 tensor-core products by the
 // split-operand scheme: with a = a_h + a_l (a_h = a truncated to TF32, which is what the tensor core
@@ -6,13 +6,20 @@
 // FP32 accumulator in tensor memory. The dropped term A_l B_l and the truncation of the low parts
 // leave about 2^-21 relative error per product, against 2^-24 for FP32 FMAs.
 //
-// One CTA computes one 128 x 128 tile of C with 6 warps:
+// A launch computes one or two such products. The products of the strip factorisation's chains are small
+// (25 tiles at an interface of 640), one after the other, and a CTA's time is its K loop: 1.2 us per
+// slice of 32, of which the shared-memory traffic (the boxes written, split and read by three MMAs) is
+// 0.75. So where a launch has few tiles, the CTAs of a cluster share a tile's K range and add their
+// accumulators through distributed shared memory, in rank order.
+//
+// One CTA computes one 128 x 128 tile of C, or its share of one, with 6 warps:
 //   warp 0     TMA producer: 128 x 32 FP32 boxes of A and B (128-byte rows, 128B swizzle) into a
 //              3-stage shared-memory ring (cp.async.bulk.tensor, mbarrier completion);
 //   warps 2-5  split the staged boxes into their low parts (x - trunc_tf32(x), same swizzled layout,
 //              elementwise), then run the epilogue: tcgen05.ld of the accumulator (each warp its 32
-//              TMEM lanes = rows) into a staging tile in the idle stage buffers, then C read, scaled
-//              and written row by row (512 contiguous bytes per row and warp instruction);
+//              TMEM lanes = rows) into a staging tile in the idle stage buffers, then C0 read, scaled
+//              and C written row by row (512 contiguous bytes per row and warp instruction), in a
+//              cluster each CTA its share of the rows;
 //   warp 1     allocates 128 TMEM columns, and one thread issues the tcgen05.mma.kind::tf32
 //              instructions (M = 128, N = 128, K = 8) and the tcgen05.commit arrivals that free the
 //              stages and signal the epilogue.
@@ -22,6 +29,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -37,6 +45,7 @@ constexpr int kBoxBytes = TBM * TBK * 4;            // 16 KiB, one 128 x 32 FP32
 constexpr int kStageBytes = 4 * kBoxBytes;          // A, B, A_low, B_low
 constexpr int kTcSmem = TST * kStageBytes + 1024 + 256;
 constexpr int kTcThreads = 192;
+constexpr int SLD = TBN + 4;                        // staging tile: 16-byte aligned rows, conflict-free float4 writes
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t mbar) {
     asm volatile(
@@ -72,9 +81,38 @@ __device__ __forceinline__ void mma_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
 
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 cluster_read(uint32_t addr, int rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(at)
+                 : "memory");
+    return v;
+}
+
+struct TcTask {
+    float* C;
+    const float* C0;   // null with beta != 0: the identity
+    int64_t ldc, ldc0;
+    float alpha, beta;
+    int nk, tiles_n, tiles;
+};
+struct TcTasks {
+    TcTask t[2];
+};
+struct TcMaps {
+    CUtensorMap a[2], b[2];
+};
+
+// grid: the tiles of both products; z: the CTAs of a cluster, which share a tile's K range
 __global__ void __launch_bounds__(kTcThreads, 1)
-    tc_gemm_nt_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int K,
-                      float* __restrict__ C, int64_t ldc, float alpha, float beta, int* __restrict__ err) {
+    tc_products_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcTasks tasks,
+                       int* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = saddr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -90,8 +128,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nk = K / TBK;
-    const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
+    const int which = (int)blockIdx.x >= tasks.t[0].tiles;
+    const TcTask& task = tasks.t[which];
+    const CUtensorMap* ta = &maps.a[which];
+    const CUtensorMap* tb = &maps.b[which];
+    const int tile = blockIdx.x - (which ? tasks.t[0].tiles : 0);
+    const int m0 = tile / task.tiles_n * TBM, n0 = tile % task.tiles_n * TBN;
+    const int share = gridDim.z, rank = blockIdx.z;
+    const int k0 = task.nk * rank / share, nk = task.nk * (rank + 1) / share - k0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TST; s++) {
@@ -119,6 +163,40 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         atomicExch(err, 1);
     };
 
+    // rows r0 .. r0 + count - 1 of the tile, from the staging tiles of the cluster's CTAs
+    auto write_rows = [&](int r0, int count) {
+#pragma unroll 4
+        for (int rr = 0; rr < count; rr++) {
+            const int r = r0 + rr;
+            const uint32_t at = base + 4u * (r * SLD + 4 * lane);
+            float4 a;
+            if (share == 1) a = *reinterpret_cast<const float4*>(gbase + 4 * (r * SLD + 4 * lane));
+            else {
+                a = cluster_read(at, 0);
+                for (int c = 1; c < share; c++) {
+                    const float4 v = cluster_read(at, c);
+                    a.x += v.x;
+                    a.y += v.y;
+                    a.z += v.z;
+                    a.w += v.w;
+                }
+            }
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (task.beta != 0.f) {
+                if (task.C0) o = *(reinterpret_cast<const float4*>(task.C0 + (int64_t)(m0 + r) * task.ldc0 + n0) + lane);
+                else {
+                    const int d = m0 + r - n0 - 4 * lane;   // the diagonal's column in this quad
+                    o = make_float4(d == 0 ? 1.f : 0.f, d == 1 ? 1.f : 0.f, d == 2 ? 1.f : 0.f, d == 3 ? 1.f : 0.f);
+                }
+            }
+            o.x = task.alpha * a.x + task.beta * o.x;
+            o.y = task.alpha * a.y + task.beta * o.y;
+            o.z = task.alpha * a.z + task.beta * o.z;
+            o.w = task.alpha * a.w + task.beta * o.w;
+            *(reinterpret_cast<float4*>(task.C + (int64_t)(m0 + r) * task.ldc + n0) + lane) = o;
+        }
+    };
+
     if (warp == 0) {
         if (lane == 0) {
             int issued = 0;
@@ -130,8 +208,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
                 const uint32_t st = base + s * kStageBytes;
                 mbar_expect_tx(full_b(s), 2 * kBoxBytes);
-                tma_load_2d(st, &ta, kb * TBK, m0, full_b(s));
-                tma_load_2d(st + kBoxBytes, &tb, kb * TBK, n0, full_b(s));
+                tma_load_2d(st, ta, (k0 + kb) * TBK, m0, full_b(s));
+                tma_load_2d(st + kBoxBytes, tb, (k0 + kb) * TBK, n0, full_b(s));
                 issued = kb + 1;
             }
             // drain: every issued box must have landed before the CTA may exit
@@ -197,10 +275,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (ok && mbar_wait(accum_b, 0, abort)) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // TMEM lanes 32q..32q+31 are the tile's rows; each thread takes its row's 128 columns
-            // into a staging tile in the (now idle) stage buffers, then the warp writes C row by
-            // row, 512 contiguous bytes per row
+            // into a staging tile in the (now idle) stage buffers
             const int q = warp & 3;
-            constexpr int SLD = TBN + 4;            // 16-byte aligned rows, conflict-free float4 writes
             float* stg = reinterpret_cast<float*>(gbase) + q * (32 * SLD);
 #pragma unroll 1
             for (int c0 = 0; c0 < TBN; c0 += 32) {
@@ -225,21 +301,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                     __uint_as_float(r[v + 3]));
             }
             __syncwarp();
-#pragma unroll 4
-            for (int rr = 0; rr < 32; rr++) {
-                const float4 a = *reinterpret_cast<const float4*>(stg + rr * SLD + 4 * lane);
-                float4* p = reinterpret_cast<float4*>(C + ((int64_t)m0 + 32 * q + rr) * ldc + n0) + lane;
-                float4 o = beta != 0.f ? *p : make_float4(0.f, 0.f, 0.f, 0.f);
-                o.x = alpha * a.x + beta * o.x;
-                o.y = alpha * a.y + beta * o.y;
-                o.z = alpha * a.z + beta * o.z;
-                o.w = alpha * a.w + beta * o.w;
-                *p = o;
-            }
+            if (share == 1) write_rows(32 * q, 32);
         } else if (ok) {
             give_up();
         }
     }
+    // every thread of every CTA comes here, also after a wait that gave up
+    __syncwarp();
+    if (share > 1) cluster_sync();
+    if (share > 1 && warp >= 2) write_rows(rank * (TBM / share) + (warp - 2) * (32 / share), 32 / share);
+    __syncwarp();
+    if (share > 1) cluster_sync();   // the others may still read this CTA's staging tile
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (*abort && warp == 1 && lane == 0) {
@@ -287,29 +359,66 @@ int make_map(CUtensorMap* map, const float* p, int64_t rows, int64_t cols, int64
 
 }  // namespace
 
-int tc_gemm_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
-               float alpha, float beta, int* err, cudaStream_t st) {
-    if (M <= 0 || N <= 0 || K <= 0 || M % TBM || N % TBN || K % TBK)
-        return fail(OCMP_ERR_ARG, "tensor-core product: M, N must be multiples of 128 and K of 32");
-    if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15 || (lda | ldb) & 3 || ldc & 3 ||
-        reinterpret_cast<uintptr_t>(C) & 15)
-        return fail(OCMP_ERR_ARG, "tensor-core product: operands must be 16-byte aligned");
+// CTAs per tile: as many as keep the launch within about two thirds of the chip, so that the other
+// chain's products and the side streams' run beside it, with at least two slices of K each. At 50 tiles
+// of K = 640 one CTA per tile takes 18.4 us, two 15.4; the direct solve at an interface of 640 (25 and 50
+// tiles a launch) 20.5 and 19.5 ms.
+static int tc_share(int tiles, int nk) {
+    constexpr int kTarget = 104;
+    return tiles * 4 <= kTarget && nk >= 8 ? 4 : tiles * 2 <= kTarget && nk >= 4 ? 2 : 1;
+}
+
+int tc_products(const DenseProduct* p, int count, int* err, cudaStream_t st) {
+    for (int q = 0; q < count; q++) {
+        const DenseProduct& d = p[q];
+        if (d.M <= 0 || d.N <= 0 || d.K <= 0 || d.M % TBM || d.N % TBN || d.K % TBK)
+            return fail(OCMP_ERR_ARG, "tensor-core product: M, N must be multiples of 128 and K of 32");
+        if ((reinterpret_cast<uintptr_t>(d.A) | reinterpret_cast<uintptr_t>(d.B) | reinterpret_cast<uintptr_t>(d.C) |
+             reinterpret_cast<uintptr_t>(d.C0)) & 15 || (d.lda | d.ldb | d.ldc | d.ldc0) & 3)
+            return fail(OCMP_ERR_ARG, "tensor-core product: operands must be 16-byte aligned");
+    }
     int r = get_encode();
     if (r) return r;
     static thread_local int attr_dev = -1;
     int dev = 0;
     OCMP_CUDA(cudaGetDevice(&dev));
     if (attr_dev != dev) {
-        OCMP_CUDA(cudaFuncSetAttribute(tc_gemm_nt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
+        OCMP_CUDA(cudaFuncSetAttribute(tc_products_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
         attr_dev = dev;
     }
-    CUtensorMap ta, tb;
-    if ((r = make_map(&ta, A, M, K, lda))) return r;
-    if ((r = make_map(&tb, B, N, K, ldb))) return r;
-    const dim3 g(N / TBN, M / TBM);
-    OCMP_LAUNCH(tc_gemm_nt_kernel<<<g, kTcThreads, kTcSmem, st>>>(ta, tb, K, C, ldc, alpha, beta, err));
-    OCMP_CUDA(cudaGetLastError());
+    TcMaps maps;
+    TcTasks tasks{};
+    int tiles = 0, nk = 1 << 30;
+    for (int q = 0; q < 2; q++) {
+        const DenseProduct& d = p[q < count ? q : 0];
+        if ((r = make_map(&maps.a[q], d.A, d.M, d.K, d.lda))) return r;
+        if ((r = make_map(&maps.b[q], d.B, d.N, d.K, d.ldb))) return r;
+        if (q >= count) break;
+        tasks.t[q] = TcTask{d.C, d.C0, d.ldc, d.ldc0, d.alpha, d.beta, d.K / TBK, d.N / TBN, (d.M / TBM) * (d.N / TBN)};
+        tiles += tasks.t[q].tiles;
+        nk = std::min(nk, tasks.t[q].nk);
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    const int share = tc_share(tiles, nk);
+    cfg.gridDim = dim3(tiles, 1, share);
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = kTcSmem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = share;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchKernelEx(&cfg, tc_products_kernel, maps, tasks, err)));
     return OCMP_OK;
+}
+
+int tc_gemm_nt(int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
+               float alpha, float beta, int* err, cudaStream_t st) {
+    const DenseProduct p{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, C, ldc};
+    return tc_products(&p, 1, err, st);
 }
 
 }  // namespace ocmp

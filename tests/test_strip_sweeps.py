@@ -51,3 +51,25 @@ def test_sweeps_in_one_launch(gpu_lib, dim, kind, order, n, precision):
     r = (b - S @ xs[0])[free].norm().item()
     assert r <= TOL * 1.01 * r0, (r, r0, info.iterations)
     assert torch.equal(xs[0][~free], x0[~free])
+
+
+@pytest.mark.parametrize('M_,N,K', [(128, 128, 32), (128, 128, 96), (256, 128, 224), (640, 640, 640), (640, 512, 288),
+                                    (640, 768, 128), (1152, 1152, 128), (1152, 128, 1184)])
+def test_tensor_core_product_over_shares(gpu_lib, M_, N, K):
+    """The tensor-core product where a tile's K range is shared by one, two or four CTAs, evenly or not:
+    against FP64, to the split scheme's bound (the existing comparison's 2e-5 of sum |a||b|)."""
+    import ctypes as C
+    import torch
+    g = torch.Generator(device='cuda').manual_seed(M_ + 3 * N + 7 * K)
+    A = torch.randn(M_, K, device='cuda', generator=g)
+    B = torch.randn(N, K, device='cuda', generator=g)
+    for alpha, beta in ((1.0, 0.0), (-1.0, 1.0), (0.5, -2.0)):
+        C0 = torch.randn(M_, N, device='cuda', generator=g)
+        out = C0.clone()
+        st = gpu_lib.load().ocmp_dense_gemm_nt(1, M_, N, K, C.c_void_p(A.data_ptr()), K, C.c_void_p(B.data_ptr()), K,
+                                               C.c_void_p(out.data_ptr()), N, alpha, beta,
+                                               C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == gpu_lib.OK, gpu_lib.last_error()
+        ref = alpha * (A.double() @ B.double().T) + beta * C0.double()
+        scale = (A.double().abs() @ B.double().abs().T) + abs(beta) * C0.double().abs()
+        assert ((out.double() - ref).abs() / scale).max().item() <= 2e-5
