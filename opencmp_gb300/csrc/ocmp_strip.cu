@@ -35,8 +35,8 @@
 // product; phase 2 subtracts the Schur update from W0 and inverts it by Newton-Schulz iteration
 // started from the previous strip's interface inverse (two steps on a uniform DG mesh), then
 // assembles G_k from the 2 x 2 block inverse with three dense products.
-// The dense products are C = beta C + alpha A B^T with both operands K-contiguous: FP32 SIMT
-// (sgemm_nt) or the tensor cores (tc_gemm_nt, ocmp_tcgemm.cu).
+// The dense products are C = beta C0 + alpha A B^T with both operands K-contiguous: FP32 SIMT
+// (sgemm_nt) or the tensor cores (tc_products, ocmp_tcgemm.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,6 +55,7 @@ namespace ocmp {
 
 constexpr int kNb = 128;   // Gauss-Jordan tile and padding granule
 constexpr int kSide = 3;   // side streams of phase 1
+constexpr int kAhead = 4;  // pairs of strips that the launches of phase 1 are ahead of phase 2
 
 struct StripWork {
     float* P = nullptr;    // pivot-tile inverse, kNb x kNb
@@ -68,22 +69,20 @@ struct StripChain {
     cudaStream_t stream = nullptr;
     StripWork work;
     float* T = nullptr;              // Schur update: G_prev[J, J] A[J, I] (nJ x nIp)
-    float* Xa = nullptr;             // Newton-Schulz iterates, residual, transposes
-    float* Xb = nullptr;
-    float* R = nullptr;
-    float* Rt = nullptr;
-    float* Xt = nullptr;
-    float* H[3] = {};                // the last three interface inverses, newest first (Newton-Schulz starts)
+    // Newton-Schulz: buffers of an n x n matrix followed by its transpose; H: the last three interface
+    // inverses, newest first, cur and nxt: the iterate and the next one (they change places)
+    float* H[3] = {};
     int h_n[3] = {0, 0, 0};          // their padded sizes (0: none)
+    float* cur = nullptr;
+    float* nxt = nullptr;
+    float* Rt = nullptr;             // the residual's transpose
     float* T1 = nullptr;
     float* Zt = nullptr;
-    unsigned* rmax = nullptr;
+    unsigned* rmax = nullptr;        // the residuals' norms
     unsigned* h_rmax = nullptr;      // pinned
     cudaEvent_t ev_read = nullptr;   // the residual's copy
     cudaEvent_t ev_done = nullptr;   // the chain's last strip
     // a strip in progress
-    float* cur = nullptr;
-    float* nxt = nullptr;
     float rprev = 0.f;
     int it = 0;
 };
@@ -165,13 +164,15 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 inline int pad(int64_t v) { return (int)((v + kNb - 1) / kNb * kNb); }
 
 // ------------------------------------------------------------------ dense products (FP32 SIMT)
-// C[M x N] = beta C + alpha A[M x K] B[N x K]^T, row-major with leading dimensions lda/ldb/ldc;
+// C[M x N] = beta C0 + alpha A[M x K] B[N x K]^T (DenseProduct), row-major with leading dimensions;
 // M, N multiples of 128, K a multiple of 16, rows 16-byte aligned. 256 threads, 128 x 128 tile,
 // 8 x 8 outputs per thread, double-buffered K slices of 16.
 constexpr int GB = 128, GK = 16;
-__global__ void __launch_bounds__(256) sgemm_nt(int M, int N, int K, const float* __restrict__ A, int64_t lda,
-                                                const float* __restrict__ B, int64_t ldb, float* __restrict__ C,
-                                                int64_t ldc, float alpha, float beta) {
+__global__ void __launch_bounds__(256) sgemm_nt(const DenseProduct d) {
+    const float* __restrict__ A = d.A;
+    const float* __restrict__ B = d.B;
+    const int M = d.M, N = d.N, K = d.K;
+    const int64_t lda = d.lda, ldb = d.ldb;
     __shared__ __align__(16) float As[2][GK][GB + 4];
     __shared__ __align__(16) float Bs[2][GK][GB + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -234,13 +235,17 @@ __global__ void __launch_bounds__(256) sgemm_nt(int M, int N, int K, const float
         const int64_t r = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            float4* p = reinterpret_cast<float4*>(C + r * ldc + n0 + h * 64 + tx * 4);
-            float4 o = beta != 0.f ? *p : make_float4(0.f, 0.f, 0.f, 0.f);
-            o.x = alpha * acc[i][h * 4 + 0] + beta * o.x;
-            o.y = alpha * acc[i][h * 4 + 1] + beta * o.y;
-            o.z = alpha * acc[i][h * 4 + 2] + beta * o.z;
-            o.w = alpha * acc[i][h * 4 + 3] + beta * o.w;
-            *p = o;
+            const int64_t c = n0 + h * 64 + tx * 4;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (d.beta != 0.f)
+                o = d.C0 ? *reinterpret_cast<const float4*>(d.C0 + r * d.ldc0 + c)
+                         : make_float4(r == c ? 1.f : 0.f, r == c + 1 ? 1.f : 0.f, r == c + 2 ? 1.f : 0.f,
+                                       r == c + 3 ? 1.f : 0.f);
+            o.x = d.alpha * acc[i][h * 4 + 0] + d.beta * o.x;
+            o.y = d.alpha * acc[i][h * 4 + 1] + d.beta * o.y;
+            o.z = d.alpha * acc[i][h * 4 + 2] + d.beta * o.z;
+            o.w = d.alpha * acc[i][h * 4 + 3] + d.beta * o.w;
+            *reinterpret_cast<float4*>(d.C + r * d.ldc + c) = o;
         }
     }
 }
@@ -679,19 +684,33 @@ __global__ void k_transpose(const float* __restrict__ src, int64_t lds, int rows
     }
 }
 
-// dst = scale * src (rows x cols, leading dimensions) or, with src == null, the identity
+// dst = scale * src (rows x cols, leading dimensions)
 __global__ void k_copy2d(const float* __restrict__ src, int64_t lds, int rows, int cols, float* __restrict__ dst,
                          int64_t ldd, float scale) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= (int64_t)rows * cols) return;
     const int r = (int)(t / cols), c = (int)(t % cols);
-    dst[(int64_t)r * ldd + c] = src ? scale * src[(int64_t)r * lds + c] : (r == c ? 1.f : 0.f);
+    dst[(int64_t)r * ldd + c] = scale * src[(int64_t)r * lds + c];
 }
 
-// X0 = c1 H1 + c2 H2 + c3 H3 over n4 float4s (c3 = 0: H3 unused)
-__global__ void k_extrap(int64_t n4, const float4* __restrict__ h1, const float4* __restrict__ h2,
-                         const float4* __restrict__ h3, float c1, float c2, float c3, float4* __restrict__ x) {
+// the last blocks of a strip's inverse: S_NI = -T1 (nN x n), S_II = X (n x n)
+__global__ void k_store_ni_ii(int nN, int n, int mp, const float4* __restrict__ T1, const float4* __restrict__ X,
+                              float* __restrict__ S) {
+    const int n4 = n / 4;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int r = (int)(t / n4), c = (int)(t % n4);
+    if (r >= nN + n) return;
+    float4 v = r < nN ? T1[t] : X[t - (int64_t)nN * n4];
+    if (r < nN) v = make_float4(-v.x, -v.y, -v.z, -v.w);
+    *(reinterpret_cast<float4*>(S + (int64_t)r * mp + nN) + c) = v;
+}
+
+// X0 = c1 H1 + c2 H2 + c3 H3 over n4 float4s (c3 = 0: H3 unused); clears the norms
+__global__ void k_extrap(int64_t n4, const float4* __restrict__ h1, const float4* __restrict__ h2,
+                         const float4* __restrict__ h3, float c1, float c2, float c3, float4* __restrict__ x,
+                         unsigned* __restrict__ zero, int nzero) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t < nzero) zero[t] = 0u;
     if (t >= n4) return;
     const float4 a = h1[t];
     const float4 b = h2 ? h2[t] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -700,17 +719,22 @@ __global__ void k_extrap(int64_t n4, const float4* __restrict__ h1, const float4
                        c1 * a.w + c2 * b.w + c3 * c.w);
 }
 
-// *out = max over rows of sum |A[r, :]| (the infinity norm; non-negative floats order like their
-// bits, NaN above all): a warp per row
-__global__ void k_infnorm(const float* __restrict__ A, int64_t lda, int rows, int cols, unsigned* __restrict__ out) {
-    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (r >= rows) return;
-    const float* a = A + (int64_t)r * lda;
+// *out = max over columns of sum |At[:, c]|, the infinity norm of A from its transpose (n x n;
+// non-negative floats order like their bits, NaN above all): a block per 32 columns, a warp per eighth of
+// the rows
+__global__ void __launch_bounds__(256) k_infnorm_t(const float* __restrict__ At, int n, unsigned* __restrict__ out) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
     float sm = 0.f;
-    for (int c = lane; c < cols; c += 32) sm += fabsf(a[c]);
+#pragma unroll 16
+    for (int r = w; r < n; r += 8) sm += fabsf(At[(int64_t)r * n + c]);
+    part[w][lane] = sm;
+    __syncthreads();
+    if (w > 0) return;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, off);
-    if (lane == 0) atomicMax(out, sm == sm ? __float_as_uint(sm) : 0x7FFFFFFFu);
+    for (int v = 1; v < 8; v++) sm += part[v][lane];
+    const unsigned top = __reduce_max_sync(0xffffffffu, sm == sm ? __float_as_uint(sm) : 0x7FFFFFFFu);
+    if (lane == 0) atomicMax(out, top);
 }
 
 // ------------------------------------------------------------------ around the sweeps
@@ -752,7 +776,7 @@ void strip_free(Strip* p) {
     void* qs[] = {p->d_gptr, p->d_gidx, p->d_gcomp};
     for (void* q : qs) dfree(q);
     for (auto& c : p->chain) {
-        void* cs[] = {c.work.P, c.work.Ck, c.work.Rt, c.T, c.Xa, c.Xb, c.R, c.Rt, c.Xt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax};
+        void* cs[] = {c.work.P, c.work.Ck, c.work.Rt, c.T, c.cur, c.nxt, c.Rt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax};
         for (void* q : cs) dfree(q);
         if (c.h_rmax) cudaFreeHost(c.h_rmax);
         if (c.ev_read) cudaEventDestroy(c.ev_read);
@@ -789,24 +813,32 @@ int tend(Strip* p, cudaStream_t st, int tag) {
     return OCMP_OK;
 }
 
-int gemm(Strip* p, int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
-         float alpha, float beta, cudaStream_t st) {
-    if (M % GB || N % GB || K % 32 || M <= 0 || N <= 0 || K <= 0)
-        return fail(OCMP_ERR_ARG, "strip gemm: sizes must be multiples of the tile");
+int products(Strip* p, const DenseProduct* d, int count, cudaStream_t st) {
+    for (int q = 0; q < count; q++)
+        if (d[q].M % GB || d[q].N % GB || d[q].K % 32 || d[q].M <= 0 || d[q].N <= 0 || d[q].K <= 0)
+            return fail(OCMP_ERR_ARG, "strip gemm: sizes must be multiples of the tile");
     const bool t = p->timing;
     if (t && tbegin(p, st)) return OCMP_ERR_CUDA;
     if (p->gemm_kind == 1) {
-        const int r = tc_gemm_nt(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, p->d_flag + 1, st);
+        const int r = tc_products(d, count, p->d_flag + 1, st);
         if (r) return r;
-    } else {
-        const dim3 g(N / GB, M / GB);
-        OCMP_LAUNCH(sgemm_nt<<<g, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta));
-    }
+    } else
+        for (int q = 0; q < count; q++)
+            OCMP_LAUNCH(sgemm_nt<<<dim3(d[q].N / GB, d[q].M / GB), 256, 0, st>>>(d[q]));
     if (t && tend(p, st, 0)) return OCMP_ERR_CUDA;
-    p->gemm_flops_pending += 2.0 * M * N * (double)K;
-    // operands read once, C written (and read when beta != 0): the product's algorithmic bytes
-    p->gemm_bytes_pending += 4.0 * ((double)M * K + (double)N * K + (beta != 0.f ? 2.0 : 1.0) * M * (double)N);
+    for (int q = 0; q < count; q++) {
+        p->gemm_flops_pending += 2.0 * d[q].M * d[q].N * (double)d[q].K;
+        // operands read once, C written (and C0 read when beta != 0): the product's algorithmic bytes
+        p->gemm_bytes_pending += 4.0 * ((double)d[q].M * d[q].K + (double)d[q].N * d[q].K +
+                                        (d[q].beta != 0.f ? 2.0 : 1.0) * d[q].M * (double)d[q].N);
+    }
     return OCMP_OK;
+}
+// C = beta C + alpha A B^T
+int gemm(Strip* p, int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc,
+         float alpha, float beta, cudaStream_t st) {
+    const DenseProduct d{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, C, ldc};
+    return products(p, &d, 1, st);
 }
 
 // Gauss-Jordan over the pivot tiles [t_begin, t_end) of S (mp x mp) on stream st with workspace w
@@ -868,44 +900,43 @@ int phase1_groups(Strip* p, int k, float* S, int q, cudaStream_t ss) {
 constexpr float kSchulzTol = 1e-5f;
 constexpr int kSchulzMax = 8;
 
-// the residual of the current iterate and its norm, on the way to the host
+// The transpose of the current iterate's residual, R^T = I - X^T W^T, and its norm, on the way to the host.
+// Working with both X and X^T, and with R^T alone, every product has its operands in place: no
+// transposes and no copies on the chain.
 int schulz_residual(Strip* p, StripChain& c, const float* W, int mp, int n) {
     cudaStream_t cs = c.stream;
-    int r = transpose(c.cur, n, n, n, c.Xt, n, cs);
-    if (!r) r = copy2d(nullptr, 0, n, n, c.R, n, 1.f, cs);
-    if (!r) r = gemm(p, n, n, n, W, mp, c.Xt, n, c.R, n, -1.f, 1.f, cs);
+    const float* Xt = c.cur + (int64_t)n * n;
+    const DenseProduct d{n, n, n, Xt, n, W, mp, c.Rt, n, -1.f, 1.f, nullptr, 0};
+    const int r = products(p, &d, 1, cs);
     if (r) return r;
-    OCMP_CUDA(cudaMemsetAsync(c.rmax, 0, sizeof(unsigned), cs));
-    OCMP_LAUNCH(k_infnorm<<<nblk(n, 8), 256, 0, cs>>>(c.R, n, n, n, c.rmax));
-    OCMP_CUDA(cudaMemcpyAsync(c.h_rmax, c.rmax, sizeof(unsigned), cudaMemcpyDeviceToHost, cs));
+    unsigned* at = c.rmax + c.it;
+    OCMP_LAUNCH(k_infnorm_t<<<n / 32, 256, 0, cs>>>(c.Rt, n, at));
+    OCMP_CUDA(cudaMemcpyAsync(c.h_rmax, at, sizeof(unsigned), cudaMemcpyDeviceToHost, cs));
     OCMP_CUDA(cudaEventRecord(c.ev_read, cs));
     return OCMP_OK;
 }
 
 // start of an interface inversion: *pending when a residual is on its way
 int schulz_begin(Strip* p, StripChain& c, const float* W, int mp, int n, bool* pending) {
-    c.cur = c.Xa;
-    c.nxt = c.Xb;
     c.rprev = INFINITY;
     c.it = 0;
     *pending = false;
     int hist = 0;
     while (hist < 3 && c.h_n[hist] == n) hist++;
     if (!p->schulz || hist == 0) return OCMP_OK;
-    const int64_t n4 = (int64_t)n * n / 4;
+    const int64_t n4 = (int64_t)n * n / 2;   // with the transpose
     const float co[3][3] = {{1.f, 0.f, 0.f}, {2.f, -1.f, 0.f}, {3.f, -3.f, 1.f}};
     const float* cc = co[hist - 1];
     OCMP_LAUNCH(k_extrap<<<nblk(n4, 256), 256, 0, c.stream>>>(
         n4, reinterpret_cast<const float4*>(c.H[0]), hist > 1 ? reinterpret_cast<const float4*>(c.H[1]) : nullptr,
         hist > 2 ? reinterpret_cast<const float4*>(c.H[2]) : nullptr, cc[0], cc[1], cc[2],
-        reinterpret_cast<float4*>(c.cur)));
+        reinterpret_cast<float4*>(c.cur), c.rmax, kSchulzMax));
     *pending = true;
     return schulz_residual(p, c, W, mp, n);
 }
 
 // the residual is there: done (*pending false; *ok whether the iterate is taken) or one more step
 int schulz_step(Strip* p, StripChain& c, const float* W, int mp, int n, bool* pending, bool* ok) {
-    cudaStream_t cs = c.stream;
     OCMP_CUDA(cudaEventSynchronize(c.ev_read));
     float rho;
     std::memcpy(&rho, c.h_rmax, sizeof(float));
@@ -917,58 +948,67 @@ int schulz_step(Strip* p, StripChain& c, const float* W, int mp, int n, bool* pe
         return OCMP_OK;
     }
     c.rprev = rho;
-    int r = transpose(c.R, n, n, n, c.Rt, n, cs);
-    if (!r) r = copy2d(c.cur, n, n, n, c.nxt, n, 1.f, cs);
-    if (!r) r = gemm(p, n, n, n, c.cur, n, c.Rt, n, c.nxt, n, 1.f, 1.f, cs);
+    // X + X R and its transpose
+    const int64_t nn = (int64_t)n * n;
+    const DenseProduct d[2] = {{n, n, n, c.cur, n, c.Rt, n, c.nxt, n, 1.f, 1.f, c.cur, n},
+                               {n, n, n, c.Rt, n, c.cur, n, c.nxt + nn, n, 1.f, 1.f, c.cur + nn, n}};
+    const int r = products(p, d, 2, c.stream);
     if (r) return r;
     std::swap(c.cur, c.nxt);
     p->ns_iters++;
     if (rho * rho <= kSchulzTol) {
         *ok = true;
-        return transpose(c.cur, n, n, n, c.Xt, n, cs);
+        return OCMP_OK;
     }
     if (++c.it >= kSchulzMax) return OCMP_OK;
     *pending = true;
     return schulz_residual(p, c, W, mp, n);
 }
 
-// End of an interface inversion: the fallback, the history. The end strip's inverse (step 0 of the chain)
+// End of an interface inversion: the fallback. In the history (schulz_keep) the end strip's inverse (step 0 of the chain)
 // starts the second strip's iteration (spectral radius 0.9, eight steps at 96 x 96 DG P2), but it lacks a
 // Schur update and would spoil the extrapolation (2 X_1 - X_0 for the third: 0.87, against 0.05 for X_1).
-int schulz_end(Strip* p, StripChain& c, const float* W, int mp, int n, int step, bool started, bool ok) {
+int schulz_end(Strip* p, StripChain& c, const float* W, int mp, int n, bool started, bool ok) {
     cudaStream_t cs = c.stream;
     if (ok) p->ns_strips++;
     else if (started) p->ns_fallbacks++;
     if (!ok) {
         int r = copy2d(W, mp, n, n, c.cur, n, 1.f, cs);
         if (!r) r = gj_tiles(p, c.cur, n, 0, n, c.work, cs);
-        if (!r) r = transpose(c.cur, n, n, n, c.Xt, n, cs);
+        if (!r) r = transpose(c.cur, n, n, n, c.cur + (int64_t)n * n, n, cs);
         if (r) return r;
     }
-    // the new inverse joins the history, the oldest buffer taking it
+    return OCMP_OK;
+}
+
+// the new inverse joins the history, the oldest one's buffer becomes the next iterate's
+void schulz_keep(StripChain& c, int n, int step) {
     float* h = c.H[2];
     c.H[2] = c.H[1];
     c.H[1] = c.H[0];
-    c.H[0] = h;
+    c.H[0] = c.cur;
+    c.cur = h;
     c.h_n[2] = step == 1 ? 0 : c.h_n[1];
     c.h_n[1] = step == 1 ? 0 : c.h_n[0];
     c.h_n[0] = n;
-    OCMP_CUDA(cudaMemcpyAsync(h, c.cur, sizeof(float) * (size_t)n * n, cudaMemcpyDeviceToDevice, cs));
-    return OCMP_OK;
 }
 
 // Phase 2 of a block-diagonal-N strip after the Schur update: with X_I = W^-1 (W = S_II),
 //   G_II = X_I, G_IN = X_I Z, G_NI = -T, G_NN = X - T Z, T = Y X_I.
+// Z^T is in Zt: it is made while the host waits for the first residual.
 int phase2_assemble(Strip* p, StripChain& c, int k, float* S) {
     cudaStream_t cs = c.stream;
     const int mp = p->mp[k], nNp = p->nNp[k], n = mp - nNp;
-    int r = gemm(p, nNp, n, n, S + nNp, mp, c.Xt, n, c.T1, n, 1.f, 0.f, cs);
-    if (!r) r = transpose(S + (int64_t)nNp * mp, mp, n, nNp, c.Zt, n, cs);
+    const float* Xt = c.cur + (int64_t)n * n;
+    const DenseProduct d[2] = {
+        {nNp, n, n, S + nNp, mp, Xt, n, c.T1, n, 1.f, 0.f, nullptr, 0},
+        {n, nNp, n, c.cur, n, c.Zt, n, S + (int64_t)nNp * mp, mp, 1.f, 0.f, nullptr, 0}};
+    int r = products(p, d, 2, cs);
     if (!r) r = gemm(p, nNp, nNp, n, c.T1, n, c.Zt, n, S, mp, -1.f, 1.f, cs);
-    if (!r) r = gemm(p, n, nNp, n, c.cur, n, c.Zt, n, S + (int64_t)nNp * mp, mp, 1.f, 0.f, cs);
-    if (!r) r = copy2d(c.T1, n, nNp, n, S + nNp, mp, -1.f, cs);
-    if (!r) r = copy2d(c.cur, n, n, n, S + (int64_t)nNp * mp + nNp, mp, 1.f, cs);
-    return r;
+    if (r) return r;
+    OCMP_LAUNCH(k_store_ni_ii<<<nblk((int64_t)mp * (n / 4), 256), 256, 0, cs>>>(
+        nNp, n, mp, reinterpret_cast<const float4*>(c.T1), reinterpret_cast<const float4*>(c.cur), S));
+    return OCMP_OK;
 }
 
 // S_k[I, I] -= A[I, J] G_prev[J, J] A[J, I], the couplings given by the lists at offset lists
@@ -997,8 +1037,10 @@ int phase2(Strip* p, const int (&ks)[2], int step) {
     auto W = [&](int q) { return S(q) + (int64_t)p->nNp[ks[q]] * p->mp[ks[q]] + p->nNp[ks[q]]; };
     auto n = [&](int q) { return p->mp[ks[q]] - p->nNp[ks[q]]; };
     auto finish = [&](int q) {
-        const int r = schulz_end(p, p->chain[q], W(q), p->mp[ks[q]], n(q), step, started[q], ok[q]);
-        return r ? r : phase2_assemble(p, p->chain[q], ks[q], S(q));
+        int r = schulz_end(p, p->chain[q], W(q), p->mp[ks[q]], n(q), started[q], ok[q]);
+        if (!r) r = phase2_assemble(p, p->chain[q], ks[q], S(q));
+        schulz_keep(p->chain[q], n(q), step);
+        return r;
     };
     for (int q = 0; q < 2; q++) {
         const int k = ks[q];
@@ -1010,6 +1052,8 @@ int phase2(Strip* p, const int (&ks)[2], int step) {
         int r = fast[q] ? schulz_begin(p, c, W(q), p->mp[k], n(q), &pending[q])
                         : gj_tiles(p, S(q), p->mp[k], p->nNp[k], p->mp[k], c.work, c.stream);
         started[q] = pending[q];
+        const int nNp = p->nNp[k];
+        if (!r && fast[q]) r = transpose(S(q) + (int64_t)nNp * p->mp[k], p->mp[k], n(q), nNp, c.Zt, n(q), c.stream);
         if (!r && fast[q] && !pending[q]) r = finish(q);
         if (r) return r;
     }
@@ -1344,7 +1388,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
     for (int k = 0; k < K; k++)
         if (p->fast[k]) ns_max = std::max(ns_max, p->mp[k] - p->nNp[k]);
     const int chains = mid + 1 < K ? 2 : 1;
-    const int64_t fast_floats = p->nfast ? (int64_t)chains * (8 * (int64_t)ns_max * ns_max + 2 * (int64_t)p->mp_max * ns_max) +
+    const int64_t fast_floats = p->nfast ? (int64_t)chains * (11 * (int64_t)ns_max * ns_max + 2 * (int64_t)p->mp_max * ns_max) +
                                                 (int64_t)kSide * p->mp_max * ns_max
                                           : 0;
     const int64_t need = total * 4 + (int64_t)chains * p->nJp_max * p->nIp_max * 4 +
@@ -1526,15 +1570,13 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         U(&p->d_gcomp, gcomp);
         for (int q = 0; q < chains; q++) {
             StripChain& c = p->chain[q];
-            A(&c.Xa, i2);
-            A(&c.Xb, i2);
-            A(&c.R, i2);
+            A(&c.cur, 2 * i2);
+            A(&c.nxt, 2 * i2);
+            for (float*& h : c.H) A(&h, 2 * i2);
             A(&c.Rt, i2);
-            A(&c.Xt, i2);
-            for (float*& h : c.H) A(&h, i2);
             A(&c.T1, mi);
             A(&c.Zt, mi);
-            A(&c.rmax, 1);
+            A(&c.rmax, kSchulzMax);
             if (!st && cudaMallocHost((void**)&c.h_rmax, sizeof(unsigned)) != cudaSuccess)
                 st = fail(OCMP_ERR_NOMEM, "strip preconditioner: pinned flag");
         }
@@ -1551,8 +1593,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             const StripChain& c = p->chain[q];
             need_ptr.insert(need_ptr.end(), {c.T, c.work.P, c.work.Ck, c.work.Rt});
             if (p->nfast)
-                need_ptr.insert(need_ptr.end(), {c.Xa, c.Xb, c.R, c.Rt, c.Xt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax,
-                                                 c.h_rmax});
+                need_ptr.insert(need_ptr.end(), {c.cur, c.nxt, c.Rt, c.H[0], c.H[1], c.H[2], c.T1, c.Zt, c.rmax, c.h_rmax});
         }
         if (p->nfast)
             need_ptr.insert(need_ptr.end(), {p->d_gptr, p->d_gidx, p->d_gcomp, p->d_Yt[0], p->d_Yt[1], p->d_Yt[2]});
@@ -1631,7 +1672,7 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
         if (K - 1 - t > mid) order.push_back(K - 1 - t);
     }
     order.push_back(mid);
-    for (int o = 0; o < K; o++) {
+    auto phase1 = [&](int o) {
         const int k = order[o], q = o % kSide;
         cudaStream_t ss = p->side[q];
         const int mp = p->mp[k];
@@ -1643,10 +1684,15 @@ int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream
                                               : gj_tiles(p, S, mp, 0, p->nNp[k], p->work[q], ss);
         if (r) return r;
         OCMP_CUDA(cudaEventRecord(p->ev_phase1[k], ss));
-    }
+        return (int)OCMP_OK;
+    };
+    // a few pairs ahead of phase 2, which then does not wait for the host to have launched all of phase 1
+    int issued = 0;
     // phase 2: the two chains side by side, then the middle strip on the first
     for (int t = 0; t <= mid; t++) {
         const int ks[2] = {t, t < mid && K - 1 - t > mid ? K - 1 - t : -1};
+        for (; issued < K && issued < 2 * (t + kAhead); issued++)
+            if (const int r = phase1(issued)) return r;
         for (int q = 0; q < 2; q++) {
             const int k = ks[q];
             if (k < 0) continue;
@@ -1756,7 +1802,7 @@ extern "C" int ocmp_dense_gemm_nt(int32_t kind, int32_t M, int32_t N, int32_t K,
         if (M <= 0 || N <= 0 || K <= 0 || M % GB || N % GB || K % GK || (lda | ldb | ldc) & 3)
             return fail(OCMP_ERR_ARG, "ocmp_dense_gemm_nt: M, N must be multiples of 128, K of 16");
         const dim3 g(N / GB, M / GB);
-        OCMP_LAUNCH(sgemm_nt<<<g, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, alpha, beta));
+        OCMP_LAUNCH(sgemm_nt<<<g, 256, 0, st>>>(DenseProduct{M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, C, ldc}));
         OCMP_CUDA(cudaGetLastError());
         return OCMP_OK;
     }
