@@ -19,7 +19,7 @@
 // only rows and columns the Schur update A_k,k-1 S_{k-1}^-1 A_k-1,k touches), N = the rest, each
 // part padded to a multiple of 128 with decoupled unit rows. G_k is the block Gauss-Jordan inverse
 // of S_k with 128 x 128 diagonal-tile pivots (each tile inverted with partial pivoting inside it):
-// per tile one small inversion, two panel kernels and one rank-128 update of the whole strip, the
+// per tile one small inversion, one kernel for the panels and one rank-128 update of the whole strip, the
 // dominant flops. Since the Schur update only adds to the II block, the N pivots can be eliminated
 // before it:
 //   phase 1 (side streams, all strips independent): fill S_k, eliminate its N tiles;
@@ -58,7 +58,7 @@ constexpr int kSide = 3;   // side streams of phase 1
 constexpr int kAhead = 4;  // pairs of strips that the launches of phase 1 are ahead of phase 2
 
 struct StripWork {
-    float* P = nullptr;    // pivot-tile inverse, kNb x kNb
+    float* P = nullptr;    // pivot-tile inverse, kNb x kNb, and its transpose
     float* Ck = nullptr;   // column panel, mp_max x kNb
     float* Rt = nullptr;   // row panel (transposed), mp_max x kNb
 };
@@ -339,20 +339,21 @@ __global__ void __launch_bounds__(128) k_schur_u(int nI, int nIp, int nNp, int64
 }
 
 // ------------------------------------------------------------------ block Gauss-Jordan
-// P <- inverse of the tile S[t0:t0+128, t0:t0+128] by Gauss-Jordan with partial pivoting inside
-// the tile. The tile stays in registers, 8 x 8 per thread, and rows are never moved: step k takes as
-// pivot the largest |a_rk| over the rows not yet used, and the row and column permutation is applied
-// when the result is written (P[step(r)][piv(c)] = M[r][c]). Per step the half warp that holds column
-// k publishes it with the pivot, the half warps' owners of the pivot row publish that row (both
-// double-buffered in shared memory): two barriers per step. The rank-1 update reads 16 values per 64
-// products; one row of 16 entries per thread (1,024 threads) read one value per product and was bound
-// by issue: 286 us a tile. A zero or non-finite pivot is counted in *flag and replaced by a tiny
-// value.
+// P <- inverse of the tile S[t0:t0+128, t0:t0+128], followed by its transpose, by Gauss-Jordan with
+// partial pivoting inside the tile. The tile stays in registers, 8 x 8 per thread, a half warp per 8
+// columns (every 16th, so that the code of a column's steps is one short loop: unrolled over eight
+// neighbouring columns it was bound by fetching its instructions), and rows are never moved: step k takes as pivot the largest |a_rk| over the rows not yet used,
+// and the row and column permutation is applied when the result is written (P[step(r)][piv(c)] =
+// M[r][c]). A step is a chain of latencies on one SM: the half warp that holds column k publishes it
+// with the pivot (double-buffered in shared memory), one barrier, every half warp gets its part of the
+// pivot row from its own lane by shuffles, and the update starts with the next pivot column, which is
+// searched and published while the other warps update the rest. 286 us a tile with 16 x 1 entries per
+// thread (bound by issue), 108 with 8 x 8 and a second barrier for the pivot row, TILEUS so. A zero or
+// non-finite pivot is counted in *flag and replaced by a tiny value.
 constexpr int kTileThreads = 256;
 __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restrict__ S, int mp, int t0,
                                                            float* __restrict__ P, int* __restrict__ flag) {
     __shared__ __align__(16) float colk[2][kNb];
-    __shared__ __align__(16) float prow[2][kNb];
     __shared__ int pk[2];
     __shared__ float dk[2];
     __shared__ int piv[kNb];
@@ -363,72 +364,77 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(S + (int64_t)(t0 + tr * 8 + i) * mp + t0 + tc * 8 + j);
-            v[i][j] = x.x;
-            v[i][j + 1] = x.y;
-            v[i][j + 2] = x.z;
-            v[i][j + 3] = x.w;
-        }
+        for (int j = 0; j < 8; j++) v[i][j] = S[(int64_t)(t0 + tr * 8 + i) * mp + t0 + tc + 16 * j];
     unsigned used = 0;       // which of this thread's rows have been pivots
     // (a column of NaNs leaves rows without a step: those keep their own places)
     if (tid < kNb) piv[tid] = step[tid] = tid;
     __syncthreads();
-    // step k = 8 kb + kk; kk is a constant so that v stays in registers
-    auto eliminate = [&](int kb, auto col) {
-        constexpr int kk = decltype(col)::value, b = kk & 1;
-        const int k = kb * 8 + kk;
-        if (tc == kb) {
-            // 1 + the bits of |a|: 0 for a used row and for a NaN
-            unsigned key[8], best = 0u;
+    // pivot of column k = tc + 16 kk, by the half warp that holds it; kk is a constant so that v stays in
+    // registers
+    auto publish = [&](int k, auto col) {
+        constexpr int kk = decltype(col)::value;
+        const int b = k & 1;
+        // 1 + the bits of |a|: 0 for a used row and for a NaN
+        unsigned key[8], best = 0u;
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const float a = fabsf(v[i][kk]);
-                key[i] = (used >> i) & 1u || !(a == a) ? 0u : __float_as_uint(a) + 1u;
-                best = max(best, key[i]);
-            }
-            const unsigned top = __reduce_max_sync(group, best);
-            const int leader = __ffs(__ballot_sync(group, best == top)) - 1;
-            float pv = 0.f;
-            int p = k;   // every remaining |a_rk| is NaN
-            bool mine = lane == leader && top != 0u;
-#pragma unroll
-            for (int i = 7; i >= 0; i--)
-                if (key[i] == top) {
-                    pv = v[i][kk];
-                    if (top) p = tr * 8 + i;
-                }
-#pragma unroll
-            for (int i = 0; i < 8; i++) colk[b][tr * 8 + i] = v[i][kk];
-            if (lane == leader) {
-                if (!mine || !(fabsf(pv) > 0.f) || !isfinite(pv)) {
-                    atomicAdd(flag, 1);
-                    pv = 1e-30f;
-                }
-                // the pivot row becomes prow: 0 - (-1) prow below
-                if (mine) colk[b][p] = -1.f;
-                pk[b] = p;
-                dk[b] = 1.f / pv;
-                piv[k] = p;
-                step[p] = k;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i][kk] = 0.f;
-            // the pivot row's entry of column k is 1 before the scaling
-            if (mine)
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i][kk] = p == tr * 8 + i ? 1.f : v[i][kk];
+        for (int i = 0; i < 8; i++) {
+            const float a = fabsf(v[i][kk]);
+            key[i] = (used >> i) & 1u || !(a == a) ? 0u : __float_as_uint(a) + 1u;
+            best = max(best, key[i]);
         }
-        __syncthreads();
-        const int p = pk[b];
-        if (tr == p >> 3) {
+        const unsigned top = __reduce_max_sync(group, best);
+        const int leader = __ffs(__ballot_sync(group, best == top)) - 1;
+        const bool mine = lane == leader && top != 0u;
+        float pv = 0.f;
+        int p = k;   // every remaining |a_rk| is NaN
+#pragma unroll
+        for (int i = 7; i >= 0; i--)
+            if (key[i] == top) {
+                pv = v[i][kk];
+                if (top) p = tr * 8 + i;
+            }
+#pragma unroll
+        for (int i = 0; i < 8; i += 4)
+            *reinterpret_cast<float4*>(&colk[b][tr * 8 + i]) = make_float4(v[i][kk], v[i + 1][kk], v[i + 2][kk], v[i + 3][kk]);
+        if (lane == leader) {
+            if (!mine || !(fabsf(pv) > 0.f) || !isfinite(pv)) {
+                atomicAdd(flag, 1);
+                pv = 1e-30f;
+            }
+            // the pivot row's update is 0 - (-1) times the scaled pivot row
+            if (mine) colk[b][p] = -1.f;
+            pk[b] = p;
+            dk[b] = 1.f / pv;
+            piv[k] = p;
+            step[p] = k;
+        }
+        // column k becomes a column of the inverse: 1 in the pivot row before the scaling, 0 elsewhere
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i][kk] = mine && p == tr * 8 + i ? 1.f : 0.f;
+    };
+    // steps 16 kk .. 16 kk + 15
+    auto eliminate = [&](auto col) {
+        constexpr int kk = decltype(col)::value;
+        if (tc == 0) publish(16 * kk, col);
+#pragma unroll 1
+        for (int t = 0; t < 16; t++) {
+            const int b = t & 1;
+            __syncthreads();
+            const int p = pk[b];
             const float d = dk[b];
+            const bool owner = tr == p >> 3;
+            float cr[8], pr[8];
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) {
+                const float4 x = *reinterpret_cast<const float4*>(&colk[b][tr * 8 + i]);
+                cr[i] = x.x, cr[i + 1] = x.y, cr[i + 2] = x.z, cr[i + 3] = x.w;
+            }
             auto take = [&](auto row) {
                 constexpr int i = decltype(row)::value;
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    prow[b][tc * 8 + j] = v[i][j] * d;
-                    v[i][j] = 0.f;
+                    pr[j] = v[i][j];
+                    v[i][j] = owner ? 0.f : v[i][j];
                 }
             };
             switch (p & 7) {
@@ -441,103 +447,104 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
                 case 6: take(std::integral_constant<int, 6>{}); break;
                 default: take(std::integral_constant<int, 7>{});
             }
-            used |= 1u << (p & 7);
+            if (owner) used |= 1u << (p & 7);
+#pragma unroll
+            for (int j = 0; j < 8; j++) pr[j] = __shfl_sync(0xffffffffu, pr[j], p >> 3, 16) * d;
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i][kk] -= cr[i] * pr[kk];
+            if (tc == t + 1) publish(16 * kk + t + 1, col);
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j != kk) v[i][j] -= cr[i] * pr[j];
         }
-        __syncthreads();
-        float cr[8], pr[8];
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(&colk[b][tr * 8 + i]);
-            const float4 y = *reinterpret_cast<const float4*>(&prow[b][tc * 8 + i]);
-            cr[i] = x.x, cr[i + 1] = x.y, cr[i + 2] = x.z, cr[i + 3] = x.w;
-            pr[i] = y.x, pr[i + 1] = y.y, pr[i + 2] = y.z, pr[i + 3] = y.w;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[i][j] -= cr[i] * pr[j];
     };
-    for (int kb = 0; kb < kNb / 8; kb++) {
-        eliminate(kb, std::integral_constant<int, 0>{});
-        eliminate(kb, std::integral_constant<int, 1>{});
-        eliminate(kb, std::integral_constant<int, 2>{});
-        eliminate(kb, std::integral_constant<int, 3>{});
-        eliminate(kb, std::integral_constant<int, 4>{});
-        eliminate(kb, std::integral_constant<int, 5>{});
-        eliminate(kb, std::integral_constant<int, 6>{});
-        eliminate(kb, std::integral_constant<int, 7>{});
-    }
-    __syncthreads();
+    eliminate(std::integral_constant<int, 0>{});
+    eliminate(std::integral_constant<int, 1>{});
+    eliminate(std::integral_constant<int, 2>{});
+    eliminate(std::integral_constant<int, 3>{});
+    eliminate(std::integral_constant<int, 4>{});
+    eliminate(std::integral_constant<int, 5>{});
+    eliminate(std::integral_constant<int, 6>{});
+    eliminate(std::integral_constant<int, 7>{});
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int r = step[tr * 8 + i];
 #pragma unroll
-        for (int j = 0; j < 8; j++) P[r * kNb + piv[tc * 8 + j]] = v[i][j];
-    }
-}
-
-// For the 32 columns c0..c0+31: Rt[c, r] = sum_l P[r, l] S[t0 + l, c] (the pivot rows times P, stored
-// transposed), and for the 32 rows c0..c0+31: Ck[i, l] = S[i, t0 + l], zero on the pivot rows.
-constexpr int kPrepSmem = (kNb * kNb + kNb * 33) * (int)sizeof(float);
-__global__ void __launch_bounds__(256) k_panel_prep(const float* __restrict__ S, int mp, int t0,
-                                                    const float* __restrict__ P, float* __restrict__ Rt,
-                                                    float* __restrict__ Ck) {
-    extern __shared__ float sm[];
-    float* Ps = sm;                  // kNb x kNb
-    float* Sc = sm + kNb * kNb;      // kNb x 33: S[t0 + l, c0 + j]
-    const int tid = threadIdx.x, c0 = blockIdx.x * 32;
-    for (int e = tid; e < kNb * kNb; e += 256) Ps[e] = P[e];
-    for (int e = tid; e < kNb * 32; e += 256) {
-        const int l = e / 32, j = e % 32;
-        Sc[l * 33 + j] = S[(int64_t)(t0 + l) * mp + c0 + j];
-    }
-    for (int e = tid; e < 32 * kNb; e += 256) {
-        const int i = c0 + e / kNb, l = e % kNb;
-        Ck[(int64_t)i * kNb + l] = (i >= t0 && i < t0 + kNb) ? 0.f : S[(int64_t)i * mp + t0 + l];
-    }
-    __syncthreads();
-    const int j = tid & 31, rw = tid >> 5;   // column c0 + j, rows rw, rw + 8, ...
-    float acc[16];
-#pragma unroll
-    for (int q = 0; q < 16; q++) acc[q] = 0.f;
-    for (int l = 0; l < kNb; l++) {
-        const float sv = Sc[l * 33 + j];
-#pragma unroll
-        for (int q = 0; q < 16; q++) acc[q] = fmaf(Ps[(rw + 8 * q) * kNb + l], sv, acc[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) Rt[(int64_t)(c0 + j) * kNb + rw + 8 * q] = acc[q];
-}
-
-// After the rank-128 update: S[i, t0 + l] = -(Ck P)[i, l] for the non-pivot rows i of this block's 32
-// rows; S[t0 + r, c] = Rt[c, r] for this block's 32 columns c outside the tile, P inside it.
-constexpr int kFinishSmem = (kNb * kNb + 32 * (kNb + 1)) * (int)sizeof(float);
-__global__ void __launch_bounds__(256) k_panel_finish(float* __restrict__ S, int mp, int t0,
-                                                      const float* __restrict__ P, const float* __restrict__ Rt,
-                                                      const float* __restrict__ Ck) {
-    extern __shared__ float sm[];
-    float* Ps = sm;                  // kNb x kNb
-    float* Cs = sm + kNb * kNb;      // 32 x (kNb + 1)
-    const int tid = threadIdx.x, c0 = blockIdx.x * 32;
-    for (int e = tid; e < kNb * kNb; e += 256) Ps[e] = P[e];
-    for (int e = tid; e < 32 * kNb; e += 256)
-        Cs[(e / kNb) * (kNb + 1) + e % kNb] = Ck[(int64_t)(c0 + e / kNb) * kNb + e % kNb];
-    __syncthreads();
-    {
-        const int l = tid & (kNb - 1), r0 = tid >> 7;
-        for (int ii = r0; ii < 32; ii += 2) {
-            const int i = c0 + ii;
-            if (i >= t0 && i < t0 + kNb) continue;
-            float acc = 0.f;
-            for (int q = 0; q < kNb; q++) acc = fmaf(Cs[ii * (kNb + 1) + q], Ps[q * kNb + l], acc);
-            S[(int64_t)i * mp + t0 + l] = -acc;
+        for (int j = 0; j < 8; j++) {
+            const int c = piv[tc + 16 * j];
+            P[r * kNb + c] = v[i][j];
+            P[kNb * kNb + c * kNb + r] = v[i][j];
         }
     }
-    for (int e = tid; e < 32 * kNb; e += 256) {
-        const int jj = e / kNb, r = e % kNb;
-        const int c = c0 + jj;
-        const float v = (c >= t0 && c < t0 + kNb) ? Ps[r * kNb + (c - t0)] : Rt[(int64_t)c * kNb + r];
-        S[(int64_t)(t0 + r) * mp + c] = v;
+}
+
+// The panels of a pivot tile, 16 columns and 16 rows per block. Columns c: R = P S[T, c] goes into the
+// pivot rows S[T, c] and, transposed, into Rt. Rows i: Ck = S[i, T], S[i, T] = -Ck P. The rank-128 update
+// S -= Ck Rt^T that follows leaves the pivot rows and columns alone because Ck is zero on the former and
+// Rt on the latter; the tile itself becomes P. Both products have the form out[x][y] = sum_k M[k][y]
+// V[k][x] with M = P^T or P in shared memory: four warps each, 4 x 4 outputs per lane, so that a product
+// costs 1.25 shared-memory reads per 16 FMAs' issue slots. Two kernels (one of them after the update) with one or two
+// reads per FMA and strided stores took 36 us each at 1,280; this one PANELUS.
+constexpr int kPanel = 16;
+constexpr int kPanelSmem = (2 * kNb * kNb + 2 * kNb * kPanel) * (int)sizeof(float);
+__global__ void __launch_bounds__(256) k_panels(float* __restrict__ S, int mp, int t0, const float* __restrict__ P,
+                                                float* __restrict__ Rt, float* __restrict__ Ck) {
+    extern __shared__ __align__(16) float sm[];
+    float* Pt = sm;                        // [l][r]
+    float* Ps = sm + kNb * kNb;            // [q][l]
+    float* Sc = Ps + kNb * kNb;            // [l][16]: S[t0 + l, c0 + j]
+    float* Cs = Sc + kNb * kPanel;         // [q][16]: S[c0 + i, t0 + q]
+    const int tid = threadIdx.x, c0 = blockIdx.x * kPanel, lane = tid & 31, w = tid >> 5;
+    const bool pivot = c0 >= t0 && c0 < t0 + kNb;
+    for (int e = tid; e < kNb * kNb / 4; e += 256) {
+        reinterpret_cast<float4*>(Ps)[e] = reinterpret_cast<const float4*>(P)[e];
+        reinterpret_cast<float4*>(Pt)[e] = reinterpret_cast<const float4*>(P + kNb * kNb)[e];
+    }
+    for (int e = tid; e < kNb * kPanel / 4; e += 256) {
+        const int l = e / (kPanel / 4), q = e % (kPanel / 4);
+        reinterpret_cast<float4*>(Sc)[e] = *(reinterpret_cast<const float4*>(S + (int64_t)(t0 + l) * mp + c0) + q);
+    }
+    for (int e = tid; e < kNb * kPanel; e += 256) {
+        const int i = e / kNb, q = e % kNb;
+        const float x = pivot ? 0.f : S[(int64_t)(c0 + i) * mp + t0 + q];
+        Cs[q * kPanel + i] = x;
+        Ck[(int64_t)(c0 + i) * kNb + q] = x;
+    }
+    __syncthreads();
+    const float* M = w < 4 ? Pt : Ps;
+    const float* V = (w < 4 ? Sc : Cs) + 4 * (w & 3);
+    float acc[4][4] = {};   // [x][y]
+#pragma unroll 4
+    for (int k = 0; k < kNb; k++) {
+        const float4 m = *reinterpret_cast<const float4*>(M + k * kNb + 4 * lane);
+        const float4 x = *reinterpret_cast<const float4*>(V + k * kPanel);
+        const float xv[4] = {x.x, x.y, x.z, x.w}, mv[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++) acc[a][b] = fmaf(mv[b], xv[a], acc[a][b]);
+    }
+    const int x0 = c0 + 4 * (w & 3);
+    if (w >= 4) {
+        if (!pivot)
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+                *reinterpret_cast<float4*>(S + (int64_t)(x0 + a) * mp + t0 + 4 * lane) =
+                    make_float4(-acc[a][0], -acc[a][1], -acc[a][2], -acc[a][3]);
+        return;
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+        *reinterpret_cast<float4*>(Rt + (int64_t)(x0 + a) * kNb + 4 * lane) =
+            pivot ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        const int r = 4 * lane + b;
+        *reinterpret_cast<float4*>(S + (int64_t)(t0 + r) * mp + x0) =
+            pivot ? *reinterpret_cast<const float4*>(Ps + r * kNb + x0 - t0)
+                  : make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
     }
 }
 
@@ -848,12 +855,9 @@ int gj_tiles(Strip* p, float* S, int mp, int t_begin, int t_end, const StripWork
         OCMP_LAUNCH(k_tile_inv<<<1, kTileThreads, 0, st>>>(S, mp, t0, w.P, p->d_flag));
         if (!r) r = tend(p, st, 1);
         if (!r) r = tbegin(p, st);
-        OCMP_LAUNCH(k_panel_prep<<<mp / 32, 256, kPrepSmem, st>>>(S, mp, t0, w.P, w.Rt, w.Ck));
+        OCMP_LAUNCH(k_panels<<<mp / kPanel, 256, kPanelSmem, st>>>(S, mp, t0, w.P, w.Rt, w.Ck));
         if (!r) r = tend(p, st, 2);
         if (!r) r = gemm(p, mp, mp, kNb, w.Ck, kNb, w.Rt, kNb, S, mp, -1.f, 1.f, st);
-        if (!r) r = tbegin(p, st);
-        OCMP_LAUNCH(k_panel_finish<<<mp / 32, 256, kFinishSmem, st>>>(S, mp, t0, w.P, w.Rt, w.Ck));
-        if (!r) r = tend(p, st, 2);
         if (r) return r;
     }
     return OCMP_OK;
@@ -1392,7 +1396,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
                                                 (int64_t)kSide * p->mp_max * ns_max
                                           : 0;
     const int64_t need = total * 4 + (int64_t)chains * p->nJp_max * p->nIp_max * 4 +
-                         (int64_t)(kSide + chains) * (2 * p->mp_max * kNb + kNb * kNb) * 4 + fast_floats * 4;
+                         (int64_t)(kSide + chains) * (2 * (int64_t)p->mp_max * kNb + 2 * kNb * kNb) * 4 + fast_floats * 4;
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
     if ((size_t)need > fr) {
@@ -1419,7 +1423,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
     U(&p->d_ccol, ccol);
     p->bytes += (int64_t)(cptr.size() + 3 * cb.size()) * 4;
     auto work = [&](StripWork& w) {
-        A(&w.P, (size_t)kNb * kNb);
+        A(&w.P, 2 * (size_t)kNb * kNb);
         A(&w.Ck, (size_t)p->mp_max * kNb);
         A(&w.Rt, (size_t)p->mp_max * kNb);
     };
@@ -1623,8 +1627,7 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         if (cudaEventCreateWithFlags(&p->ev_phase1[k], cudaEventDisableTiming) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "cudaEventCreate");
     if (!st) {
-        if (cudaFuncSetAttribute(k_panel_prep, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(k_panel_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishSmem) != cudaSuccess ||
+        if (cudaFuncSetAttribute(k_panels, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_sweeps<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess ||
             cudaFuncSetAttribute(k_sweeps<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "strip preconditioner: shared-memory attribute");
