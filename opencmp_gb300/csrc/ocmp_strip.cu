@@ -340,88 +340,60 @@ __global__ void __launch_bounds__(128) k_schur_u(int nI, int nIp, int nNp, int64
 
 // ------------------------------------------------------------------ block Gauss-Jordan
 // P <- inverse of the tile S[t0:t0+128, t0:t0+128], followed by its transpose, by Gauss-Jordan with
-// partial pivoting inside the tile. The tile stays in registers, 8 x 8 per thread, a half warp per 8
-// columns (every 16th, so that the code of a column's steps is one short loop: unrolled over eight
-// neighbouring columns it was bound by fetching its instructions), and rows are never moved: step k takes as pivot the largest |a_rk| over the rows not yet used,
-// and the row and column permutation is applied when the result is written (P[step(r)][piv(c)] =
-// M[r][c]). A step is a chain of latencies on one SM: the half warp that holds column k publishes it
-// with the pivot (double-buffered in shared memory), one barrier, every half warp gets its part of the
-// pivot row from its own lane by shuffles, and the update starts with the next pivot column, which is
-// searched and published while the other warps update the rest. 286 us a tile with 16 x 1 entries per
-// thread (bound by issue), 108 with 8 x 8 and a second barrier for the pivot row, TILEUS so. A zero or
-// non-finite pivot is counted in *flag and replaced by a tiny value.
+// partial pivoting inside the tile. The tile stays in registers, 8 x 8 per thread, a half warp per every
+// 16th column, and rows are never moved: step k takes as pivot the largest |a_rk| (to 16 bits; the first
+// of equals) over the rows not yet used, and the row and column permutation is applied when the result is
+// written (P[step(r)][piv(c)] = M[r][c]). A step is a chain of latencies on one SM, so the chain is kept
+// short: the half warp that holds column k publishes it in shared memory and finds the pivot by one
+// integer reduction over keys that end in the row; one barrier; every half warp gets its part of the
+// pivot row from its own lane by shuffles, while the reciprocal is computed; the update starts with the
+// next pivot column, which is searched and published while the other warps update the rest. 286 us a tile
+// with 16 x 1 entries per thread (bound by issue), 108 with the pivot's value, reciprocal and row found
+// by the publishing half warp (800 of 1,600 clocks a step), 92 so. A zero or non-finite pivot is
+// counted in *flag and replaced by a tiny value.
 constexpr int kTileThreads = 256;
 __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restrict__ S, int mp, int t0,
                                                            float* __restrict__ P, int* __restrict__ flag) {
     __shared__ __align__(16) float colk[2][kNb];
     __shared__ int pk[2];
-    __shared__ float dk[2];
     __shared__ int piv[kNb];
     __shared__ int step[kNb];
-    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4, lane = tid & 31;
-    const unsigned group = 0xffffu << (lane & 16);
+    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
     float v[8][8];
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
         for (int j = 0; j < 8; j++) v[i][j] = S[(int64_t)(t0 + tr * 8 + i) * mp + t0 + tc + 16 * j];
-    unsigned used = 0;       // which of this thread's rows have been pivots
-    // (a column of NaNs leaves rows without a step: those keep their own places)
-    if (tid < kNb) piv[tid] = step[tid] = tid;
-    __syncthreads();
-    // pivot of column k = tc + 16 kk, by the half warp that holds it; kk is a constant so that v stays in
-    // registers
-    auto publish = [&](int k, auto col) {
+    unsigned open[8];       // all ones while this thread's row has not been a pivot
+#pragma unroll
+    for (int i = 0; i < 8; i++) open[i] = ~0u;
+    // column k = tc + 16 kk and its pivot, by the half warp that holds it (own; the whole warp comes
+    // along: a reduction over a part of a warp is slow); kk is a constant so that v stays in registers
+    auto publish = [&](int k, bool own, auto col) {
         constexpr int kk = decltype(col)::value;
         const int b = k & 1;
-        // 1 + the bits of |a|: 0 for a used row and for a NaN
-        unsigned key[8], best = 0u;
+        unsigned best = 0u;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float a = fabsf(v[i][kk]);
-            key[i] = (used >> i) & 1u || !(a == a) ? 0u : __float_as_uint(a) + 1u;
-            best = max(best, key[i]);
-        }
-        const unsigned top = __reduce_max_sync(group, best);
-        const int leader = __ffs(__ballot_sync(group, best == top)) - 1;
-        const bool mine = lane == leader && top != 0u;
-        float pv = 0.f;
-        int p = k;   // every remaining |a_rk| is NaN
+        for (int i = 0; i < 8; i++)
+            best = max(best, ((__float_as_uint(v[i][kk]) & 0x7fffff80u) | (0x80000000u + 127 - 8 * tr - i)) & open[i]);
+        if (own)
 #pragma unroll
-        for (int i = 7; i >= 0; i--)
-            if (key[i] == top) {
-                pv = v[i][kk];
-                if (top) p = tr * 8 + i;
-            }
-#pragma unroll
-        for (int i = 0; i < 8; i += 4)
-            *reinterpret_cast<float4*>(&colk[b][tr * 8 + i]) = make_float4(v[i][kk], v[i + 1][kk], v[i + 2][kk], v[i + 3][kk]);
-        if (lane == leader) {
-            if (!mine || !(fabsf(pv) > 0.f) || !isfinite(pv)) {
-                atomicAdd(flag, 1);
-                pv = 1e-30f;
-            }
-            // the pivot row's update is 0 - (-1) times the scaled pivot row
-            if (mine) colk[b][p] = -1.f;
-            pk[b] = p;
-            dk[b] = 1.f / pv;
-            piv[k] = p;
-            step[p] = k;
-        }
-        // column k becomes a column of the inverse: 1 in the pivot row before the scaling, 0 elsewhere
-#pragma unroll
-        for (int i = 0; i < 8; i++) v[i][kk] = mine && p == tr * 8 + i ? 1.f : 0.f;
+            for (int i = 0; i < 8; i += 4)
+                *reinterpret_cast<float4*>(&colk[b][tr * 8 + i]) =
+                    make_float4(v[i][kk], v[i + 1][kk], v[i + 2][kk], v[i + 3][kk]);
+        const unsigned top = __reduce_max_sync(0xffffffffu, own ? best : 0u);
+        if (own && tr == 0) pk[b] = 127 - (int)(top & 127u);
     };
     // steps 16 kk .. 16 kk + 15
     auto eliminate = [&](auto col) {
         constexpr int kk = decltype(col)::value;
-        if (tc == 0) publish(16 * kk, col);
+        if (tc < 2) publish(16 * kk, tc == 0, col);
 #pragma unroll 1
         for (int t = 0; t < 16; t++) {
             const int b = t & 1;
             __syncthreads();
             const int p = pk[b];
-            const float d = dk[b];
+            float pv = colk[b][p];
             const bool owner = tr == p >> 3;
             float cr[8], pr[8];
 #pragma unroll
@@ -429,6 +401,11 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
                 const float4 x = *reinterpret_cast<const float4*>(&colk[b][tr * 8 + i]);
                 cr[i] = x.x, cr[i + 1] = x.y, cr[i + 2] = x.z, cr[i + 3] = x.w;
             }
+            // column k becomes a column of the inverse: 1 in the pivot row before the scaling, 0 elsewhere
+            const bool here = tc == t;
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i][kk] = here ? 0.f : v[i][kk];
+            // the pivot row's update is 0 - (-1) times the scaled pivot row
             auto take = [&](auto row) {
                 constexpr int i = decltype(row)::value;
 #pragma unroll
@@ -436,23 +413,41 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
                     pr[j] = v[i][j];
                     v[i][j] = owner ? 0.f : v[i][j];
                 }
+                cr[i] = owner ? -1.f : cr[i];
+                open[i] = owner ? 0u : open[i];
             };
-            switch (p & 7) {
-                case 0: take(std::integral_constant<int, 0>{}); break;
-                case 1: take(std::integral_constant<int, 1>{}); break;
-                case 2: take(std::integral_constant<int, 2>{}); break;
-                case 3: take(std::integral_constant<int, 3>{}); break;
-                case 4: take(std::integral_constant<int, 4>{}); break;
-                case 5: take(std::integral_constant<int, 5>{}); break;
-                case 6: take(std::integral_constant<int, 6>{}); break;
-                default: take(std::integral_constant<int, 7>{});
+            if (p & 4) {
+                if (p & 2) {
+                    if (p & 1) take(std::integral_constant<int, 7>{});
+                    else take(std::integral_constant<int, 6>{});
+                } else {
+                    if (p & 1) take(std::integral_constant<int, 5>{});
+                    else take(std::integral_constant<int, 4>{});
+                }
+            } else {
+                if (p & 2) {
+                    if (p & 1) take(std::integral_constant<int, 3>{});
+                    else take(std::integral_constant<int, 2>{});
+                } else {
+                    if (p & 1) take(std::integral_constant<int, 1>{});
+                    else take(std::integral_constant<int, 0>{});
+                }
             }
-            if (owner) used |= 1u << (p & 7);
+            if (!(fabsf(pv) > 0.f) || !isfinite(pv)) {
+                if (tid == 0) atomicAdd(flag, 1);
+                pv = 1e-30f;
+            }
+            const float d = 1.f / pv;
+            if (tid == 0) {
+                piv[16 * kk + t] = p;
+                step[p] = 16 * kk + t;
+            }
 #pragma unroll
             for (int j = 0; j < 8; j++) pr[j] = __shfl_sync(0xffffffffu, pr[j], p >> 3, 16) * d;
+            pr[kk] = here ? d : pr[kk];
 #pragma unroll
             for (int i = 0; i < 8; i++) v[i][kk] -= cr[i] * pr[kk];
-            if (tc == t + 1) publish(16 * kk + t + 1, col);
+            if (tc >> 1 == (t + 1) >> 1) publish(16 * kk + t + 1, tc == t + 1, col);
 #pragma unroll
             for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -468,6 +463,7 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
     eliminate(std::integral_constant<int, 5>{});
     eliminate(std::integral_constant<int, 6>{});
     eliminate(std::integral_constant<int, 7>{});
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int r = step[tr * 8 + i];
@@ -486,7 +482,7 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_inv(const float* __restri
 // Rt on the latter; the tile itself becomes P. Both products have the form out[x][y] = sum_k M[k][y]
 // V[k][x] with M = P^T or P in shared memory: four warps each, 4 x 4 outputs per lane, so that a product
 // costs 1.25 shared-memory reads per 16 FMAs' issue slots. Two kernels (one of them after the update) with one or two
-// reads per FMA and strided stores took 36 us each at 1,280; this one PANELUS.
+// reads per FMA and strided stores took 36 us each at 1,280; this one 5.
 constexpr int kPanel = 16;
 constexpr int kPanelSmem = (2 * kNb * kNb + 2 * kNb * kPanel) * (int)sizeof(float);
 __global__ void __launch_bounds__(256) k_panels(float* __restrict__ S, int mp, int t0, const float* __restrict__ P,
