@@ -73,7 +73,8 @@ struct ocmp_solver_s {
     // GMRES
     double* small = nullptr;    // per system: R, rotations, scales (kept between the launches of phases)
     ocmp::GmResult* gout = nullptr;  // per system: what the host reads
-    ocmp::GmResult* hout = nullptr;  // pinned
+    ocmp::GmResult* hout = nullptr;  // pinned; behind the systems' results two slots for the phases' checks
+    cudaEvent_t ev_check[2] = {nullptr, nullptr};
     ocmp::GmTeams* teams = nullptr;  // the blocks' teams
     double* As64 = nullptr;     // A D^-1 (Jacobi folded) or A, FP64 Krylov matrix (owned)
     float* As32 = nullptr;      // same in FP32 (OCMP_MIXED)
@@ -495,7 +496,9 @@ int gm_full(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st) {
 }
 
 // A solve whose preconditioner runs in kernels of its own: a launch per phase, the host reading the
-// convergence flags every check_every iterations (launches queued past convergence return at once).
+// convergence flags every check_every iterations (launches queued past convergence return at once). The
+// flags of an iteration are looked at when the next one is queued, so that the GPU does not wait for the
+// host between them (10 us of 135 at 148,739 dofs); the one queued in vain returns at once.
 template <class T>
 int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, int* cycles) {
     const int m = sv->m, maxit = sv->prm.maxit;
@@ -529,6 +532,7 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
     const bool adaptive = sv->prm.check_every < 0;
     int next_check = std::max(1, sv->last_iters - 1);
     while (!H->flags[F_OUTER] && !H->flags[F_NONFIN] && it < maxit) {
+        int pending = -1;   // the slot of a check on its way
         for (int j = 0; j < m; j++) {
             if ((r = apply(V + (int64_t)j * a.one.ld, scale, j, flags))) return r;
             if (sv->time_spmv && it < kTimedProducts) {
@@ -537,14 +541,26 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
             } else
                 a.tlog = nullptr;
             if ((r = launch(GM_ITER, j))) return r;
-            it++;
+            if (++it >= maxit) break;
             // fixed interval, or (check_every < 0) the first check one iteration before the
             // previous solve's count and then after every iteration
             const bool check = adaptive ? it >= next_check : ((j + 1) % std::max(1, sv->prm.check_every)) == 0;
-            if (check || it >= maxit) {
-                if ((r = read())) return r;
-                if (H->flags[F_CONV] || it >= maxit) break;
+            const int before = pending;
+            pending = -1;
+            if (check) {
+                pending = it & 1;
                 next_check = it + 1;
+                OCMP_CUDA(cudaMemcpyAsync(&sv->hout[1 + pending], sv->gout, sizeof(GmResult), cudaMemcpyDeviceToHost, st));
+                OCMP_CUDA(cudaEventRecord(sv->ev_check[pending], st));
+            }
+            if (before >= 0) {
+                OCMP_CUDA(cudaEventSynchronize(sv->ev_check[before]));
+                const GmResult& R = sv->hout[1 + before];
+                if (R.bits & GM_ABORT) break;   // found again, and cleared, by the read below
+                if (R.flags[F_CONV]) {
+                    it--;
+                    break;
+                }
             }
         }
         a.tlog = nullptr;
@@ -588,6 +604,8 @@ static void free_solver(ocmp_solver_s* sv) {
         delete sv->cc;
     }
     if (sv->hout) cudaFreeHost(sv->hout);
+    for (cudaEvent_t e : sv->ev_check)
+        if (e) cudaEventDestroy(e);
     if (sv->hcg) cudaFreeHost(sv->hcg);
 }
 
@@ -645,6 +663,10 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
         }
     }
     if (blk) A(&sv->Binv, (size_t)s->mesh->ne * s->nloc * s->nloc);
+    if (prm->precond == OCMP_PRE_STRIP || prm->precond == OCMP_PRE_CAHOUET_CHABARD)
+        for (cudaEvent_t& e : sv->ev_check)
+            if (!st && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+                st = fail(OCMP_ERR_CUDA, "ocmp_solver_create: event");
     if (!st && prm->precond == OCMP_PRE_STRIP) st = strip_create(s, &sv->strip);
     if (mixed) {
         A(&sv->dinv32, (size_t)n * NB);
@@ -673,7 +695,7 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
                               (mixed ? sizeof(float) : sizeof(double)) * (size_t)(m + 1) * gm_ld(n) * NB) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "cudaMemset");
         if (!st && cudaMemset(sv->gout, 0, sizeof(GmResult) * NB) != cudaSuccess) st = fail(OCMP_ERR_CUDA, "cudaMemset");
-        if (!st && cudaMallocHost((void**)&sv->hout, sizeof(GmResult) * NB) != cudaSuccess)
+        if (!st && cudaMallocHost((void**)&sv->hout, sizeof(GmResult) * (NB + 2)) != cudaSuccess)
             st = fail(OCMP_ERR_NOMEM, "cudaMallocHost");
     }
     sv->borrow = gm && prm->precond == OCMP_PRE_JACOBI && mat->dinv &&
