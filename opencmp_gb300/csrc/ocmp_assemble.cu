@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "ocmp_internal.h"
@@ -1524,12 +1525,25 @@ int launch_scatter_values(const std::vector<int32_t>& idx, const std::vector<dou
     return OCMP_OK;
 }
 
+// f with the built (threads per row, unroll) pair as constants
+template <class F>
+static void with_rows(const RowCfg& rc, F f) {
+    using std::integral_constant;
+    if (rc.tpr == 2 && rc.u == 4) f(integral_constant<int, 2>{}, integral_constant<int, 4>{});
+    else if (rc.tpr == 2) f(integral_constant<int, 2>{}, integral_constant<int, 8>{});
+    else if (rc.tpr == 4 && rc.u == 4) f(integral_constant<int, 4>{}, integral_constant<int, 4>{});
+    else if (rc.tpr == 4) f(integral_constant<int, 4>{}, integral_constant<int, 8>{});
+    else if (rc.tpr == 8 && rc.u == 4) f(integral_constant<int, 8>{}, integral_constant<int, 4>{});
+    else if (rc.tpr == 8) f(integral_constant<int, 8>{}, integral_constant<int, 8>{});
+    else f(integral_constant<int, 16>{}, integral_constant<int, 8>{});
+}
+
 // Autotuner: times the FP64 SpMV for every built (threads per row, unroll) pair on this matrix with
 // CUDA events (warm-up launch, then `reps` timed launches each) and records the fastest in the
 // space; every kernel built on the row kernel then uses it.
 int autotune_spmv(ocmp_space_s* s, const double* vals, const double* x, double* y, cudaStream_t st, int reps,
                   int* best_tpr, int* best_u, float* best_ms) {
-    static const int cand[][2] = {{2, 4}, {4, 4}, {4, 8}, {8, 4}, {8, 8}, {16, 8}};
+    static const int cand[][2] = {{2, 4}, {2, 8}, {4, 4}, {4, 8}, {8, 4}, {8, 8}, {16, 8}};
     cudaEvent_t e0, e1;
     OCMP_CUDA(cudaEventCreate(&e0));
     OCMP_CUDA(cudaEventCreate(&e1));
@@ -1540,12 +1554,9 @@ int autotune_spmv(ocmp_space_s* s, const double* vals, const double* x, double* 
         const int tpr = c[0], u = c[1];
         const unsigned g = nblk(n * tpr, 256);
         auto launch = [&]() {
-            if (tpr == 2) OCMP_LAUNCH(spmv64_kernel<2, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-            else if (tpr == 4 && u == 4) OCMP_LAUNCH(spmv64_kernel<4, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-            else if (tpr == 4) OCMP_LAUNCH(spmv64_kernel<4, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-            else if (tpr == 8 && u == 4) OCMP_LAUNCH(spmv64_kernel<8, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-            else if (tpr == 8) OCMP_LAUNCH(spmv64_kernel<8, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-            else OCMP_LAUNCH(spmv64_kernel<16, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
+            with_rows({tpr, u}, [&](auto t, auto q) {
+                OCMP_LAUNCH(spmv64_kernel<decltype(t)::value, decltype(q)::value><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
+            });
         };
         launch();
         OCMP_CUDA(cudaEventRecord(e0, st));
@@ -1573,31 +1584,24 @@ int autotune_spmv(ocmp_space_s* s, const double* vals, const double* x, double* 
 }
 
 int launch_spmv64(const ocmp_space_s* s, const double* vals, const double* x, double* y, cudaStream_t st) {
-    const RowCfg rc = row_cfg(s);
+    const RowCfg rc = row_cfg64(s);
     const int64_t n = s->ndof;
-    const unsigned g = nblk(n * rc.tpr, 256);
-    if (rc.tpr == 2) OCMP_LAUNCH(spmv64_kernel<2, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-    else if (rc.tpr == 4 && rc.u == 4) OCMP_LAUNCH(spmv64_kernel<4, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-    else if (rc.tpr == 4) OCMP_LAUNCH(spmv64_kernel<4, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-    else if (rc.tpr == 8 && rc.u == 4) OCMP_LAUNCH(spmv64_kernel<8, 4><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-    else if (rc.tpr == 8) OCMP_LAUNCH(spmv64_kernel<8, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
-    else OCMP_LAUNCH(spmv64_kernel<16, 8><<<g, 256, 0, st>>>(n, s->d_rowptr, s->d_col, vals, x, y));
+    with_rows(rc, [&](auto t, auto q) {
+        OCMP_LAUNCH(spmv64_kernel<decltype(t)::value, decltype(q)::value><<<nblk(n * rc.tpr, 256), 256, 0, st>>>(
+            n, s->d_rowptr, s->d_col, vals, x, y));
+    });
     OCMP_CUDA(cudaGetLastError());
     return OCMP_OK;
 }
 
 int launch_spmv_axpby(const ocmp_space_s* s, const double* vals, double alpha, const double* x, double beta, double* y,
                       cudaStream_t st) {
-    const RowCfg rc = row_cfg(s);
+    const RowCfg rc = row_cfg64(s);
     const int64_t n = s->ndof;
-    const unsigned g = nblk(n * rc.tpr, 256);
-    const int32_t *rp = s->d_rowptr, *col = s->d_col;
-    if (rc.tpr == 2) OCMP_LAUNCH(spmv64_axpby_kernel<2, 4><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
-    else if (rc.tpr == 4 && rc.u == 4) OCMP_LAUNCH(spmv64_axpby_kernel<4, 4><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
-    else if (rc.tpr == 4) OCMP_LAUNCH(spmv64_axpby_kernel<4, 8><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
-    else if (rc.tpr == 8 && rc.u == 4) OCMP_LAUNCH(spmv64_axpby_kernel<8, 4><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
-    else if (rc.tpr == 8) OCMP_LAUNCH(spmv64_axpby_kernel<8, 8><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
-    else OCMP_LAUNCH(spmv64_axpby_kernel<16, 8><<<g, 256, 0, st>>>(n, rp, col, vals, alpha, x, beta, y));
+    with_rows(rc, [&](auto t, auto q) {
+        OCMP_LAUNCH(spmv64_axpby_kernel<decltype(t)::value, decltype(q)::value><<<nblk(n * rc.tpr, 256), 256, 0, st>>>(
+            n, s->d_rowptr, s->d_col, vals, alpha, x, beta, y));
+    });
     OCMP_CUDA(cudaGetLastError());
     return OCMP_OK;
 }
