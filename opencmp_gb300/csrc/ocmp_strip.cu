@@ -1454,7 +1454,10 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
             t.p0 = (int32_t)p->poff[k];
             t.mp = p->mp[k];
             t.gs = gs;
-            t.per = sweep_rows(t.mp, gs);
+            t.m = p->m[k];
+            t.nN = p->nN[k];
+            t.gap = p->nNp[k] - p->nN[k];
+            t.per = sweep_rows(t.m, gs);
             std::vector<int32_t> cols, list;
             for (int q = 0; q < t.mp; q++) {
                 const int32_t r = prow[t.p0 + q];
@@ -1513,28 +1516,27 @@ int strip_create(const ocmp_space_s* s, Strip** out) {
         SweepArgs& a = p->sweep;
         a.nsteps = (int)steps.size() / 2;
         a.nfwd = nfwd;
-        int most = 1, words = 0;   // floats of a step's rows in a block, words of its lists
+        int most = 1;   // floats of a step's rows and lists in a block
         for (const SweepStep& t : steps) {
             a.rows = std::max(a.rows, t.per);
             a.mp_max = std::max(a.mp_max, t.mp);
             a.nj_max = std::max(a.nj_max, t.nj);
-            most = std::max(most, t.per * t.mp);
-            words = std::max(words, t.words);
         }
-        // the lists are staged when they take no more than a third of the ring, in stages of a multiple
-        // of 128 bytes
+        // the lists are staged when they take no more than a third of the ring
         const size_t fixed = sweep_fixed_smem(a.mp_max, a.nj_max, a.rows);
         const int room = fixed < kSweepSmem ? (int)((kSweepSmem - fixed) / sizeof(float)) & ~31 : 0;
-        words = (words + 31) & ~31;
-        a.lists = words <= room / 3 ? words : 0;
-        a.stages = std::max(1, std::min({kSweepStages, room / (most + a.lists), a.nsteps}));
-        a.stage = std::min(most + a.lists, room);
+        for (SweepStep& t : steps) {
+            if (t.words > room / 3) t.words = 0;
+            most = std::max(most, t.words + t.per * t.mp);
+        }
+        a.stages = std::max(1, std::min({kSweepStages, room / most, a.nsteps}));
+        a.stage = std::min(most, room);
         p->sweep_smem = fixed + sizeof(float) * (size_t)a.stages * a.stage;
         if (!st && (blob.size() > (size_t)INT32_MAX || a.nj_max >= 0xffff || p->sweep_smem > kSweepSmem))
             st = fail(OCMP_ERR_UNSUPPORTED, "strip preconditioner: the couplings between the strips are too large");
         for (SweepStep& t : steps) {
             if (t.gs == 0) continue;
-            t.ns = std::min(t.per, (a.stage - a.lists) / t.mp);
+            t.ns = std::min(t.per, (a.stage - t.words) / t.mp);
             const int groups = (t.ns + 7) / 8 + (t.per - t.ns + 7) / 8;
             while (t.lwg < 4 && groups << (t.lwg + 1) <= kSweepWarps) t.lwg++;
         }

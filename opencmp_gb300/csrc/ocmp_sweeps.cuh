@@ -18,7 +18,8 @@
 //  - the few loads of a step that go to registers are issued one or two steps ahead.
 //
 // Measured (us per preconditioner application): 16,641 pressure dofs in 17 strips 226 -> 85 in one launch
-// -> 49 from both ends; before, two launches per strip and sweep, replayed from a graph. A step is
+// -> 49 from both ends; 110,592 in 96 strips 1,430 -> 690 -> 314 (one stage, a padded strip's rows) -> 290
+// (two, its real rows in one or two copies); before, two launches per strip and sweep, replayed from a graph. A step is
 // 5,000 clocks: 1,500 until the polled results are there, 1,500 for the product, the rest the gather,
 // the stores and the block's own barriers.
 #pragma once
@@ -42,10 +43,12 @@ constexpr long long kSweepWaitCycles = 8000000000LL;
 struct SweepStep {
     const float* G;
     int64_t blob;               // the lists, in words: values, jd, then 16-bit indices and positions
-    int32_t words, p0;          // their words (a multiple of 4); the strip's first position
+    int32_t words, p0;          // their words (a multiple of 32; 0: read in place); the strip's first position
     int32_t mp, cnt, len, nj;
     int32_t per, ns, lwg, gs;   // rows of a block, of which staged; log2 of the warps per group of 8 rows; blocks
+    int32_t m, nN, gap, pad;    // rows without the padding: row r is position r, from nN on r + gap
 };
+__device__ __forceinline__ int sweep_position(const SweepStep& s, int r) { return r < s.nN ? r : r + s.gap; }
 
 // `left` blocks are done with this launch; the last one counts the epoch on.
 struct SweepState {
@@ -66,7 +69,6 @@ struct SweepArgs {
     int* err;                 // a bit is set when a wait gave up
     int64_t n;
     int stages, stage;        // the ring: stages of so many floats
-    int lists;                // words of a stage in front of the rows, for the lists (0: they are read in place)
     int rows;                 // largest number of rows of a block
     int mp_max, nj_max;
 };
@@ -79,7 +81,7 @@ __host__ __device__ __forceinline__ SweepLists sweep_lists(int cnt, int len, int
     l.jd = cnt * len;
     l.idx = l.jd + nj;
     l.cq = l.idx + (cnt * len + 1) / 2;
-    l.words = (l.cq + (cnt + 1) / 2 + 3) & ~3;
+    l.words = (l.cq + (cnt + 1) / 2 + 31) & ~31;
     return l;
 }
 
@@ -88,12 +90,13 @@ inline size_t sweep_fixed_smem(int mp_max, int nj_max, int rows) {
 }
 
 // rows of a strip that a block of a group of gs takes
-inline int sweep_rows(int mp, int gs) { return (mp + gs - 1) / gs; }
+inline int sweep_rows(int m, int gs) { return (m + gs - 1) / gs; }
 
-// Rows against r, up to 8: a warp takes every wg-th group of 128 columns.
+// Rows against r, up to 8: a warp takes every wg-th group of 128 columns. In global memory the rows from
+// the split-th on lie gap rows further.
 template <bool SM>
-__device__ __forceinline__ void sweep_rows8(const float* g, int mp, int nrow, const float4* r, int part, int lwg,
-                                            int lane, float acc[8]) {
+__device__ __forceinline__ void sweep_rows8(const float* g, int mp, int nrow, int split, int gap, const float4* r,
+                                            int part, int lwg, int lane, float acc[8]) {
     const int nq = mp >> 2;
     for (int q = part * 32 + lane; q < nq; q += 32 << lwg) {
         const float4 b = r[q];
@@ -102,7 +105,8 @@ __device__ __forceinline__ void sweep_rows8(const float* g, int mp, int nrow, co
             float4 a[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                const float4* p = reinterpret_cast<const float4*>(g + (int64_t)(h + u) * mp) + q;
+                const int64_t at = SM || h + u < split ? h + u : h + u + gap;
+                const float4* p = reinterpret_cast<const float4*>(g + at * mp) + q;
                 a[u] = h + u >= nrow ? make_float4(0.f, 0.f, 0.f, 0.f) : SM ? *p : __ldcs(p);
             }
 #pragma unroll
@@ -165,19 +169,21 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     __syncthreads();
     auto at = [&](int t) -> const SweepStep& { return desc[t & (2 * kSweepAhead - 1)]; };
     auto rows_of = [&](const SweepStep& s, int* r0) {
-        *r0 = min(s.mp, (s.gs == size || block < half ? block : block - half) * s.per);
-        return min(s.per, s.mp - *r0);
+        *r0 = min(s.m, (s.gs == size || block < half ? block : block - half) * s.per);
+        return min(s.per, s.m - *r0);
     };
     // the copies of a step into its stage
     auto fetch = [&](int t, int i) {
         const SweepStep& s = at(t);
         int r0;
-        const int mp = s.mp, nr = min(rows_of(s, &r0), s.ns), words = a.lists ? s.words : 0;
-        const float* g = s.G + (int64_t)r0 * mp;
-        const uint32_t dst = saddr(ring + (int64_t)i * a.stage), row = dst + a.lists * 4;
+        const int mp = s.mp, nr = min(rows_of(s, &r0), s.ns), words = s.words;
+        const uint32_t dst = saddr(ring + (int64_t)i * a.stage), row = dst + words * 4;
         mbar_expect_tx(full + 8 * i, (uint32_t)(nr * mp + words) * 4);
         if (words) bulk_load(dst, a.blob + s.blob, words * 4, full + 8 * i);
-        for (int q = 0; q < nr; q++) bulk_load(row + q * mp * 4, g + (int64_t)q * mp, mp * 4, full + 8 * i);
+        // the rows are contiguous but for the padding between the two parts of the strip
+        const int n0 = max(0, min(nr, s.nN - r0)), n1 = nr - n0;
+        if (n0 > 0) bulk_load(row, s.G + (int64_t)r0 * mp, n0 * mp * 4, full + 8 * i);
+        if (n1 > 0) bulk_load(row + n0 * mp * 4, s.G + (int64_t)(r0 + n0 + s.gap) * mp, n1 * mp * 4, full + 8 * i);
     };
     constexpr int kFetcher = kSweepThreads - 1, kLoader = kSweepThreads - 64;
     if (tid == kFetcher)
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     auto load_row = [&](int t) {
         int r0;
         const int nr = rows_of(at(t), &r0);
-        return tid < nr ? __ldg(a.prow + at(t).p0 + r0 + tid) : -1;
+        return tid < nr ? __ldg(a.prow + at(t).p0 + sweep_position(at(t), r0 + tid)) : -1;
     };
 
     load_dofs(0);
@@ -252,7 +258,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         const int nr = rows_of(s, &r0);
         const float* stage = ring + i * a.stage;
         const SweepLists li = sweep_lists(cnt, len, nj);
-        const uint32_t* list = a.lists ? reinterpret_cast<const uint32_t*>(stage) : a.blob + s.blob;
+        const uint32_t* list = s.words ? reinterpret_cast<const uint32_t*>(stage) : a.blob + s.blob;
         // what nothing waits for before the end of this step: a descriptor, the next step's values,
         // this thread's own result of the forward sweep
         int32_t word = 0, was[kSweepValues];
@@ -298,11 +304,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
             const int row = gr < g1 ? 8 * gr : ns + 8 * (gr - g1), nrow = min(8, (gr < g1 ? ns : nr) - row);
             float acc[8] = {};
             if (gr < g1)
-                sweep_rows8<true>(stage + a.lists + row * mp, mp, nrow, reinterpret_cast<const float4*>(rs), pt, lwg, lane,
-                                  acc);
+                sweep_rows8<true>(stage + s.words + row * mp, mp, nrow, s.nN, 0, reinterpret_cast<const float4*>(rs), pt, lwg,
+                                  lane, acc);
             else
-                sweep_rows8<false>(s.G + (int64_t)(r0 + row) * mp, mp, nrow, reinterpret_cast<const float4*>(rs), pt, lwg,
-                                   lane, acc);
+                sweep_rows8<false>(s.G + (int64_t)(r0 + row) * mp, mp, nrow, s.nN - r0 - row, s.gap,
+                                   reinterpret_cast<const float4*>(rs), pt, lwg, lane, acc);
             // 8 sums over 32 lanes: halve the values three times, then two plain steps
 #pragma unroll
             for (int o = 16, h = 4; h > 0; o >>= 1, h >>= 1)
