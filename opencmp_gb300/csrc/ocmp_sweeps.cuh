@@ -19,8 +19,8 @@
 //
 // Measured (us per preconditioner application): 16,641 pressure dofs in 17 strips 226 -> 85 in one launch
 // -> 49 from both ends; 110,592 in 96 strips 1,430 -> 690 -> 314 (one stage, a padded strip's rows) -> 290
-// (two, its real rows in one or two copies); before, two launches per strip and sweep, replayed from a graph. A step is
-// 5,000 clocks: 1,500 until the polled results are there, 1,500 for the product, the rest the gather,
+// (two, its real rows in one or two copies) -> 279 (an entry's loads not waiting for another's); before, two
+// launches per strip and sweep, replayed from a graph. A step is 5,000 clocks: 1,500 until the polled results are there, 1,500 for the product, the rest the gather,
 // the stores and the block's own barriers.
 #pragma once
 
@@ -275,21 +275,27 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         }
         ok = __syncthreads_and(ok);
         if (!ok) break;
-        // r: minus (forward) or plus (backward) the couplings to the strip before
-        if (nr > 0) {
-            const float* val = reinterpret_cast<const float*>(list);
-            const uint16_t* idx = reinterpret_cast<const uint16_t*>(list + li.idx);
-            const uint16_t* cq = reinterpret_cast<const uint16_t*>(list + li.cq);
+        // r: minus (forward) or plus (backward) the couplings to the strip before; an entry's loads do not
+        // wait for another's
+        auto couple = [&](const uint32_t* l) {
+            const float* val = reinterpret_cast<const float*>(l);
+            const uint16_t* idx = reinterpret_cast<const uint16_t*>(l + li.idx);
+            const uint16_t* cq = reinterpret_cast<const uint16_t*>(l + li.cq);
             for (int c = tid; c < cnt; c += kSweepThreads) {
                 float acc = 0.f;
-#pragma unroll 4
+#pragma unroll 6
                 for (int e = 0; e < len; e++) {
                     const int k = idx[e * cnt + c];
-                    if (k != 0xffff) acc = fmaf(val[e * cnt + c], js[k], acc);
+                    const float v0 = val[e * cnt + c], g = js[k == 0xffff ? 0 : k];
+                    acc = k == 0xffff ? acc : fmaf(v0, g, acc);
                 }
                 float* r = rs + cq[c];
                 *r = mode == 0 ? *r - acc : acc;
             }
+        };
+        if (nr > 0) {
+            if (s.words) couple(reinterpret_cast<const uint32_t*>(stage));
+            else couple(a.blob + s.blob);
         }
         int32_t dof2 = -1;
         if (t + 2 < a.nsteps) {
