@@ -519,6 +519,14 @@ struct GmRun {
                                 x.w = fmaf(c, v[u].w, x.w);
                             }
                         }
+                        // the padding past n stays zero whatever the coefficients (a NaN there would outlive
+                        // the solve: nothing else writes it)
+                        if (r + 3 >= n) {
+                            if (r >= n) x.x = 0.f;
+                            if (r + 1 >= n) x.y = 0.f;
+                            if (r + 2 >= n) x.z = 0.f;
+                            x.w = 0.f;
+                        }
                         *reinterpret_cast<float4*>(W + r) = x;
                         ff_add(ah, al, x.x * x.x, 0.f);
                         ff_add(ah, al, x.y * x.y, 0.f);
