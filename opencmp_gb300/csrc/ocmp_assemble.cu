@@ -1257,7 +1257,7 @@ int ensure_contrib(ocmp_space_s* s, cudaStream_t st) {
     if (!s->d_csrc) OCMP_CUDA(cudaMalloc((void**)&s->d_csrc, sizeof(int32_t) * (size_t)ncon));
     const int ct = 128;
     const size_t csm = sizeof(int32_t) * (size_t)s->maxrow * ct;
-    OCMP_CUDA(cudaFuncSetAttribute(contrib_build_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+    if (const int r = smem_limit((const void*)contrib_build_kernel<L>, kMaxSmem)) return r;
     OCMP_LAUNCH(contrib_build_kernel<L><<<nblk(nd, ct), ct, csm, st>>>(nd, s->d_rowptr, s->d_inc_ptr, s->d_inc, s->d_slot,
                                                                   s->slot_stride, s->maxrow, s->d_cseg, s->d_csrc));
     const int32_t last = (int32_t)ncon;
@@ -1368,10 +1368,9 @@ int assemble_impl(ocmp_matrix_s* m, const ocmp_form_t* f, cudaStream_t st) {
     }
     // rows in ranges of similar length (vertex rows, then the rest) so short rows get small stripes
     const int rt = 128;
-    OCMP_CUDA(cudaFuncSetAttribute(row_scatter_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * (size_t)s->maxrow * (rt + 1))));
-    OCMP_CUDA(cudaFuncSetAttribute(row_scatter_ff_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double) * (size_t)s->maxrow * (rt + 1))));
+    int limit = smem_limit((const void*)row_scatter_kernel<L>, kMaxSmem);
+    if (!limit) limit = smem_limit((const void*)row_scatter_ff_kernel<L>, kMaxSmem);
+    if (limit) return limit;
     for (size_t q = 0; q + 1 < s->row_ranges.size(); q++) {
         const int64_t r0 = s->row_ranges[q], r1 = s->row_ranges[q + 1];
         if (r1 <= r0) continue;

@@ -678,6 +678,9 @@ static int launch_spmv_t(ocmp_space_s* s, const double* A, const double* x, doub
     return OCMP_OK;
 }
 
+// dynamic shared memory of the gradient kernel
+static size_t grad_smem(int F) { return sizeof(float) * (((layout(F).n + 3) & ~3) + kRowsPerBlock * kRecord); }
+
 // K dispatch (history length 1..6) for a kernel template taking <int K>
 #define OCMP_K_DISPATCH(k, ...)                           \
     switch (k) {                                          \
@@ -697,7 +700,8 @@ int ocmp_guess_create(int32_t n_features, uint64_t seed, ocmp_guess_t* out) {
     g->F = n_features;
     g->L = layout(n_features);
     const int n = g->L.n;
-    int st = dalloc(&g->P, n);
+    int st = smem_limit((const void*)mlp_grad_partial_kernel, grad_smem(kMaxF));
+    if (!st) st = dalloc(&g->P, n);
     if (!st) st = dalloc(&g->G, n);
     if (!st) st = dalloc(&g->M, n);
     if (!st) st = dalloc(&g->V, n);
@@ -772,8 +776,7 @@ static int grad_launch(ocmp_guess_t g, const float* X, const float* T, const flo
     if (st) return st;
     // two blocks fit on an SM; more blocks would only mean more partial vectors
     const int nb = (int)std::min<int64_t>((rows + kRowsPerBlock - 1) / kRowsPerBlock, kGradBlocks);
-    const size_t smem = sizeof(float) * (((g->L.n + 3) & ~3) + kRowsPerBlock * kRecord);
-    OCMP_CUDA(cudaFuncSetAttribute(mlp_grad_partial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = grad_smem(g->F);
     OCMP_LAUNCH(mlp_grad_partial_kernel<<<nb, kRowsPerBlock, smem, s>>>(rows, g->F, g->P, X, T, dY, g->Gpart, g->Lpart));
     OCMP_LAUNCH(mlp_grad_reduce_kernel<<<(g->L.n + 31) / 32, 256, 0, s>>>(nb, g->L.n, g->Gpart, g->G, g->Lpart, T ? nb : 0,
                                                                        g->loss));

@@ -52,6 +52,15 @@ int upload(T** p, const T* h, size_t n) {
 }
 void dfree(void* p);
 
+// Lets launches of kernel k take up to `bytes` of dynamic shared memory on the current device. The limit
+// belongs to the kernel, not to a launch: a kernel whose launches differ is always given the same
+// constant, since another host thread may launch it between this call and the caller's launch.
+constexpr size_t kMaxSmem = 227 * 1024;
+inline int smem_limit(const void* k, size_t bytes) {
+    OCMP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return OCMP_OK;
+}
+
 }  // namespace ocmp
 
 struct ocmp_mesh_s {

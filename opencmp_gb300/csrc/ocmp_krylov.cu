@@ -177,7 +177,6 @@ int team_blocks(int* out) {
 
 template <class T>
 int cg_launch(const void* k, CgArgs<T>& a, int grid, int threads, size_t smem, cudaStream_t st) {
-    if (smem) OCMP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* kp[] = {&a};
     OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(threads), kp, smem, st)));
     return OCMP_OK;
@@ -188,6 +187,11 @@ int cg_launch(const void* k, CgArgs<T>& a, int grid, int threads, size_t smem, c
 constexpr int64_t kCgOneBlockRows = 1024, kCgOneBlockNnz = 8192;
 constexpr int64_t kCgFuseNnz = 4900;   // entries per block whose second FMA costs the barrier's 2,450 clocks
 constexpr size_t kCgSmem = 200 * 1024;
+
+template <class T>
+int cg_smem_limit() {
+    return smem_limit((const void*)cg_res_kernel<T>, kCgSmem);
+}
 
 template <class T>
 int cg_solve(const CgArgs<T>& args, const ocmp_space_s* s, bool two_p, cudaStream_t st, CgState* out) {
@@ -427,6 +431,14 @@ GmArgs gm_args(const GmTeams* t, int m) {
 }
 
 constexpr size_t kGmSmem = 160 * 1024;   // the rest is left to L1, which the gathers live on
+constexpr int kGmMaxRestart = 128;
+static_assert(GmCfg<double>::smem(kGmMaxRestart) <= kGmSmem && GmCfg<float>::smem(kGmMaxRestart) <= kGmSmem,
+              "the largest restart's tables");
+
+template <class T>
+int gm_smem_limit() {
+    return smem_limit((const void*)gm_kernel<T>, kGmSmem);
+}
 
 template <class T>
 int gm_launch(GmArgs& a, const GmTeams* t, cudaStream_t st) {
@@ -435,7 +447,6 @@ int gm_launch(GmArgs& a, const GmTeams* t, cudaStream_t st) {
     const size_t base = GmCfg<T>::smem(a.m);
     a.rp_slices = a.mode == GM_FULL && base < kGmSmem ? (int)std::min<int64_t>(t->max_slices, (kGmSmem - base) / (33 * 4)) : 0;
     const size_t smem = base + (size_t)a.rp_slices * 33 * 4;
-    OCMP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* kp[] = {&a};
     OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(t->grid), dim3(GmCfg<T>::NT), kp, smem, st)));
     return OCMP_OK;
@@ -640,11 +651,12 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
         delete sv;
         return fail(OCMP_ERR_UNSUPPORTED, "ocmp_solver_create: batches are solved with GMRES + point Jacobi");
     }
-    sv->m = std::max(1, std::min(128, prm->restart > 0 ? prm->restart : 30));
+    sv->m = std::max(1, std::min(kGmMaxRestart, prm->restart > 0 ? prm->restart : 30));
     const int m = sv->m;
     const bool gm = prm->method == OCMP_GMRES, mixed = prm->precision == OCMP_MIXED;
     const bool blk = prm->precond == OCMP_PRE_BLOCK_JACOBI;
-    int st = OCMP_OK;
+    int st = gm ? (mixed ? gm_smem_limit<float>() : gm_smem_limit<double>())
+                : (mixed ? cg_smem_limit<float>() : cg_smem_limit<double>());
     auto A = [&](auto** p, size_t cnt) {
         if (!st) st = dalloc(p, cnt);
     };
@@ -1164,6 +1176,7 @@ extern "C" int ocmp_solve_cg_noalloc(ocmp_matrix_t mat, const double* b, double*
                                       std::to_string(kNoAllocMaxN) + "-dof limit of its static workspace");
     double* scr = nullptr;
     int st = noalloc_scratch(&scr);
+    if (!st) st = cg_smem_limit<double>();
     if (st) return st;
     // the second search direction fits beside the other five vectors in every system of the resident form
     cudaStream_t cst = (cudaStream_t)stream;
