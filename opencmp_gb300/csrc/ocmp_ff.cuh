@@ -32,6 +32,25 @@ __device__ __forceinline__ double f2d_exact(float f) {
     const unsigned long long d = sgn | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29);
     return __longlong_as_double((long long)d);
 }
+// the double of any float (f2d_exact without its flush of subnormals)
+__device__ __forceinline__ double f2d(float f) {
+    return (__float_as_uint(f) << 1) - 1u >= 0x00ffffffu ? f2d_exact(f) : (double)f;
+}
+// s += a b. The error of the FMA is recovered from the difference of the sums: exactly where that
+// difference is exact (the sum keeps its binade or so), else to the rounding of a b. So the sum loses no
+// more than if every product were rounded once, in half the operations of an exact product and a TwoSum.
+__device__ __forceinline__ void ff_mac(float& sh, float& sl, float a, float b) {
+    const float t = __fmaf_rn(a, b, sh);
+    sl = __fadd_rn(sl, __fmaf_rn(a, b, __fsub_rn(sh, t)));
+    sh = t;
+}
+// |lo| back below half a unit of hi
+__device__ __forceinline__ void ff_norm(float& sh, float& sl) {
+    const float s = __fadd_rn(sh, sl);
+    sl = __fsub_rn(sl, __fsub_rn(s, sh));
+    sh = s;
+}
+__device__ __forceinline__ double ff_wide(float h, float l) { return f2d(h) + f2d(l); }
 __device__ __forceinline__ double ff_to_double(float h, float l) { return f2d_exact(h) + f2d_exact(l); }
 __device__ __forceinline__ float2 ff_split(double x) {
     const float h = __double2float_rn(x);
