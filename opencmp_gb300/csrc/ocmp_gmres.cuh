@@ -364,25 +364,33 @@ struct GmRun {
     }
 
     // tab[k][wg] = V_k . w over the rows of warp wg of gw, for k in [k0, k0 + 8) or [k0, k0 + 4): float pairs
-    // through the lanes
+    // over the rows and through the lanes. One FP32 chain per lane, up to 111 products at 2.1 M rows, is three
+    // times less exact there than the 14 products and FP64 lanes of a reduction spread over the chip: error
+    // over |v||w| of random vectors 1.4e-10 against 5.8e-11 (and 1.0e-9 of both at 1,000 rows). The pairs' is
+    // 1.3e-11 (6.2e-10); they cost nothing at 2.1 M rows (178.7 -> 176.6 us an iteration) and up to 3% of it
+    // below 10^5 (21.7 -> 22.2 us at 79,507), 6% with element blocks, whose rows are read one at a time (49.3 ->
+    // 52.2 at 307,200).
     __device__ __forceinline__ void lanes_to_tab(float h, float l, int k, int nv, int wg) {
 #pragma unroll
         for (int off = 2; off > 0; off >>= 1) {
             const float oh = __shfl_xor_sync(0xffffffffu, h, off), ol = __shfl_xor_sync(0xffffffffu, l, off);
             ff_add(h, l, oh, ol);
         }
-        if ((lane & 3) == 0 && k < nv) tab[k * ES + wg] = ff_to_double(h, l);
+        if ((lane & 3) == 0 && k < nv) tab[k * ES + wg] = ff_wide(h, l);
     }
     __device__ __forceinline__ void dots8(const float* Vb, const float* W, int k0, int nv, int wg, int gw) {
         float h[8] = {0, 0, 0, 0, 0, 0, 0, 0}, l[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int s = wg; s < nsl; s += gw) {
+        for (int s = wg, c = 1; s < nsl; s += gw, c++) {
             const int64_t at = slice(s) + lane, r = min(at, n - 1);   // (a tile's rows may reach past n)
             const float wr = at < n ? W[r] : 0.f;
             float v[8];
 #pragma unroll
             for (int u = 0; u < 8; u++) v[u] = Vb[(int64_t)min(k0 + u, nv - 1) * ld + r];
 #pragma unroll
-            for (int u = 0; u < 8; u++) h[u] = fmaf(v[u], wr, h[u]);
+            for (int u = 0; u < 8; u++) ff_mac(h[u], l[u], v[u], wr);
+            if ((c & 7) == 0)
+#pragma unroll
+                for (int u = 0; u < 8; u++) ff_norm(h[u], l[u]);
         }
         gm_halve<4, 16>(h, l, lane);
         gm_halve<2, 8>(h, l, lane);
@@ -391,7 +399,7 @@ struct GmRun {
     }
     __device__ __forceinline__ void dots4(const float* Vb, const float* W, int k0, int nv, int wg, int gw) {
         float h[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0};
-        for (int s = 4 * wg; s < nsl; s += 4 * gw) {
+        for (int s = 4 * wg, c = 1; s < nsl; s += 4 * gw, c++) {
             const int64_t r = slice(s) + 4 * lane;
             const float4 wr = *reinterpret_cast<const float4*>(W + r);
             float4 v[4];
@@ -399,8 +407,15 @@ struct GmRun {
             for (int u = 0; u < 4; u++)
                 v[u] = *reinterpret_cast<const float4*>(Vb + (int64_t)min(k0 + u, nv - 1) * ld + r);
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                h[u] = fmaf(v[u].w, wr.w, fmaf(v[u].z, wr.z, fmaf(v[u].y, wr.y, fmaf(v[u].x, wr.x, h[u]))));
+            for (int u = 0; u < 4; u++) {
+                ff_mac(h[u], l[u], v[u].x, wr.x);
+                ff_mac(h[u], l[u], v[u].y, wr.y);
+                ff_mac(h[u], l[u], v[u].z, wr.z);
+                ff_mac(h[u], l[u], v[u].w, wr.w);
+            }
+            if ((c & 7) == 0)
+#pragma unroll
+                for (int u = 0; u < 4; u++) ff_norm(h[u], l[u]);
         }
         gm_halve<2, 16>(h, l, lane);
         gm_halve<1, 8>(h, l, lane);
@@ -528,10 +543,11 @@ struct GmRun {
                             x.w = 0.f;
                         }
                         *reinterpret_cast<float4*>(W + r) = x;
-                        ff_add(ah, al, x.x * x.x, 0.f);
-                        ff_add(ah, al, x.y * x.y, 0.f);
-                        ff_add(ah, al, x.z * x.z, 0.f);
-                        ff_add(ah, al, x.w * x.w, 0.f);
+                        ff_mac(ah, al, x.x, x.x);
+                        ff_mac(ah, al, x.y, x.y);
+                        ff_mac(ah, al, x.z, x.z);
+                        ff_mac(ah, al, x.w, x.w);
+                        ff_norm(ah, al);
                     });
                     done = true;
                 }
@@ -549,7 +565,10 @@ struct GmRun {
                 w0 += w1;
                 W[r] = w0;
                 if constexpr (D) ah += w0 * w0;
-                else ff_add(ah, al, w0 * w0, 0.f);
+                else {
+                    ff_mac(ah, al, w0, w0);
+                    ff_norm(ah, al);
+                }
             });
             if constexpr (D) acc[0] = ah;
             else fh = ah, fl = al;

@@ -8,8 +8,8 @@
 //
 // Precision: OCMP_FP64 runs everything in FP64. OCMP_MIXED runs an outer FP64 iterative
 // refinement (r = b - A x with the FP64 matrix, x += correction) around an inner GMRES/CG whose
-// matrix values, vectors and preconditioner are FP32; dot products are accumulated per thread in FP32
-// and across threads as float pairs or in FP64; the Hessenberg matrix and rotations stay FP64.
+// matrix values, vectors and preconditioner are FP32; dot products are sums of FP32 products in float
+// pairs or FP64; the Hessenberg matrix and rotations stay FP64.
 #include <cuda_runtime.h>
 
 #include <algorithm>

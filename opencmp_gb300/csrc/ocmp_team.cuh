@@ -231,7 +231,7 @@ __device__ __forceinline__ bool team_reduce_ff(Team& t, float h, float l, double
         const float oh = __shfl_xor_sync(0xffffffffu, h, o), ol = __shfl_xor_sync(0xffffffffu, l, o);
         ff_add(h, l, oh, ol);
     }
-    if (lane == 0) wv[w] = ff_to_double(h, l);
+    if (lane == 0) wv[w] = ff_wide(h, l);
     __syncthreads();
     double s = 0;
     if (w == 0) s = team_list_sum<1>(nw, lane, [&](int i) { return wv[i]; });

@@ -1,5 +1,6 @@
 """What the sums of the mixed-precision Krylov solves keep: systems whose FP32 products are all equal, so
-that a long FP32 chain of them rounds the same way at every addition."""
+that a long FP32 chain of them rounds the same way at every addition, and squares below FP32's normal
+range."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,45 @@ def test_cg_curvature_is_summed_beyond_fp32(gpu_lib):
     alpha = float((r.double() * z.double()).sum()) / pap
     got = float(x[inner].mean()) / (beta * float(c))
     assert abs(got / alpha - 1) <= 4 * U, (got / alpha - 1) / U
+
+
+def test_gmres_dots_are_summed_beyond_fp32(gpu_lib):
+    """A batch of 262,144-row systems, a block each, so 256 rows per thread: one iteration from zero,
+    x = D^-1 r (r.w) / (w.w) with w = A D^-1 r, at eighty scales of r = s D e. (e is 1/2 on a sixteenth of
+    the rows: were w parallel to r, a second orthogonalisation would repair the sums.) Rounded in FP32:
+    r (in w and in the dot product), D^-1, A D^-1, four additions of a row, w's scale twice, the products,
+    y and x's two: 16 U in all. Summed in FP32 per thread, r.w is up to 60 U off."""
+    import torch
+    from opencmp_gb300 import fem
+    B = 80
+    sp, A, A1, D = _mass(511, batch=B, jacobi32=True)
+    e = torch.ones_like(D)
+    e[:sp.ndof // 16] = 0.5
+    scales = 2.0 ** np.linspace(0, 1, B)
+    b = torch.cat([s * D * e for s in scales])
+    x = torch.zeros_like(b)
+    fem.KrylovSolver(A, method='GMRES', restart=1, precision='mixed', tol=1e-12, maxit=1).solve_batch(
+        b, x, raise_on_fail=False)
+    w = torch.empty_like(D)
+    A1.mult(e, w)                            # A D^-1 r = s A e
+    c = float((D * e * w).sum() / (w * w).sum())
+    err = [(float((x[q * sp.ndof:(q + 1) * sp.ndof] / (s * e)).mean()) / c - 1) / U for q, s in enumerate(scales)]
+    assert max(map(abs, err)) <= 16, (min(err), max(err))
+
+
+@pytest.mark.parametrize('scale', [1.0, 1e-31, 1e-33])
+@pytest.mark.parametrize('path', ['csr', 'sell'])
+def test_gmres_with_products_below_the_normal_range(gpu_lib, path, scale):
+    """The last cycles' residuals are 1e-9 of the right-hand side's: their products with the basis are
+    subnormal in FP32 but still add up."""
+    import torch
+    from opencmp_gb300 import fem
+    m = M.unit_square(22)
+    sp = fem.Space(m, 'H1', 1, m.bc_names)
+    A = fem.Matrix(sp, jacobi32=True, dfloat=path == 'sell', sell=path == 'sell')
+    A.assemble(fem.make_form(mass=1.0, diff=0.05, wind=(1.0, 0.5)))
+    g = torch.Generator(device='cuda').manual_seed(3)
+    b = scale * torch.randn(sp.ndof, dtype=torch.float64, device='cuda', generator=g)
+    sv = fem.KrylovSolver(A, method='GMRES', restart=30, precision='mixed', tol=1e-9, maxit=2000)
+    info = sv.solve(b, torch.zeros_like(b), raise_on_fail=False)
+    assert info.status == 0 and info.iterations <= 200, (info.status, info.iterations, info.relres)
