@@ -30,6 +30,11 @@ constexpr int kCgRowsRes = kCgRowsPerThread * kCgThreadsRes;
 constexpr int kCgSlicesRes = kCgRowsRes / 32;
 
 enum { CG_NONFIN = 1, CG_BREAK = 2 };
+// FP32: p . A p of up to so many times sum |p_i| |a_ij| |p_j| may be rounding alone (an entry's and a
+// product's). More negative curvature than that is the matrix's own and stepped along. From 1 to 64 times
+// 2^-24 the solves of the nearly singular Neumann pressure operator stop where they should; at 4 and above
+// P1 triangles on 200 x 200 with one negative eigenvalue (-div grad - 30) diverge, at 64 those on 100 x 100.
+constexpr double kCgUnresolved = 2.0 / 16777216;
 // What the host reads after a solve.
 struct CgResult {
     double res0, res;
@@ -278,9 +283,21 @@ __global__ void __launch_bounds__(kCgThreadsRes, 1) cg_res_kernel(CgArgs<T> a) {
                 else if (!MIX) o.brk = true;
                 break;
             }
-            // a step against the descent direction: the FP32 matrix is not definite (a mode the rounded
-            // values do not resolve). What was reached is kept, and refined from its true residual.
-            if (MIX && pap * rz <= 0) break;
+            // a step against the descent direction that rounding explains: a mode that the FP32 values do
+            // not resolve. What was reached is kept, and refined from its true residual.
+            if (MIX && pap * rz <= 0) {
+                const T* p = a.fuse ? pn : pc;   // everyone's is there since the last exchange
+                part[0] = 0;
+#pragma unroll 1
+                for (int k = 0; k < RPT; k++) {
+                    T s = 0;
+                    const int base = w + k * nw < own ? soff[w + k * nw] + lane : 0;
+                    for (int j = 0; j < len[k]; j++) s += fabs(sval[base + j * 32] * p[scol[base + j * 32]]);
+                    if (fr[k]) part[0] += cg_wide(fabs(pv[k]) * s);
+                }
+                if (!team_reduce<1>(tm, part, sum, live)) return;
+                if (!(fabs(pap) > kCgUnresolved * sum[0])) break;
+            }
             if (tid == 0) s_scal = rz / pap;
             __syncthreads();
             // x += alpha p, r -= alpha q, z, r . z, |r|^2
@@ -413,9 +430,19 @@ __global__ void __launch_bounds__(kCgThreadsStream, 1) cg_stream_kernel(CgArgs<T
                 else if (!MIX) o.brk = true;
                 break;
             }
-            // a step against the descent direction: the FP32 matrix is not definite (a mode the rounded
-            // values do not resolve). What was reached is kept, and refined from its true residual.
-            if (MIX && pap * rz <= 0) break;
+            // a step against the descent direction that rounding explains: a mode that the FP32 values do
+            // not resolve. What was reached is kept, and refined from its true residual.
+            if (MIX && pap * rz <= 0) {
+                CgSum<T> s;
+                each([&](int64_t r) {
+                    T v = 0;
+                    for (int32_t k = a.rp[r]; k < a.rp[r + 1]; k++) v += fabs(a.K[k] * a.p0[a.col[k]]);
+                    if (a.freed[r]) s.add(fabs(a.p0[r]), v);
+                });
+                part[0] = s.value();
+                if (!team_reduce<1>(tm, part, sum, live)) return;
+                if (!(fabs(pap) > kCgUnresolved * sum[0])) break;
+            }
             if (tid == 0) s_scal = rz / pap;
             __syncthreads();
             // x += alpha p, r -= alpha q, z, r . z, |r|^2

@@ -98,3 +98,32 @@ def test_gmres_with_products_below_the_normal_range(gpu_lib, path, scale):
     sv = fem.KrylovSolver(A, method='GMRES', restart=30, precision='mixed', tol=1e-9, maxit=2000)
     info = sv.solve(b, torch.zeros_like(b), raise_on_fail=False)
     assert info.status == 0 and info.iterations <= 200, (info.status, info.iterations, info.relres)
+
+
+@pytest.mark.parametrize('dim,n,order', [(2, 6, 1), (2, 24, 1), (2, 40, 2), (2, 100, 1), (3, 24, 1), (3, 56, 1)])
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+def test_cg_on_an_indefinite_matrix(gpu_lib, dim, n, order, precision):
+    """-div grad - 30 (2D: one negative eigenvalue at 2 pi^2 - 30) or - 40 (3D: at 3 pi^2 - 40): CG goes on
+    through steps of negative curvature. One block, all blocks' rows in shared memory, and streaming."""
+    import torch
+    from opencmp_gb300 import fem
+    m = M.unit_square(n) if dim == 2 else M.unit_cube(n)
+    sp = fem.Space(m, 'H1', order, m.bc_names)
+    A = fem.Matrix(sp, fp32=precision == 'mixed')
+    A.assemble(fem.make_form(mass=-30.0 if dim == 2 else -40.0, diff=1.0))
+    b = torch.zeros(sp.ndof, dtype=torch.float64, device='cuda')
+    fem.assemble_rhs(sp, fem.make_form(diff=1.0), fem.make_rhs(src_const=1.0), b)
+    info = fem.KrylovSolver(A, method='CG', precision=precision, tol=1e-9, maxit=2000).solve(b, torch.zeros_like(b),
+                                                                                            raise_on_fail=False)
+    assert info.status == 0 and info.relres <= 1e-9, (info.status, info.iterations, info.relres)
+
+
+@pytest.mark.parametrize('n,most', [(16, 150), (24, 170), (32, 160)])
+def test_pressure_solves_keep_what_they_reached(gpu_lib, n, most):
+    """The Neumann pressure operator's constant mode is below FP32's rounding. An inner solve that steps along
+    it as if it were negative curvature diverges, and the outer iteration pays: 450, 360 and 169 iterations
+    when it did, 149, 164 and 156 when it stops there (and FP64: 149, 159, 156)."""
+    import test_saddle as S
+    th, A, b, u, sv = S._gpu_cavity(n, 'mixed', impl='host')
+    info = sv.solve(b, u.clone(), raise_on_fail=False)
+    assert info.status == 0 and info.iterations <= most, (info.status, info.iterations)
