@@ -99,8 +99,17 @@ struct GmTeams {
     GmInst* inst = nullptr;      // device descriptors (several systems)
 };
 
-// stride of the basis vectors: tiles of 128 rows with 16-byte loads
-__host__ __device__ constexpr int64_t gm_ld(int64_t n) { return (n + 127) / 128 * 128; }
+// FP32 systems of this many rows a block have tiles of 128 rows (16-byte loads of the basis).
+constexpr int64_t kGmVecRows = 512;
+
+// Stride of the basis vectors: whole tiles of 128 rows where they are read in 16-byte loads; elsewhere 16
+// values (64 or 128 bytes), since the vectors of a batch of tiny systems would be mostly padding (9 rows,
+// restart 30, FP64: 36 KB a system, and 9 KB so; a stride of n without alignment before took 11).
+template <class T>
+__host__ __device__ constexpr int64_t gm_ld(int64_t n) {
+    const int64_t pad = sizeof(T) == 4 && n >= kGmVecRows ? 128 : 16;
+    return (n + pad - 1) / pad * pad;
+}
 
 __host__ __device__ constexpr int gm_small_doubles(int m) { return m * (m + 1) / 2 + 4 * m + 8; }
 

@@ -302,7 +302,7 @@ GmInst gm_inst(const ocmp_solver_s* sv, int q, const double* b, double* x, int t
     const bool diag = pre == OCMP_PRE_JACOBI || pre == OCMP_PRE_USER;
     GmInst d{};
     d.n = n;
-    d.ld = gm_ld(n);
+    d.ld = gm_ld<T>(n);
     d.rp = s->d_rowptr;
     d.col = s->d_col;
     d.freed = s->d_free;
@@ -350,9 +350,6 @@ void gm_teams_free(GmTeams* t) {
     for (void* p : ps) dfree(p);
     delete t;
 }
-
-// FP32 systems of this many rows a block have tiles of 128 rows (16-byte loads of the basis).
-constexpr int64_t kGmVecRows = 512;
 
 int gm_teams_create(const std::vector<GmInst>& inst, const std::vector<int64_t>& nnz, int m, bool fp64, GmTeams** out) {
     int sms = 1;
@@ -668,7 +665,7 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
         A(&sv->r, n);
     }
     if (!mixed) {
-        if (gm) A(&sv->V, (size_t)(m + 1) * gm_ld(n) * NB);
+        if (gm) A(&sv->V, (size_t)(m + 1) * gm_ld<double>(n) * NB);
         else {
             A(&sv->p, n);
             A(&sv->pb, n);
@@ -683,7 +680,7 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
     if (mixed) {
         A(&sv->dinv32, (size_t)n * NB);
         A(&sv->z32, n);
-        if (gm) A(&sv->V32, (size_t)(m + 1) * gm_ld(n) * NB);
+        if (gm) A(&sv->V32, (size_t)(m + 1) * gm_ld<float>(n) * NB);
         else {
             A(&sv->w32, n);
             A(&sv->d32, n);
@@ -704,7 +701,8 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
         A(&sv->gout, (size_t)NB);
         // the basis is read past n (its stride is padded)
         if (!st && cudaMemset(mixed ? (void*)sv->V32 : (void*)sv->V, 0,
-                              (mixed ? sizeof(float) : sizeof(double)) * (size_t)(m + 1) * gm_ld(n) * NB) != cudaSuccess)
+                              (mixed ? sizeof(float) * gm_ld<float>(n) : sizeof(double) * gm_ld<double>(n)) *
+                                  (size_t)(m + 1) * NB) != cudaSuccess)
             st = fail(OCMP_ERR_CUDA, "cudaMemset");
         if (!st && cudaMemset(sv->gout, 0, sizeof(GmResult) * NB) != cudaSuccess) st = fail(OCMP_ERR_CUDA, "cudaMemset");
         if (!st && cudaMallocHost((void**)&sv->hout, sizeof(GmResult) * (NB + 2)) != cudaSuccess)

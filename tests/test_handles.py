@@ -1,4 +1,5 @@
-"""Krylov handles and their neighbours used from several host threads, a handle each."""
+"""Krylov handles and their neighbours used from several host threads, a handle each; what a handle of many
+tiny systems holds."""
 import ctypes as C
 import threading
 
@@ -117,3 +118,24 @@ def test_threads_with_a_matrix_each(gpu_lib):
         jobs.append((LB.load().ocmp_assemble_matrix, (A.h, C.byref(form)), 2, [A.device_values()[0]]))
     torch.cuda.synchronize()
     _side_by_side(jobs)
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+def test_memory_of_a_batch_of_tiny_systems(gpu_lib, precision):
+    """The bases of 9-dof systems take (restart + 1) vectors of at most 16 values each."""
+    import torch
+    from opencmp_gb300 import fem
+    m = M.unit_square(2)
+    sp = fem.Space(m, 'H1', 1, m.bc_names)
+    B, restart = 20000, 30
+    A = fem.Matrix(sp, batch=B, jacobi64=precision == 'fp64', jacobi32=precision == 'mixed')
+    small = 8 * (restart * (restart + 1) // 2 + 4 * restart + 8) * B        # Hessenberg matrices, rotations
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    sv = fem.KrylovSolver(A, method='GMRES', restart=restart, precision=precision, tol=1e-8, maxit=10)
+    torch.cuda.synchronize()
+    used = free0 - torch.cuda.mem_get_info()[0]
+    basis = (8 if precision == 'fp64' else 4) * (restart + 1) * 16 * B
+    # beside these a few vectors and results per system, and the allocator's granularity
+    assert used <= small + basis + 1000 * B + (64 << 20), (used, small, basis)
+    assert sv.h
