@@ -36,15 +36,16 @@ constexpr double kReorth = 1e-6;
 
 // device flags of a solve in phases (its preconditioner's kernels return at once when F_CONV is set)
 enum { F_CONV = 0, F_BREAK, F_NONFIN, F_JDONE, F_ITERS, F_OUTER, F_NFLAG = 8 };
-enum { GM_NONFIN = 1, GM_BREAK = 2, GM_ABORT = 4 };
+enum { GM_NONFIN = 1, GM_BREAK = 2 };
 // phases: GM_FULL a whole solve; for the preconditioners applied by other kernels: GM_FIRST / GM_START
 // the residual and the start of a cycle, GM_ITER iteration j, GM_COMBINE z = sum_k y_k v_k
 enum { GM_FULL = 0, GM_FIRST, GM_START, GM_ITER, GM_COMBINE };
 
-// What the host reads after a solve (flags: the phases' device flags).
+// What the host reads after a solve (flags: the phases' device flags). gaveup is set by any block whose wait
+// ran out and cleared by the host alone, so that no result of a block that had passed hides it.
 struct GmResult {
     double res0, res;
-    int iters, cycles, bits, pad;
+    int iters, cycles, bits, gaveup;
     int flags[F_NFLAG];
 };
 
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(GmCfg<T>::NT, 1) gm_kernel(const __grid_consta
         run.s_end = &s_end;
         run.s_bits = &s_bits;
         if (!(a.mode == GM_FULL ? run.solve() : run.phase())) {
-            if (threadIdx.x == 0) atomicOr(&run.d.out->bits, GM_ABORT);
+            if (threadIdx.x == 0) atomicExch(&run.d.out->gaveup, 1);
             return;
         }
         team_leave(tm);

@@ -204,12 +204,12 @@ int strip_create(const ocmp_space_s* s, Strip** out);
 void strip_destroy(Strip* p);
 int strip_factor(Strip* p, const ocmp_space_s* s, const double* vals, cudaStream_t st);
 // z = M^-1 (sc v), sc = scale[j] (scale != null) or 1; z may be v; the kernel returns at once when
-// flags[0] (the solver's convergence flag) is set, and sets a bit of *err when a wait gave up (after
-// which strip_reset makes the preconditioner usable again)
-constexpr int kSweepAbort = 4;
+// flags[0] (the solver's convergence flag) is set, and sets *err when a wait gave up (after which
+// strip_reset makes the preconditioner usable again)
 template <class T>
 int strip_apply(Strip* p, const T* v, const double* scale, int j, T* z, const int* flags, int* err, cudaStream_t st);
 int strip_reset(Strip* p, cudaStream_t st);
+int strip_starve(Strip* p);
 template <class T>
 int strip_add(int64_t n, const T* z, double* x, cudaStream_t st);
 void strip_stats(const Strip* p, ocmp_strip_stats_t* out);

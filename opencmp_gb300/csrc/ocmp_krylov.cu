@@ -454,7 +454,7 @@ int gm_read(const GmTeams* t, GmResult* out, GmResult* dev, int count, cudaStrea
     OCMP_CUDA(cudaMemcpyAsync(out, dev, sizeof(GmResult) * count, cudaMemcpyDeviceToHost, st));
     OCMP_CUDA(cudaStreamSynchronize(st));
     for (int q = 0; q < count; q++)
-        if (out[q].bits & GM_ABORT) {
+        if (out[q].gaveup) {
             OCMP_CUDA(cudaMemsetAsync(t->state, 0, sizeof(TeamState) * std::max(1, t->nteams), st));
             OCMP_CUDA(cudaMemsetAsync(dev, 0, sizeof(GmResult) * count, st));
             return fail(OCMP_TIMEOUT, "GMRES: a block gave up waiting for the others");
@@ -517,7 +517,6 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
     int* flags = sv->gout->flags;
     double* scale = sv->small + m * (m + 1) / 2 + 3 * m + 2;
     const GmResult* H = sv->hout;
-    static_assert(kSweepAbort == GM_ABORT, "one bit for a wait that gave up");
     auto read = [&]() {
         const int r = gm_read(sv->teams, sv->hout, sv->gout, 1, st);
         if (r == OCMP_TIMEOUT) strip_reset(sv->strip ? sv->strip : sv->cc->strip, st);
@@ -529,8 +528,8 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
         return gm_launch<T>(a, sv->teams, st);
     };
     auto apply = [&](const T* v, const double* sc, int j, const int* fl) {
-        return sv->strip ? strip_apply<T>(sv->strip, v, sc, j, z, fl, &sv->gout->bits, st)
-                         : cc_apply<T>(sv->cc, v, sc, j, z, fl, &sv->gout->bits, st);
+        return sv->strip ? strip_apply<T>(sv->strip, v, sc, j, z, fl, &sv->gout->gaveup, st)
+                         : cc_apply<T>(sv->cc, v, sc, j, z, fl, &sv->gout->gaveup, st);
     };
     if (sv->time_spmv) OCMP_CUDA(cudaMemsetAsync(sv->tlog, 0, sizeof(unsigned long long) * 2 * kTimedProducts, st));
     int r = launch(GM_FIRST, 0);
@@ -564,7 +563,7 @@ int gm_phases(ocmp_solver_s* sv, const double* b, double* x, cudaStream_t st, in
             if (before >= 0) {
                 OCMP_CUDA(cudaEventSynchronize(sv->ev_check[before]));
                 const GmResult& R = sv->hout[1 + before];
-                if (R.bits & GM_ABORT) break;   // found again, and cleared, by the read below
+                if (R.gaveup) break;   // found again, and cleared, by the read below
                 if (R.flags[F_CONV]) {
                     it--;
                     break;
@@ -912,6 +911,21 @@ int ocmp_solver_strip_schulz(ocmp_solver_t sv, int32_t on) {
     if (!sv) return fail(OCMP_ERR_ARG, "ocmp_solver_strip_schulz: null solver");
     if (!sv->strip) return fail(OCMP_ERR_ARG, "ocmp_solver_strip_schulz: solver not created with OCMP_PRE_STRIP");
     strip_set_schulz(sv->strip, on != 0);
+    return OCMP_OK;
+}
+
+// A test's entry, not part of the interface: in the next solve a wait of one block for another (which 0),
+// or of the strip's sweeps (1), runs out.
+int ocmp_test_starve(ocmp_solver_t sv, int32_t which) {
+    if (!sv) return fail(OCMP_ERR_ARG, "ocmp_test_starve: null solver");
+    if (which == 1) {
+        Strip* p = sv->strip ? sv->strip : sv->cc ? sv->cc->strip : nullptr;
+        return p ? strip_starve(p) : fail(OCMP_ERR_ARG, "ocmp_test_starve: no strip");
+    }
+    const int on = 1;
+    TeamState* t = sv->dcg ? &sv->dcg->t : sv->teams->state;
+    for (int k = 0; k < (sv->dcg ? 1 : std::max(1, sv->teams->nteams)); k++)
+        OCMP_CUDA(cudaMemcpy(&t[k].starve, &on, sizeof(int), cudaMemcpyHostToDevice));
     return OCMP_OK;
 }
 

@@ -1758,6 +1758,13 @@ int strip_reset(Strip* p, cudaStream_t st) {
     return OCMP_OK;
 }
 
+// a test: a wait of the next application runs out
+int strip_starve(Strip* p) {
+    const int on = 1;
+    OCMP_CUDA(cudaMemcpy(&p->d_state->starve, &on, sizeof(int), cudaMemcpyHostToDevice));
+    return OCMP_OK;
+}
+
 template <class T>
 int strip_add(int64_t n, const T* z, double* x, cudaStream_t st) {
     OCMP_LAUNCH(k_add_to<T><<<nblk(n, 256), 256, 0, st>>>(n, z, x));

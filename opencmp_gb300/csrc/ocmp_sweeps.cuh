@@ -25,6 +25,7 @@
 #pragma once
 
 #include "ocmp_mbar.cuh"
+#include "ocmp_team.cuh"
 
 namespace ocmp {
 
@@ -50,10 +51,11 @@ struct SweepStep {
 };
 __device__ __forceinline__ int sweep_position(const SweepStep& s, int r) { return r < s.nN ? r : r + s.gap; }
 
-// `left` blocks are done with this launch; the last one counts the epoch on.
+// `left` blocks are done with this launch; the last one counts the epoch on. starve (a test): the first
+// block of the next launch keeps its share of the vector to itself.
 struct SweepState {
     unsigned epoch, left;
-    int abort, pad;
+    int abort, starve;   // side by side: a wait gets the address of the first
 };
 
 struct SweepArgs {
@@ -66,7 +68,7 @@ struct SweepArgs {
     uint2* y;
     uint2* x;
     SweepState* state;
-    int* err;                 // a bit is set when a wait gave up
+    int* err;                 // set when a wait gave up
     int64_t n;
     int stages, stage;        // the ring: stages of so many floats
     int rows;                 // largest number of rows of a block
@@ -133,7 +135,7 @@ __device__ __forceinline__ bool sweep_poll(const uint2* p, unsigned epoch, volat
         if (spin & 63u) continue;
         if (*abort) return false;
         if (t0 == 0) t0 = clock64();
-        else if (clock64() - t0 > kSweepWaitCycles) return false;
+        else if (clock64() - t0 > (abort[1] ? kStarvedCycles : kSweepWaitCycles)) return false;
     }
 }
 __device__ __forceinline__ void sweep_put(uint2* p, float v, unsigned epoch) {
@@ -190,7 +192,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         for (int t = 0; t < min(a.stages, a.nsteps); t++) fetch(t, t);
     {
         const double sc = scale ? scale[j] : 1.0;
-        for (int64_t q = block * (int64_t)kSweepThreads + tid; q < a.n; q += (int64_t)size * kSweepThreads)
+        const int64_t n = block == 0 && abort[1] ? 0 : a.n;
+        for (int64_t q = block * (int64_t)kSweepThreads + tid; q < n; q += (int64_t)size * kSweepThreads)
             sweep_put(a.b + q, scale ? (float)(T)((double)v[q] * sc) : (float)v[q], epoch);
     }
 
@@ -351,7 +354,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     if (!ok) {
         if (tid == 0) {
             atomicExch(&a.state->abort, 1);
-            if (a.err) atomicOr(a.err, kSweepAbort);
+            if (a.err) atomicExch(a.err, 1);
         }
         // the copies in flight: the last one of each stage
         if (tid == kFetcher)

@@ -24,6 +24,7 @@ namespace ocmp {
 // A poll gives up after about four seconds of SM clock; no phase between two exchanges takes longer
 // than a few milliseconds.
 constexpr long long kTeamWaitCycles = 8000000000LL;
+constexpr long long kStarvedCycles = 1000000LL;   // of a wait that a test lets run out
 constexpr int kTeamMaxBlocks = 160;   // one block per SM of this part
 constexpr int kTeamMaxValues = 2;     // values of one exchange
 constexpr int kTeamMaxThreads = 1024;
@@ -31,11 +32,13 @@ constexpr int kTeamMaxThreads = 1024;
 // Device state of a team: arrivals at the barrier (never reset: a launch starts from the count its
 // predecessor left), the blocks that have left, the flag of a poll that gave up, and the blocks'
 // partial sums (exchanges alternate between two sets: a set is written again only after another
-// exchange, which no block passes before all have read it). Zeroed at creation.
+// exchange, which no block passes before all have read it). Zeroed at creation, and by the host after a
+// wait that gave up. starve (a test): the next launch waits for one arrival too many.
 struct TeamState {
     unsigned arrive, left;
     int abort;
     unsigned start;
+    int starve, pad;
     double part[2][kTeamMaxValues][kTeamMaxBlocks];
 };
 
@@ -47,7 +50,7 @@ struct Team {
 };
 
 __device__ __forceinline__ Team team_join(TeamState* s, int rank, int size) {
-    return Team{s, rank, size, size > 1 ? *(volatile unsigned*)&s->start : 0u, 0};
+    return Team{s, rank, size, size > 1 ? *(volatile unsigned*)&s->start + (*(volatile int*)&s->starve ? 1u : 0u) : 0u, 0};
 }
 
 // Sum of cnt <= 32 CAP doubles, entry i read by get(i), by one warp; every lane returns it.
@@ -155,7 +158,7 @@ __device__ __forceinline__ bool team_barrier(Team& t) {
             if (spin & 63u) continue;
             if (*(volatile int*)&t.s->abort) ok = 0;
             else if (t0 == 0) t0 = clock64();
-            else if (clock64() - t0 > kTeamWaitCycles) {
+            else if (clock64() - t0 > (*(volatile int*)&t.s->starve ? kStarvedCycles : kTeamWaitCycles)) {
                 atomicExch(&t.s->abort, 1);
                 ok = 0;
             }
