@@ -79,7 +79,7 @@ struct GmArgs {
     int nqueue;
     TeamState* teams;
     double* part;           // (m + 2) x blocks
-    unsigned long long* tlog;   // product timing: start and end per product, or null
+    unsigned long long* tlog;   // product timing: complement of the start, and end per product, or null
     int tcap, m, mode, j;
     int rp_slices;          // slices of 32 rows whose row pointers fit the blocks' shared memory
 };
@@ -320,7 +320,7 @@ struct GmRun {
         unsigned long long* tl = nullptr;
         if (a.tlog && products < (unsigned)a.tcap) {
             tl = a.tlog + 2 * products;
-            if (threadIdx.x == 0 && tm.rank == 0) tl[0] = gm_time();
+            if (threadIdx.x == 0) atomicMax(tl, ~gm_time());   // the first block's start
         }
         products++;
         const T* xin = basis ? V + (int64_t)j * ld : (const T*)d.z;

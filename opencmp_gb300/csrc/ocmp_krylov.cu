@@ -84,7 +84,7 @@ struct ocmp_solver_s {
     int B = 1;                  // systems in the batch (matrix instances)
     // optional timing of the Krylov products (ocmp_solver_spmv_timing)
     bool time_spmv = false;
-    unsigned long long* tlog = nullptr;   // per product: start and end (global timer, ns)
+    unsigned long long* tlog = nullptr;   // per product: complement of the start, and end (global timer, ns)
     // the FP32 Krylov matrix is the assembly's SELL-32 copy (OCMP_MAT_SELL32, borrowed)
     bool sell = false;
     int last_iters = 0;         // iterations of the last GMRES solve (adaptive host checks)
@@ -471,8 +471,8 @@ int gm_collect_times(ocmp_solver_s* sv, cudaStream_t st) {
     OCMP_CUDA(cudaMemcpyAsync(t.data(), sv->tlog, sizeof(unsigned long long) * t.size(), cudaMemcpyDeviceToHost, st));
     OCMP_CUDA(cudaStreamSynchronize(st));
     for (int k = 0; k < kTimedProducts; k++)
-        if (t[2 * k] && t[2 * k + 1] > t[2 * k]) {
-            sv->spmv_ms += 1e-6 * (double)(t[2 * k + 1] - t[2 * k]);
+        if (t[2 * k + 1]) {   // (a product shorter than the timer's step takes 0)
+            sv->spmv_ms += 1e-6 * (double)(t[2 * k + 1] - ~t[2 * k]);
             sv->spmv_launches++;
         }
     return OCMP_OK;

@@ -1,5 +1,5 @@
 """Krylov handles and their neighbours used from several host threads, a handle each; what a handle of many
-tiny systems holds."""
+tiny systems holds; the products that a handle counts."""
 import ctypes as C
 import threading
 
@@ -139,3 +139,20 @@ def test_memory_of_a_batch_of_tiny_systems(gpu_lib, precision):
     # beside these a few vectors and results per system, and the allocator's granularity
     assert used <= small + basis + 1000 * B + (64 << 20), (used, small, basis)
     assert sv.h
+
+
+@pytest.mark.parametrize('precond', ['jacobi', 'strip'])
+@pytest.mark.parametrize('n', [2, 12, 60])
+def test_every_product_is_counted(gpu_lib, precond, n):
+    import torch
+    from opencmp_gb300 import fem
+    sp, A, b = _system(n, 1)
+    sv = fem.KrylovSolver(A, method='GMRES', restart=30, precond=precond, tol=1e-10, maxit=2000)
+    sv.update()
+    sv.spmv_timing(True)
+    total = 0
+    for _ in range(3):
+        total += sv.solve(b, torch.zeros_like(b)).iterations
+        # one more may be queued past convergence with the strip; it does no product
+        count, ms = sv.spmv_stats()
+        assert count == total and ms >= 0.0
