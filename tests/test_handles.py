@@ -156,3 +156,20 @@ def test_every_product_is_counted(gpu_lib, precond, n):
         # one more may be queued past convergence with the strip; it does no product
         count, ms = sv.spmv_stats()
         assert count == total and ms >= 0.0
+
+
+def test_graph_switch_is_accepted_for_gmres_and_changes_nothing(gpu_lib):
+    import torch
+    from opencmp_gb300 import _lib as LB, fem
+    sp, A, b = _system(20, 2)
+    xs = []
+    for on in (False, True):
+        sv = fem.KrylovSolver(A, method='GMRES', restart=20, tol=1e-10, maxit=500)
+        sv.set_graph(on)
+        xs.append(torch.zeros_like(b))
+        sv.solve(b, xs[-1])
+    assert torch.equal(*xs)
+    for kw in (dict(method='CG'), dict(method='GMRES', precond='strip')):
+        with pytest.raises(LB.OcmpError) as e:
+            fem.KrylovSolver(A, tol=1e-10, **kw).set_graph(True)
+        assert e.value.status == LB.ERR_UNSUPPORTED
