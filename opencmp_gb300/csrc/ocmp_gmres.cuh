@@ -68,6 +68,7 @@ struct GmInst {
     GmResult* out;
     double tol, inner;
     int maxit, L, TR, tpr, rtpr;  // rows per tile; lanes per row of the Krylov product and of the FP64 one
+    int u64, pad;           // entries in flight per lane of an FP64 solve's products
 };
 
 struct GmArgs {
@@ -254,15 +255,22 @@ struct GmRun {
             if (r < n && lane % TPR == 0) fn(r, v);
         }
     }
-    template <class TM, class F>
-    __device__ __forceinline__ void products_by(int tpr, const TM* val, const TM* x, F fn) const {
-        // entries in flight per lane, as the threads' registers allow
-        constexpr int U = sizeof(TM) == 4 ? 8 : 4;
+    template <int U, class TM, class F>
+    __device__ __forceinline__ void products_lanes(int tpr, const TM* val, const TM* x, F fn) const {
         if (tpr == 1) products_of<1, U>(val, x, fn);
         else if (tpr == 2) products_of<2, U>(val, x, fn);
         else if (tpr == 4) products_of<4, U>(val, x, fn);
         else if (tpr == 8) products_of<8, U>(val, x, fn);
         else products_of<16, U>(val, x, fn);
+    }
+    template <class TM, class F>
+    __device__ __forceinline__ void products_by(int tpr, const TM* val, const TM* x, F fn) const {
+        // entries in flight per lane, as the threads' registers allow
+        if constexpr (D) {
+            if (d.u64 == 8) products_lanes<8>(tpr, val, x, fn);
+            else products_lanes<4>(tpr, val, x, fn);
+        } else
+            products_lanes<sizeof(TM) == 4 ? 8 : 4>(tpr, val, x, fn);
     }
 
     // z = B^-1 v (or x += B^-1 v) over the owned elements (their rows are the block's own)

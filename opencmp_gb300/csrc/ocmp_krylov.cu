@@ -82,6 +82,7 @@ struct ocmp_solver_s {
     const float* K32 = nullptr;
     bool borrow = false;        // Jacobi-scaled values and D^-1 come from the assembly
     int B = 1;                  // systems in the batch (matrix instances)
+    int u64 = 4;                // GMRES: entries in flight per lane of the FP64 products
     // optional timing of the Krylov products (ocmp_solver_spmv_timing)
     bool time_spmv = false;
     unsigned long long* tlog = nullptr;   // per product: complement of the start, and end (global timer, ns)
@@ -293,6 +294,21 @@ int gm_lanes(const ocmp_space_s* s, bool fp64) {
     return fp64 ? std::max(1, t / 2) : t;
 }
 
+// Entries in flight per lane of an FP64 solve's products: 8, unless that pads the rows (an entry past a
+// row's end takes its turn on the FP64 pipe) by over 4% more than 4 does, the longest row of each slice of
+// 32 counted. Per iteration: P2 tetrahedra (3% more) 30.9 -> 30.3 us at 79,507 rows, 391 -> 367 at 1,771,561;
+// P3 tetrahedra (2%) 245 -> 213 at 753,571; but DG P2 triangles, rows of 24 (33%), 28.2 -> 29.8 at 62,208 and
+// P3 triangles (5%) 183 -> 185 at 811,801.
+int gm_unroll(const ocmp_space_s* s) {
+    const int lanes = gm_lanes(s, true);
+    int64_t pad4 = 0, pad8 = 0;
+    for (const int w : s->slice_width) {
+        pad4 += (w + 4 * lanes - 1) / (4 * lanes) * 4;
+        pad8 += (w + 8 * lanes - 1) / (8 * lanes) * 8;
+    }
+    return 25 * pad8 <= 26 * pad4 ? 8 : 4;
+}
+
 template <class T>
 GmInst gm_inst(const ocmp_solver_s* sv, int q, const double* b, double* x, int tile) {
     const ocmp_space_s* s = sv->s;
@@ -338,6 +354,7 @@ GmInst gm_inst(const ocmp_solver_s* sv, int q, const double* b, double* x, int t
     d.TR = d.Binv ? (d.L == 10 ? 160 : 96) : tile;
     d.tpr = gm_lanes(s, D);
     d.rtpr = gm_lanes(s, true);
+    d.u64 = sv->u64;
     return d;
 }
 
@@ -716,6 +733,7 @@ int ocmp_solver_create(ocmp_matrix_t mat, const ocmp_solve_params_t* prm, ocmp_s
     sv->K64 = sv->borrow ? mat->svals64 : sv->As64;
     sv->K32 = sv->borrow ? mat->svals32 : sv->As32;
     sv->sell = sv->borrow && mixed && (mat->flags & OCMP_MAT_SELL32) && s->d_sell_off != nullptr;
+    if (gm && !mixed) sv->u64 = gm_unroll(s);
     if (gm && !st) {
         std::vector<GmInst> inst;
         for (int q = 0; q < NB; q++) inst.push_back(mixed ? gm_inst<float>(sv, q, nullptr, nullptr, 32)
