@@ -74,7 +74,7 @@ struct GmInst {
 struct GmArgs {
     GmInst one;
     const GmInst* list;     // null: `one`
-    const int4* map;        // per block: team, rank, size, instance (-1: none); null: one team
+    const int4* map;        // per block: team, rank, size, instance (-1: none); null: one team, or (with a queue) none
     const int* queue_inst;  // instances of single blocks, largest first
     int* queue;             // next of them
     int nqueue;
@@ -91,6 +91,7 @@ struct GmArgs {
 // system per block, largest first.
 struct GmTeams {
     int grid = 0, nqueue = 0, nteams = 0;
+    bool small = false;          // queue only, blocks of kGmSmallThreads
     std::vector<int> tile;       // per system: rows per tile
     int64_t max_slices = 0;      // slices of 32 rows of the largest block
     TeamState* state = nullptr;
@@ -115,9 +116,15 @@ __host__ __device__ constexpr int64_t gm_ld(int64_t n) {
 
 __host__ __device__ constexpr int gm_small_doubles(int m) { return m * (m + 1) / 2 + 4 * m + 8; }
 
+// Threads of a block: one block per SM, or kGmSmallThreads where several blocks of an SM each solve systems of
+// few rows.
 template <class T>
+constexpr int kGmThreads = sizeof(T) == 8 ? 512 : 1024;
+constexpr int kGmSmallThreads = 128;
+
+template <class T, int NT_>
 struct GmCfg {
-    static constexpr int NT = sizeof(T) == 8 ? 512 : 1024;
+    static constexpr int NT = NT_;
     static constexpr int DT = 128;                         // FP64: threads holding a dot product's partials
     static constexpr int rows(int m) { return m + 8 < 64 ? m + 8 : 64; }   // values in that table at a time
     static constexpr int ES = sizeof(T) == 8 ? DT + 8 : NT / 32 + 1;   // stride of their shared table
@@ -174,9 +181,9 @@ __device__ __forceinline__ void gm_halve(float (&h)[N], float (&l)[N], int lane)
 }
 
 // A block's work on one system of its team.
-template <class T>
+template <class T, int NT_>
 struct GmRun {
-    using C = GmCfg<T>;
+    using C = GmCfg<T, NT_>;
     static constexpr int NT = C::NT, NW = NT / 32, DT = C::DT, ES = C::ES;
     static constexpr bool D = sizeof(T) == 8;
     const GmArgs& a;
@@ -320,7 +327,7 @@ struct GmRun {
             __syncthreads();
             block_apply(V, (T*)d.z, nullptr);
         }
-        return team_reduce<2>(tm, acc, out, NT);
+        return team_reduce<2, NT>(tm, acc, out, NT);
     }
 
     // V_{j+1} = sc (K xin)_free
@@ -595,8 +602,8 @@ struct GmRun {
             __syncthreads();
             block_apply(W, (T*)d.z, nullptr);
         }
-        if constexpr (D) return team_reduce<1>(tm, acc, hn2, live);
-        else return team_reduce_ff(tm, fh, fl, hn2);
+        if constexpr (D) return team_reduce<1, NT>(tm, acc, hn2, live);
+        else return team_reduce_ff<NT>(tm, fh, fl, hn2);
     }
 
     // Residual and start of a cycle; false when the team gave up. Sets `beta`, `nb`, `res`.
@@ -853,8 +860,8 @@ struct GmRun {
     }
 };
 
-template <class T>
-__global__ void __launch_bounds__(GmCfg<T>::NT, 1) gm_kernel(const __grid_constant__ GmArgs a) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(const __grid_constant__ GmArgs a) {
     extern __shared__ double gm_smem[];
     __shared__ int s_end, s_bits, s_next;
     __shared__ GmInst s_inst;
@@ -865,11 +872,12 @@ __global__ void __launch_bounds__(GmCfg<T>::NT, 1) gm_kernel(const __grid_consta
     };
     int4 at = make_int4(0, (int)blockIdx.x, (int)gridDim.x, 0);   // team, rank, size, instance
     if (a.map) at = a.map[blockIdx.x];
+    else if (a.queue) at.w = -1;
     int inst = at.w;
     if (inst >= 0) {
         if (a.list) fetch(inst);
         Team tm = team_join(a.teams + at.x, at.y, at.z);
-        GmRun<T> run(a, a.list ? s_inst : a.one, tm, gm_smem,
+        GmRun<T, NT> run(a, a.list ? s_inst : a.one, tm, gm_smem,
                      a.part + (int64_t)(a.map ? blockIdx.x - at.y : 0) * (a.m + 2));
         run.s_end = &s_end;
         run.s_bits = &s_bits;
@@ -889,11 +897,15 @@ __global__ void __launch_bounds__(GmCfg<T>::NT, 1) gm_kernel(const __grid_consta
         if (q >= a.nqueue) return;
         fetch(a.queue_inst[q]);
         Team tm = team_join(nullptr, 0, 1);
-        GmRun<T> run(a, s_inst, tm, gm_smem, nullptr);
+        GmRun<T, NT> run(a, s_inst, tm, gm_smem, nullptr);
         run.s_end = &s_end;
         run.s_bits = &s_bits;
         run.solve();
     }
 }
+
+// The kernel for queues of systems of few rows (a translation unit of its own).
+template <class T>
+const void* gm_small_kernel();
 
 }  // namespace ocmp

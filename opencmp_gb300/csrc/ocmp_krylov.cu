@@ -368,6 +368,58 @@ void gm_teams_free(GmTeams* t) {
     delete t;
 }
 
+constexpr size_t kGmSmem = 160 * 1024;   // the rest is left to L1, which the gathers live on
+constexpr int kGmMaxRestart = 128;
+template <class T>
+constexpr size_t kGmLargestTables = std::max(GmCfg<T, kGmThreads<T>>::smem(kGmMaxRestart),
+                                             GmCfg<T, kGmSmallThreads>::smem(kGmMaxRestart));
+static_assert(kGmLargestTables<double> <= kGmSmem && kGmLargestTables<float> <= kGmSmem, "the largest restart's tables");
+
+template <class T>
+int gm_smem_limit() {
+    const int r = smem_limit((const void*)gm_kernel<T, kGmThreads<T>>, kGmSmem);
+    return r ? r : smem_limit(gm_small_kernel<T>(), kGmSmem);
+}
+
+// dynamic shared memory of a launch: the tables and, where there is room, the rows' pointers
+template <class T, int NT>
+size_t gm_smem(const GmTeams* t, int m, bool pointers, int* slices) {
+    const size_t base = GmCfg<T, NT>::smem(m);
+    *slices = pointers && base < kGmSmem ? (int)std::min<int64_t>(t->max_slices, (kGmSmem - base) / (33 * 4)) : 0;
+    return base + (size_t)*slices * 33 * 4;
+}
+
+template <class T>
+int gm_launch(GmArgs& a, const GmTeams* t, cudaStream_t st) {
+    void* kp[] = {&a};
+    if (t->small) {
+        const size_t smem = gm_smem<T, kGmSmallThreads>(t, a.m, true, &a.rp_slices);
+        OCMP_LAUNCH(OCMP_CUDA(cudaLaunchKernel(gm_small_kernel<T>(), dim3(t->grid), dim3(kGmSmallThreads), kp, smem, st)));
+        return OCMP_OK;
+    }
+    const size_t smem = gm_smem<T, kGmThreads<T>>(t, a.m, a.mode == GM_FULL, &a.rp_slices);
+    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel((const void*)gm_kernel<T, kGmThreads<T>>, dim3(t->grid),
+                                                      dim3(kGmThreads<T>), kp, smem, st)));
+    return OCMP_OK;
+}
+
+// A queue of more systems than SMs, each of up to so many rows, is taken by blocks of 128 threads where at
+// least so many fit an SM: such a solve is a chain of latencies, and a block per SM ran one at a time (slower
+// than a launch per operation over all systems where they are tiny). Whole solves, one block per SM against
+// these (ms): 5,000 systems of 81 rows FP64 9.1 -> 4.8, FP32 11.1 -> 3.5 (a launch per operation: 11.4, 9.7);
+// 20,000 of 9 rows 7.2 -> 4.5 and 11.2 -> 4.8 (5.5, 6.8); 500 of 1,089 rows 11.1 -> 9.7 and 6.0 -> 4.5; but at
+// restart 60 in FP64, where two fit, 1,500 of 1,089 rows 30.1 -> 42.4.
+constexpr int64_t kGmSmallRows = 1024;
+constexpr int kGmSmallBlocks = 3;
+
+template <class T>
+int gm_small_blocks(const GmTeams* t, int m, int* per_sm) {
+    int slices = 0;
+    const size_t smem = gm_smem<T, kGmSmallThreads>(t, m, true, &slices);
+    OCMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, gm_small_kernel<T>(), kGmSmallThreads, smem));
+    return OCMP_OK;
+}
+
 int gm_teams_create(const std::vector<GmInst>& inst, const std::vector<int64_t>& nnz, int m, bool fp64, GmTeams** out) {
     int sms = 1;
     if (const int r = team_blocks(&sms)) return r;
@@ -413,10 +465,19 @@ int gm_teams_create(const std::vector<GmInst>& inst, const std::vector<int64_t>&
         const int64_t tr = std::max(t->tile[k], inst[k].TR);
         t->max_slices = std::max(t->max_slices, ((inst[k].n + tr - 1) / tr + blocks - 1) / blocks * (tr / 32));
     }
-    int st = dalloc(&t->state, (size_t)std::max(1, t->nteams));
+    int st = OCMP_OK;
+    int64_t rows = 0;
+    for (const GmInst& d : inst) rows = std::max(rows, d.n);
+    if (N > sms && t->nteams == 0 && rows <= kGmSmallRows) {
+        int per_sm = 0;
+        st = fp64 ? gm_small_blocks<double>(t, m, &per_sm) : gm_small_blocks<float>(t, m, &per_sm);
+        t->small = per_sm >= kGmSmallBlocks;
+        if (t->small) t->grid = std::min(N, sms * per_sm);
+    }
+    if (!st) st = dalloc(&t->state, (size_t)std::max(1, t->nteams));
     if (!st) st = dalloc(&t->part, (size_t)(m + 2) * t->grid);
     if (!st && N > 1) {
-        st = upload(&t->map, map.data(), map.size());
+        if (!t->small) st = upload(&t->map, map.data(), map.size());
         if (!st) st = upload(&t->qinst, qinst.data(), qinst.size());
         if (!st) st = dalloc(&t->queue, 1);
         if (!st) st = dalloc(&t->inst, (size_t)N);
@@ -442,28 +503,6 @@ GmArgs gm_args(const GmTeams* t, int m) {
     a.list = t->inst;
     a.m = m;
     return a;
-}
-
-constexpr size_t kGmSmem = 160 * 1024;   // the rest is left to L1, which the gathers live on
-constexpr int kGmMaxRestart = 128;
-static_assert(GmCfg<double>::smem(kGmMaxRestart) <= kGmSmem && GmCfg<float>::smem(kGmMaxRestart) <= kGmSmem,
-              "the largest restart's tables");
-
-template <class T>
-int gm_smem_limit() {
-    return smem_limit((const void*)gm_kernel<T>, kGmSmem);
-}
-
-template <class T>
-int gm_launch(GmArgs& a, const GmTeams* t, cudaStream_t st) {
-    const void* k = (const void*)gm_kernel<T>;
-    // room left for the rows' pointers
-    const size_t base = GmCfg<T>::smem(a.m);
-    a.rp_slices = a.mode == GM_FULL && base < kGmSmem ? (int)std::min<int64_t>(t->max_slices, (kGmSmem - base) / (33 * 4)) : 0;
-    const size_t smem = base + (size_t)a.rp_slices * 33 * 4;
-    void* kp[] = {&a};
-    OCMP_LAUNCH(OCMP_CUDA(cudaLaunchCooperativeKernel(k, dim3(t->grid), dim3(GmCfg<T>::NT), kp, smem, st)));
-    return OCMP_OK;
 }
 
 // the results, and whether a block gave up waiting

@@ -174,14 +174,14 @@ __device__ __forceinline__ bool team_barrier(Team& t) {
 // barrier as well. Only the first `live` threads' contributions are looked at. Four warps (one per
 // quarter of the SM) add the block's values per lane in FP64, then sum their lanes; 16 warps summing
 // theirs at once took 2,000 clocks.
-template <int NV>
+template <int NV, int NT = kTeamMaxThreads>   // NT: threads of the block, at most
 __device__ __forceinline__ bool team_reduce(Team& t, const double* v, double* out, int live) {
     static_assert(NV >= 1 && NV <= kTeamMaxValues, "values of an exchange");
-    __shared__ double val[NV][kTeamMaxThreads];
+    __shared__ double val[NV][NT > 128 ? NT : 1];
     __shared__ double wsum[NV][4];
     __shared__ double res[NV];
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    if (live > 128) {
+    if (NT > 128 && live > 128) {
         if (tid < live)
 #pragma unroll
             for (int i = 0; i < NV; i++) val[i][tid] = v[i];
@@ -191,7 +191,7 @@ __device__ __forceinline__ bool team_reduce(Team& t, const double* v, double* ou
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             double x = 0;
-            if (live > 128) {
+            if (NT > 128 && live > 128) {
                 x = val[i][tid];
                 for (int q = tid + 128; q < live; q += 128) x += val[i][q];
             } else if (tid < live)
@@ -226,6 +226,7 @@ __device__ __forceinline__ bool team_reduce(Team& t, const double* v, double* ou
 }
 
 // The same for one value held as float pairs: summed over the warps' lanes as pairs (48 bits).
+template <int NT = kTeamMaxThreads>
 __device__ __forceinline__ bool team_reduce_ff(Team& t, float h, float l, double* out) {
     __shared__ double wv[32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -239,7 +240,7 @@ __device__ __forceinline__ bool team_reduce_ff(Team& t, float h, float l, double
     double s = 0;
     if (w == 0) s = team_list_sum<1>(nw, lane, [&](int i) { return wv[i]; });
     double v[1] = {lane == 0 ? s : 0.0};
-    return team_reduce<1>(t, v, out, 1);
+    return team_reduce<1, NT>(t, v, out, 1);
 }
 
 // After its last exchange every block leaves; the last one writes down where the count stands.
