@@ -33,14 +33,18 @@ inline RowCfg row_cfg(const ocmp_space_s* s) {
     return {16, 8};
 }
 
-// the same for an FP64 product of its own launch
+// the same for an FP64 product of its own launch: half the lanes for rows of more than 16 entries, once they
+// fill the chip's threads. Below, the loads in flight count for more: P2 tetrahedra (us, cold L2, 2 x 8
+// against 4 x 8) 20.5 and 18.0 at 9,261 rows, 26.3 and 24.1 at 68,921, 33 and 32.4 at 148,877, 45 and 46
+// at 274,625; P3 tetrahedra (4 x 8 against 8 x 8) 27.2 and 23.7 at 29,791, 36.8 and 39.6 at 117,649.
+constexpr int64_t kChipThreads = 152 * 2048;
 inline RowCfg row_cfg64(const ocmp_space_s* s) {
     if (s->tuned_tpr > 0) return {s->tuned_tpr, s->tuned_u};
     const double avg = (double)s->nnz / (double)s->ndof;
     if (avg <= 6) return {2, 4};
-    if (avg <= 32) return {2, 8};
-    if (avg <= 64) return {4, 8};
-    return {8, 8};
+    if (avg <= 16) return {2, 8};
+    const RowCfg few = {avg <= 32 ? 2 : avg <= 64 ? 4 : 8, 8};
+    return s->ndof * few.tpr < kChipThreads ? row_cfg(s) : few;
 }
 
 template <class TM, class TV, int TPR, int U>
