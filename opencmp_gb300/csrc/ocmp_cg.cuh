@@ -5,7 +5,7 @@
 //   p = z + beta p                                          barrier
 // Two forms:
 //  - resident (cg_res_kernel), systems of up to 1024 rows a block whose matrix entries fit the blocks'
-//    shared memory (34 MB over the chip): a thread owns a row (two in the largest), its vector entries
+//    shared memory (31 MB over the chip): a thread owns a row (two in the largest), its vector entries
 //    stay in registers and its matrix row in shared memory for the whole solve, in slices of 32 rows
 //    (entry j of the slice's rows side by side). Only z and p, which other blocks gather, go through
 //    global memory. A warp-wide FP64 instruction takes 64 clocks whatever its lanes do, so a lane per

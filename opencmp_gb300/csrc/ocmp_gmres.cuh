@@ -18,8 +18,11 @@
 // eight accumulators in each of 128 threads' rows, and sums over threads go through shared memory with
 // every lane adding (a butterfly wastes 31 of 32 additions). Below about 10^4 rows: the exchanges,
 // 2,430 clocks each. Five launches per iteration with two-stage reductions in each took 54 us an
-// iteration at 79,507 rows (P2 tetrahedra, FP64, basis of 15) and 33 us at 1,156; one launch takes 32
-// (product 9.5, bound by its gathers; dots 4.6, orthogonalisation 4.3) and 17 (on one block).
+// iteration at 79,507 rows (P2 tetrahedra, FP64, basis of 15) and 33 us at 1,156; one launch takes 30
+// (product 10.9 from the first block's start to the last one's end, bound by its gathers; dots 4.6,
+// orthogonalisation 4.3) and 13. From 1.8 M rows on in FP64, where everything streams from HBM, a launch per
+// operation was faster with its 64 warps per SM: 346 against 367 us at 1,771,561 rows, 506 against 575 at
+// 2,803,221.
 #pragma once
 
 #include <type_traits>
@@ -102,7 +105,8 @@ struct GmTeams {
     GmInst* inst = nullptr;      // device descriptors (several systems)
 };
 
-// FP32 systems of this many rows a block have tiles of 128 rows (16-byte loads of the basis).
+// FP32 systems of this many rows a block have tiles of 128 rows (16-byte loads of the basis). Against 32 rows
+// (us an iteration): 17.9 and 18.0 at 255 rows a block, 19.7 and 20.6 at 512, 37.3 and 41.1 at 1,807.
 constexpr int64_t kGmVecRows = 512;
 
 // Stride of the basis vectors: whole tiles of 128 rows where they are read in 16-byte loads; elsewhere 16

@@ -184,7 +184,10 @@ int cg_launch(const void* k, CgArgs<T>& a, int grid, int threads, size_t smem, c
 }
 
 // The whole CG solve in one cooperative launch. Resident form: a system of few rows and entries is one
-// block's (its exchanges are __syncthreads); above, the slices of 32 rows are dealt to the SMs.
+// block's (its exchanges are __syncthreads); above, the slices of 32 rows are dealt to the SMs. One block
+// against many (us an iteration): FP64 6.7 and 10.8 at 289 rows of 3,073 entries, 8.4 and 8.4 at 625 of
+// 4,177, 9.2 and 9.9 at 625 of 6,817, 10.7 and 9.6 at 961 of 10,591; FP32 5.7 and 8.8, 5.8 and 7.2, 6.4 and
+// 8.6, 6.5 and 8.0.
 constexpr int64_t kCgOneBlockRows = 1024, kCgOneBlockNnz = 8192;
 constexpr int64_t kCgFuseNnz = 4900;   // entries per block whose second FMA costs the barrier's 2,450 clocks
 constexpr size_t kCgSmem = 200 * 1024;
@@ -358,7 +361,9 @@ GmInst gm_inst(const ocmp_solver_s* sv, int q, const double* b, double* x, int t
     return d;
 }
 
-// One block up to these rows: its exchanges are __syncthreads, but one SM does all the arithmetic.
+// One block up to these rows: its exchanges are __syncthreads, but one SM does all the arithmetic. One block
+// against many (us an iteration): FP64 11.7 and 14.5 at 169 rows, 13.6 and 14.1 at 289, 15.0 and 14.1 at 441,
+// 17.3 and 14.1 at 529; FP32 13.9 and 17.6 at 289, 16.9 and 17.1 at 1,024, 20.5 and 15.5 at 1,681.
 constexpr int64_t kGmOneBlock64 = 512, kGmOneBlock32 = 1024;
 
 void gm_teams_free(GmTeams* t) {

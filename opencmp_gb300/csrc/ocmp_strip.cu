@@ -687,13 +687,13 @@ __global__ void k_transpose(const float* __restrict__ src, int64_t lds, int rows
     }
 }
 
-// dst = scale * src (rows x cols, leading dimensions)
+// dst = src (rows x cols, leading dimensions)
 __global__ void k_copy2d(const float* __restrict__ src, int64_t lds, int rows, int cols, float* __restrict__ dst,
-                         int64_t ldd, float scale) {
+                         int64_t ldd) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= (int64_t)rows * cols) return;
     const int r = (int)(t / cols), c = (int)(t % cols);
-    dst[(int64_t)r * ldd + c] = scale * src[(int64_t)r * lds + c];
+    dst[(int64_t)r * ldd + c] = src[(int64_t)r * lds + c];
 }
 
 // the last blocks of a strip's inverse: S_NI = -T1 (nN x n), S_II = X (n x n)
@@ -864,8 +864,8 @@ int transpose(const float* src, int64_t lds, int rows, int cols, float* dst, int
     OCMP_LAUNCH(k_transpose<<<g, b, 0, st>>>(src, lds, rows, cols, dst, ldd));
     return OCMP_OK;
 }
-int copy2d(const float* src, int64_t lds, int rows, int cols, float* dst, int64_t ldd, float scale, cudaStream_t st) {
-    OCMP_LAUNCH(k_copy2d<<<nblk((int64_t)rows * cols, 256), 256, 0, st>>>(src, lds, rows, cols, dst, ldd, scale));
+int copy2d(const float* src, int64_t lds, int rows, int cols, float* dst, int64_t ldd, cudaStream_t st) {
+    OCMP_LAUNCH(k_copy2d<<<nblk((int64_t)rows * cols, 256), 256, 0, st>>>(src, lds, rows, cols, dst, ldd));
     return OCMP_OK;
 }
 
@@ -973,7 +973,7 @@ int schulz_end(Strip* p, StripChain& c, const float* W, int mp, int n, bool star
     if (ok) p->ns_strips++;
     else if (started) p->ns_fallbacks++;
     if (!ok) {
-        int r = copy2d(W, mp, n, n, c.cur, n, 1.f, cs);
+        int r = copy2d(W, mp, n, n, c.cur, n, cs);
         if (!r) r = gj_tiles(p, c.cur, n, 0, n, c.work, cs);
         if (!r) r = transpose(c.cur, n, n, n, c.cur + (int64_t)n * n, n, cs);
         if (r) return r;
