@@ -77,10 +77,11 @@ struct GmInst {
 struct GmArgs {
     GmInst one;
     const GmInst* list;     // null: `one`
-    const int4* map;        // per block: team, rank, size, instance (-1: none); null: one team, or (with a queue) none
-    const int* queue_inst;  // instances of single blocks, largest first
-    int* queue;             // next of them
-    int nqueue;
+    const int4* map;        // per block: team, rank, size, instance (-1: none, -2: the team takes them from the
+                            // teams' queue); null: one team, or (with a queue) none
+    const int* queue_inst;  // instances of the teams' queue, then those of single blocks, largest first
+    int* queue;             // next of either: single blocks', teams'
+    int nteam, nqueue;
     TeamState* teams;
     double* part;           // (m + 2) x blocks
     unsigned long long* tlog;   // product timing: complement of the start, and end per product, or null
@@ -91,9 +92,10 @@ struct GmArgs {
 // The blocks of a launch as teams: one team of all of them for one system; for several, each system
 // gets blocks in proportion to its work (two or more: a team of its own) and the systems of less than
 // two blocks' work form a queue that the remaining blocks, and later the teams' blocks, empty one
-// system per block, largest first.
+// system per block, largest first. Where that would leave too many rows to a block, teams of one size
+// empty a queue of the larger systems first.
 struct GmTeams {
-    int grid = 0, nqueue = 0, nteams = 0;
+    int grid = 0, nteam = 0, nqueue = 0, nteams = 0;
     bool small = false;          // queue only, blocks of kGmSmallThreads
     std::vector<int> tile;       // per system: rows per tile
     int64_t max_slices = 0;      // slices of 32 rows of the largest block
@@ -864,7 +866,8 @@ struct GmRun {
     }
 };
 
-template <class T, int NT>
+// MANY: teams that take systems from their queue
+template <class T, int NT, bool MANY = false>
 __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(const __grid_constant__ GmArgs a) {
     extern __shared__ double gm_smem[];
     __shared__ int s_end, s_bits, s_next;
@@ -877,12 +880,35 @@ __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(c
     int4 at = make_int4(0, (int)blockIdx.x, (int)gridDim.x, 0);   // team, rank, size, instance
     if (a.map) at = a.map[blockIdx.x];
     else if (a.queue) at.w = -1;
-    int inst = at.w;
-    if (inst >= 0) {
-        if (a.list) fetch(inst);
+    if constexpr (MANY) {
+        if (at.w == -2) {
+            Team tm = team_join(a.teams + at.x, at.y, at.z);
+            double* part = a.part + (int64_t)(blockIdx.x - at.y) * (a.m + 2);
+            while (true) {
+                if (at.y == 0 && threadIdx.x == 0) a.teams[at.x].next = atomicAdd(a.queue + 1, 1);
+                if (!team_barrier(tm)) {
+                    if (threadIdx.x == 0) atomicExch(&a.list[0].out->gaveup, 1);
+                    return;
+                }
+                const int q = __ldcg(&a.teams[at.x].next);
+                if (q >= a.nteam) break;
+                fetch(a.queue_inst[q]);
+                GmRun<T, NT> run(a, s_inst, tm, gm_smem, part);
+                run.s_end = &s_end;
+                run.s_bits = &s_bits;
+                if (!run.solve()) {
+                    if (threadIdx.x == 0) atomicExch(&run.d.out->gaveup, 1);
+                    return;
+                }
+                __syncthreads();   // the descriptor is read to the end of the solve
+            }
+            team_leave(tm);
+        }
+    } else if (at.w >= 0) {
+        if (a.list) fetch(at.w);
         Team tm = team_join(a.teams + at.x, at.y, at.z);
         GmRun<T, NT> run(a, a.list ? s_inst : a.one, tm, gm_smem,
-                     a.part + (int64_t)(a.map ? blockIdx.x - at.y : 0) * (a.m + 2));
+                         a.part + (int64_t)(a.map ? blockIdx.x - at.y : 0) * (a.m + 2));
         run.s_end = &s_end;
         run.s_bits = &s_bits;
         if (!(a.mode == GM_FULL ? run.solve() : run.phase())) {
@@ -899,7 +925,7 @@ __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(c
         __syncthreads();
         const int q = s_next;
         if (q >= a.nqueue) return;
-        fetch(a.queue_inst[q]);
+        fetch(a.queue_inst[a.nteam + q]);
         Team tm = team_join(nullptr, 0, 1);
         GmRun<T, NT> run(a, s_inst, tm, gm_smem, nullptr);
         run.s_end = &s_end;
@@ -908,8 +934,10 @@ __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(c
     }
 }
 
-// The kernel for queues of systems of few rows (a translation unit of its own).
+// The kernels for queues of systems of few rows and for teams with a queue (translation units of their own).
 template <class T>
 const void* gm_small_kernel();
+template <class T>
+const void* gm_many_kernel();
 
 }  // namespace ocmp

@@ -38,7 +38,7 @@ struct TeamState {
     unsigned arrive, left;
     int abort;
     unsigned start;
-    int starve, pad;
+    int starve, next;   // next: the system that a team takes from its queue
     double part[2][kTeamMaxValues][kTeamMaxBlocks];
 };
 

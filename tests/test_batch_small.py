@@ -81,3 +81,33 @@ def test_group_of_many_small_systems(gpu_lib, precision):
     assert len(infos) == 200 and all(i.status == 0 and i.relres <= TOL for i in infos)
     for (sp, A, forms, b, x0, sv), x in zip(parts, xs):
         _check(sp, forms, b, x0, x, {0, len(forms) - 1})
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'mixed'])
+def test_large_systems_in_a_large_group(gpu_lib, precision):
+    """Systems whose share of the blocks would be small for their rows go one after another through teams of
+    blocks, the smaller ones one per block afterwards: each meets its tolerance, by the matrix too, and
+    equals its own solve to it (mass-dominated: condition below 1e4)."""
+    import torch
+    from opencmp_gb300 import fem
+    parts = [_members(n, order, B, 20, precision, seed=5) for n, order, B in ((128, 2, 40), (32, 2, 30), (4, 1, 50))]
+    group = fem.KrylovGroup([p[-1] for p in parts])
+    runs = []
+    for _ in range(2):
+        xs = [p[4].clone() for p in parts]
+        infos = group.solve([p[3] for p in parts], xs)
+        assert len(infos) == 120 and all(i.status == 0 and i.relres <= TOL for i in infos)
+        runs.append(xs)
+    assert all(torch.equal(u, v) for u, v in zip(*runs))
+    mixed = precision == 'mixed'
+    for (sp, A, forms, b, x0, sv), x in zip(parts, runs[0]):
+        f = torch.as_tensor(sp.FreeDofs(), device='cuda')
+        A1 = fem.Matrix(sp, jacobi64=not mixed, jacobi32=mixed)
+        for q in {0, len(forms) // 2, len(forms) - 1}:
+            A1.assemble(forms[q])
+            s = slice(q * sp.ndof, (q + 1) * sp.ndof)
+            y = x0[s].clone()
+            fem.KrylovSolver(A1, method='GMRES', restart=20, precision=precision, tol=TOL, maxit=3000).solve(
+                b[s].contiguous(), y)
+            assert torch.equal(x[s][~f], y[~f])
+            assert float((x[s] - y).norm()) <= 2 * 1e4 * TOL * max(float(y.norm()), float(b[s].norm()))
