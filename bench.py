@@ -40,11 +40,6 @@ GAUSS = dict(c=(0.25, 0.25, 0.25), s=0.1)
 METRIC = 'DOF/s to 1e-8 FP64 rel. residual: mixed+batched+learned vs plain FP64, 1 GB300'
 WORKLOAD = ('transient 3D convection-diffusion, unit cube {}^3 x 6 tets, H1 p=2, eps=1e-2, w=(1,0.5,0.25), implicit '
             'Euler dt=1e-3, full reassembly every step, GMRES({}) + Jacobi to 1e-8 FP64 relative residual')
-# DRAM bytes per matrix entry (dram__bytes_read.sum + dram__bytes_write.sum per launch / nnz) of the
-# dominant kernel from ncu captures on the 48^3 x 6 case (nnz 25,755,265): gm_spmv<float> on the CSR
-# copy (two launches: 221.7 and 222.0 MB), gm_spmv_sell on the SELL-32 copy (251.7 and 251.4 MB; the
-# slices' padding is the difference); the traffic of a launch is this figure times the launch's nnz
-TRAFFIC_PER_NNZ = {'gm_spmv_float': 8.615, 'gm_spmv_sell': 9.768}
 # DRAM bytes moved by one reassembly of the optimised path (element kernel, diagonal pass, gather;
 # ncu on the 48^3 x 6 case: 645 + 95 + 1,428 MB) per algorithmic byte of that case
 ASSEMBLY_TRAFFIC_RATIO = 2168.0 / 227.0
@@ -376,8 +371,8 @@ def run_ours(args):
                      else 'gm_kernel<float>, SELL-32 product (FP32 Krylov SpMV of the optimised path, 16-byte loads)',
                      'achieved': g_achieved, 'peak': peak, 'peak_kind': peak_kind, 'unit': 'GB/s',
                      'frac': g_achieved / peak if g_achieved else None,
-                     'traffic': TRAFFIC_PER_NNZ[kname] * nnz if kname in TRAFFIC_PER_NNZ else None,
-                     'traffic_source': 'ncu dram bytes on the 48^3 x 6 case, scaled by nnz',
+                     # (the counters of the solve's kernel hold all its phases, not the product alone)
+                     'traffic': None,
                      'algorithmic_bytes': g_bytes, 'avg_launch_ms': g_avg, 'launches_timed': g_launches,
                      'timing': 'global timer around every product of the timed steps, inside the kernel of the solve'},
         'roofline_fp64_spmv': {'bound': 'hbm', 'kernel': 'spmv64 (CSR FP64, ocmp_spmv) timed alone, 50 launches',

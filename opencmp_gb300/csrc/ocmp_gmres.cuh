@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(c
     __shared__ int s_end, s_bits, s_next;
     __shared__ GmInst s_inst;
     auto fetch = [&](int i) {   // the system's descriptor: read on every access otherwise
-        const int* src = reinterpret_cast<const int*>(a.list + i);
+        const int* src = reinterpret_cast<const int*>(a.list ? a.list + i : &a.one);
         for (int k = threadIdx.x; k < (int)(sizeof(GmInst) / 4); k += blockDim.x) reinterpret_cast<int*>(&s_inst)[k] = src[k];
         __syncthreads();
     };
@@ -905,10 +905,9 @@ __global__ void __launch_bounds__(NT, NT == kGmSmallThreads ? 4 : 1) gm_kernel(c
             team_leave(tm);
         }
     } else if (at.w >= 0) {
-        if (a.list) fetch(at.w);
+        fetch(at.w);
         Team tm = team_join(a.teams + at.x, at.y, at.z);
-        GmRun<T, NT> run(a, a.list ? s_inst : a.one, tm, gm_smem,
-                         a.part + (int64_t)(a.map ? blockIdx.x - at.y : 0) * (a.m + 2));
+        GmRun<T, NT> run(a, s_inst, tm, gm_smem, a.part + (int64_t)(a.map ? blockIdx.x - at.y : 0) * (a.m + 2));
         run.s_end = &s_end;
         run.s_bits = &s_bits;
         if (!(a.mode == GM_FULL ? run.solve() : run.phase())) {
