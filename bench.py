@@ -318,10 +318,9 @@ def run_ours(args):
     spmv_bytes = 12 * nnz + 4 * (ndof + 1) + 16 * ndof
     peak, peak_kind = peaks()
     achieved = spmv_bytes / (spmv_ms * 1e-3) / 1e9
-    # gm_spmv<float>: FP32 values + int32 columns (8 B per entry), row pointers, the input vector and
+    # the FP32 product: values + int32 columns (8 B per entry), row pointers, the input vector and
     # the new basis vector (4 B per row each), the free mask (1 B per row)
     g_bytes = 8 * nnz + 4 * (ndof + 1) + 9 * ndof
-    kname = 'gm_spmv_float' if args.csr32 else 'gm_spmv_sell'
     g_launches, g_ms = spmv_live
     g_avg = g_ms / max(g_launches, 1)
     g_achieved = g_bytes / (g_avg * 1e-3) / 1e9 if g_launches else None

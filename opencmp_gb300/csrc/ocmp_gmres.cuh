@@ -18,10 +18,10 @@
 // eight accumulators in each of 128 threads' rows, and sums over threads go through shared memory with
 // every lane adding (a butterfly wastes 31 of 32 additions). Below about 10^4 rows: the exchanges,
 // 2,430 clocks each. Five launches per iteration with two-stage reductions in each took 54 us an
-// iteration at 79,507 rows (P2 tetrahedra, FP64, basis of 15) and 33 us at 1,156; one launch takes 30
-// (product 10.9 from the first block's start to the last one's end, bound by its gathers; dots 4.6,
-// orthogonalisation 4.3) and 13. From 1.8 M rows on in FP64, where everything streams from HBM, a launch per
-// operation was faster with its 64 warps per SM: 346 against 367 us at 1,771,561 rows, 506 against 575 at
+// iteration at 79,507 rows (P2 tetrahedra, FP64, basis of 15) and 33 us at 1,156; one launch takes 29
+// (product 10.4 from the first block's start to the last one's end, bound by its gathers; dots 4.6,
+// orthogonalisation 4.3) and 13. From 1.8 M rows on in FP64, where the basis streams from HBM, a launch per
+// operation was faster with its 64 warps per SM: 349 against 362 us at 1,771,561 rows, 512 against 559 at
 // 2,803,221.
 #pragma once
 
