@@ -291,9 +291,14 @@ int cc_apply(CCPre* cc, const T* v, const double* scale, int j, T* z, const int*
 }
 
 // Lanes per row of a Krylov product: the autotuned choice, or the row length's; of an FP64 product half
-// of that (bound by the FP64 pipe, on which a shuffle-reduction step costs as much as a product).
+// of that (bound by the FP64 pipe, on which a shuffle-reduction step costs as much as a product). The
+// autotuned choice is an FP64 product's already, so rows of more than 16 entries are not left a single lane
+// by it. Halved against as tuned (us an iteration): P2 triangles (11.5 entries) 56.4 and 60.8, P1 tetrahedra
+// 40.7 and 41.6; P3 triangles (17) 50.5 and 44.3, DG P2 triangles (24) 121 and 106, P2 tetrahedra at
+// 2,146,689 rows 485 and 438.
 int gm_lanes(const ocmp_space_s* s, bool fp64) {
     const int t = row_cfg(s).tpr;
+    if (fp64 && s->tuned_tpr > 0 && s->nnz > 16 * s->ndof) return t;
     return fp64 ? std::max(1, t / 2) : t;
 }
 
