@@ -564,9 +564,8 @@ def run_ins(args):
 def run_batched(args):
     """Config 4: 512 independent steady 2D convection-diffusion problems of 12 (mesh, order) classes
     (n in {16, 32, 64, 128}, H1 p in {1, 2, 3}). One step = assemble every instance (one batched
-    assembly per class) and solve all of them with one solver group: every GMRES kernel launched once
-    over all 512 uneven instances (ocmp_group_solve), FP32 inner GMRES + FP64 refinement, one restart
-    cycle replayed from a CUDA graph. Recorded beside it: the same classes as 12 batched solves on 12
+    assembly per class) and solve all of them with one solver group: one launch over all 512 uneven
+    instances (ocmp_group_solve), FP32 inner GMRES + FP64 refinement. Recorded beside it: the same classes as 12 batched solves on 12
     host threads and streams, and the plain FP64 loop over instances."""
     import concurrent.futures as cf
     import torch
@@ -722,9 +721,8 @@ def run_batched(args):
                                    '1e-8; assembly + solve per step'.format(N, args.restart_batch),
                        'classes': len(C), 'total_dofs': total_dofs,
                        'l2': 'instances and bases exceed L2 together (no flush)'},
-            'optimised': {'kind': 'one solver group over all instances: every GMRES kernel launched once for all {} '
-                                  'uneven instances, FP32 inner GMRES + FP64 refinement, restart cycle from a CUDA '
-                                  'graph'.format(N),
+            'optimised': {'kind': 'one solver group over all instances: one launch for all {} uneven instances, FP32 '
+                                  'inner GMRES + FP64 refinement'.format(N),
                           'max_relres': float(max(i.relres for i in infos)),
                           'converged': int(sum(1 for i in infos if i.status == 0)),
                           'iters_mean': float(np.mean([i.iterations for i in infos])),

@@ -237,7 +237,8 @@ int ocmp_solve_batch(ocmp_solver_t solver, const double* b_dev, double* x_dev, v
  * (each a single or batched matrix of its own space: different sizes, orders and patterns) are
  * solved together in one launch: each system gets a team of blocks in proportion to its rows and
  * entries, systems of less than two blocks' work are taken one per block from a queue, largest
- * first, and every team iterates on its own until its system has converged. Each instance keeps its
+ * first (where that would crowd a block with rows, teams of one size take the larger systems from a
+ * queue before), and every team iterates on its own until its system has converged. Each instance keeps its
  * own Krylov space, tolerance and convergence test. Members must be GMRES with point
  * Jacobi (or no) preconditioning, CSR Krylov matrices, and share restart, precision and maxit.
  * ocmp_group_solve takes one right-hand side and solution array per member (its instances one
