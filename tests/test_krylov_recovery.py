@@ -30,7 +30,7 @@ def _system(n, order, batch=1, sell=False):
 
 def _solver(A, precond='jacobi'):
     from opencmp_gb300 import fem
-    sv = fem.KrylovSolver(A, method='GMRES', restart=20, precond=precond, precision='mixed', tol=1e-10, maxit=2000)
+    sv = fem.KrylovSolver(A, method='GMRES', restart=20, precond=precond, precision='mixed', tol=1e-10, maxit=20000)
     sv.update()
     return sv
 
@@ -110,11 +110,12 @@ def test_solve_after_a_wait_that_ran_out(gpu_lib, method, precond, n, order, whi
             assert info.iterations == ref.iterations and torch.equal(x, y)
 
 
-def test_batch_after_a_wait_that_ran_out(gpu_lib):
-    """Twenty teams of seven blocks."""
+@pytest.mark.parametrize('n,order,batch', [(40, 1, 20), (128, 2, 40)])
+def test_batch_after_a_wait_that_ran_out(gpu_lib, n, order, batch):
+    """Twenty teams of seven blocks; teams of four that take systems of 66,049 rows from a queue."""
     import torch
     from opencmp_gb300 import _lib as LB
-    sp, A, b = _system(40, 1, batch=20)
+    sp, A, b = _system(n, order, batch=batch)
     y = torch.zeros_like(b)
     _solver(A).solve_batch(b, y)
     sv = _solver(A)
